@@ -425,8 +425,6 @@ def run_gpu_arm(args):
     issue = issue_ceiling(tile[0] == 1, noise, S, alg_bytes, peak, clocks.get("sm_mhz"))
     if tile[0] != 1:
         kernel_name = "generate_kernel<%d,%d,%s>" % (tile[0], tile[1], "noise" if noise else "plain")
-    elif noise and tile[2] <= 64:
-        kernel_name = "generate_pipe_kernel"
     else:
         kernel_name = "generate_walk_kernel<%s>" % ("noise" if noise else "plain")
     line = {

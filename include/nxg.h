@@ -360,9 +360,11 @@ uint32_t nxg_validate_motion_request(const nxg_device_asset_desc *asset,
 /* Bytes of device workspace nxg_generate_packed needs for `strand_count`
  * strands of this asset at params->cvs_per_strand CVs: the strand-locality
  * sort (keys, permutation, per-guide bins) and the per-frame guide-offset
- * table (guide_count x cvs_per_strand float4, then 2 guide records per guide
- * and 32 zero entries).  The workspace must be
- * 256-byte aligned; its contents need no initialisation. */
+ * table (guide_count x cvs_per_strand float4, then 2 guide records per guide).
+ * Past 128 CVs the table is included up to 1,024 CVs while there are no more
+ * guides than strands, and optional: a workspace without room for it is
+ * accepted and takes a slower kernel.  The workspace must be 256-byte
+ * aligned; its contents need no initialisation. */
 uint64_t nxg_packed_workspace_size(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
                                    uint32_t strand_count);
 
@@ -417,12 +419,9 @@ uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset,
  * `block_size` threads (0: take nxg_launch_config::block_size).
  * lanes_per_strand 1 (with cvs_per_lane 1, strands of 2..32 CVs) selects the
  * lane-walk generator: base curve and stores lane-parallel, one lane walking
- * each strand's noise frame; with noise and block_size 64 (or below) its
- * CTAs are producer/consumer warp pairs; with noise, CTAs of eleven warps
- * keep ten noise-lattice columns per axis and strand, smaller CTAs twelve (a
- * warp holding a strand whose noise needs more evaluates gradient noise
- * directly).  It is the built-in choice for 2..32 CVs (352-thread CTAs with
- * noise, 256 without). */
+ * each strand's noise frame; its block_size is an upper bound (at most 384
+ * threads with noise, 256 without).  It is the built-in choice for 2..32
+ * CVs, and longer strands take it too while no tile is registered for them. */
 typedef struct nxg_tile {
     uint32_t lanes_per_strand;
     uint32_t cvs_per_lane;
@@ -434,14 +433,18 @@ typedef struct nxg_tile {
  * built-in choice.  Thread-safe; takes effect at the next launch. */
 uint32_t nxg_set_tile(uint32_t cvs_per_strand, uint32_t noise, const nxg_tile *tile);
 
-/* The tile the next launch for this CV count and noise setting will use. */
+/* The tile registered for this CV count and noise setting, else the built-in
+ * one (for more than 32 CVs the lane-group tile the autotuner starts from;
+ * while none is registered such strands take the lane walk, and a call that
+ * does not fill the GPU takes smaller CTAs). */
 uint32_t nxg_get_tile(uint32_t cvs_per_strand, uint32_t noise, nxg_tile *tile);
 
 /* Autotuner: prepares the strand order, then times every admissible tile
  * (lane groups and CVs per lane that hold the strand, CTAs of
- * 64/128/256/320/352 threads) over `repeats` launches of nxg_generate_packed_ordered with CUDA
+ * 64/128/256/384/512 threads) over `repeats` launches of nxg_generate_packed_ordered with CUDA
  * events on `stream`, registers the fastest with nxg_set_tile and returns
- * it.  It writes the outputs and synchronises the stream, so it is a
+ * it (for more than 32 CVs nothing stays registered when the lane walk is
+ * fastest, and the tile returned is nxg_get_tile's).  It writes the outputs and synchronises the stream, so it is a
  * set-up call, not part of the enqueue-only path. */
 uint32_t nxg_autotune_packed(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
                              const nxg_generation_params *params, const nxg_packed_output_desc *output,
@@ -506,8 +509,9 @@ uint32_t nxg_generate_batched(const nxg_device_asset_desc *assets, const nxg_def
  * synchronise the device -- using the library's own fixed scratch instead
  * of a caller workspace.  Same validation and output as
  * nxg_generate_packed; returns NXG_ERROR_STATIC_SCRATCH_LIMIT, before
- * touching the device, when nxg_packed_workspace_size for the request
- * exceeds NXG_STATIC_SCRATCH_BYTES (for a 4,096-guide description at 32
+ * touching the device, when what the request needs of
+ * nxg_packed_workspace_size (all but an optional table) exceeds
+ * NXG_STATIC_SCRATCH_BYTES (for a 4,096-guide description at 32
  * CVs, about 240,000 strands fit and a million do not).  Allocates
  * nothing.  The first call on each device looks up the scratch's device
  * address (once per device, and again after a device reset gives the device

@@ -158,8 +158,8 @@ uint32_t nxg_generate_packed_classic(const nxg_device_asset_desc *asset, const n
     const nxg_deformed_desc none{};
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
-                                config ? *config : default_config, first_strand, strand_count, workspace, s,
-                                nullptr, classic);
+                                config ? *config : default_config, first_strand, strand_count, workspace,
+                                workspace_bytes, s, nullptr, classic);
 }
 
 } // extern "C"

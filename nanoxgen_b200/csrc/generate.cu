@@ -14,17 +14,15 @@
 //   4. guide_offsets   : the frame's guide-offset table and guide frame
 //                        records;
 //   5. generate        : persistent CTAs walk contiguous ranges of the
-//                        permutation.  For 2..32 CVs (the built-in tile) the
-//                        lane-walk generator (walk.cuh): setup one lane per
-//                        strand, the base curve one lane per CV, the noise
-//                        frame one lane per strand walking the reference's
-//                        cursor, coalesced streaming stores.  Otherwise the
-//                        lane-group generator: a group of L lanes owns one
-//                        strand, the transported frame as prefix scans over
-//                        shuffles (generator_core.cuh), with a separate
-//                        roots kernel.
-// Strands longer than 128 CVs take a serial per-thread kernel that walks the
-// reference's cursor directly.
+//                        permutation with the lane-walk generator
+//                        (walk.cuh).  Where a lane-group tile is registered
+//                        (nxg_set_tile, up to 128 CVs): a group of L lanes
+//                        owns one strand, the transported frame as prefix
+//                        scans over shuffles (generator_core.cuh), with a
+//                        separate roots kernel.
+// Strands whose guide-offset table does not fit (the table's cap, more than
+// 1,024 CVs, or past 128 CVs a workspace without room for it) take a serial
+// per-thread kernel that walks the reference's cursor directly.
 #include "generator_core.cuh"
 #include "walk.cuh"
 #include "nxg_internal.h"
@@ -98,172 +96,34 @@ __global__ void generate_kernel(LaunchArgs g, const float4 *offsets) {
     }
 }
 
-// Strands of 2..32 CVs: the lane-walk generator (walk.cuh).  Persistent CTAs
-// over contiguous ranges of the strand order positions [range_begin,
-// range_end); each warp takes 32 strands at a time through setup (which also
-// writes the roots, root UVs and point counts), base, frame (with noise) and
-// store.  Without noise the base step writes the output directly (no
-// stage), applying Classic scalars itself when given.  Register budgets:
-// the noise variant runs one CTA of up to eleven warps per SM (its shared
-// memory allows no more: eleven-warp CTAs hold ten lattice columns per axis
-// and strand, smaller ones twelve); the plain one three CTAs of eight warps
-// (at most 80 registers), the plain Classic one two.
+// The lane-walk generator (walk.cuh).  Persistent CTAs over contiguous ranges
+// of the strand order; each warp takes g.batch strands at a time.  Register
+// budgets: the noise variant runs one CTA of up to sixteen warps per SM (at
+// most 128 registers); the plain one three CTAs of eight warps (at most 80
+// registers), the plain Classic one two.  The arguments stay in the constant
+// bank (__grid_constant__): an out-of-line call taking them by reference
+// otherwise copies them to every thread's stack first.
 template <bool NOISE, bool CLASSIC>
-__global__ void __launch_bounds__(NOISE ? 384 : 256, NOISE ? 1 : (CLASSIC ? 2 : 3))
-    generate_walk_kernel(LaunchArgs g, const float4 *offsets) {
-    constexpr bool kStaged = NOISE;
-    constexpr bool kWalk = NOISE;  // noise walk inside this kernel
+__global__ void __launch_bounds__(NOISE ? 32 * kWalkNoiseWarps : 256, NOISE ? 1 : (CLASSIC ? 2 : 3))
+    generate_walk_kernel(const __grid_constant__ LaunchArgs g, const float4 *offsets) {
     extern __shared__ float4 smem[];
-    const int P = static_cast<int>(g.p.cvs_per_strand);
-    const int warps = blockDim.x >> 5;
-    float4 *table = smem;
-    float *tvals = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(smem) + walk_head_bytes(kWalk) -
-                                             2u * sizeof(float) * kWalkMaxCvs);
-    float *rvals = tvals + kWalkMaxCvs;
-    unsigned char *warp_base = reinterpret_cast<unsigned char *>(rvals + kWalkMaxCvs);
-    if constexpr (kWalk) {
-        for (int i = threadIdx.x; i < kTableFloat4; i += blockDim.x) {
-            table[i] = make_float4(__ldg(g.a.gradients + 3 * i), __ldg(g.a.gradients + 3 * i + 1),
-                                   __ldg(g.a.gradients + 3 * i + 2), 0.0f);
-        }
-    }
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {  // t = cv / (P - 1) (generate.h:295-298)
-        tvals[i] = __fdiv_rn(static_cast<float>(i), static_cast<float>(P - 1));
-        rvals[i] = strand_radius(g.p, tvals[i]);
-    }
+    const uint32_t P = g.p.cvs_per_strand;
+    const uint32_t padded = walk_padded(P);
+    float *tvals = reinterpret_cast<float *>(smem + (NOISE ? kTableFloat4 << walk_table_copies(blockDim.x >> 5) : 0));
+    float *rvals = tvals + padded;
+    walk_fill_head<NOISE>(g, smem, tvals, rvals);
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int columns = walk_lattice_columns(warps);
-    const size_t warp_bytes = walk_warp_bytes(kWalk, kStaged, columns);
-    unsigned char *mine = warp_base + warp_bytes * warp;
-    float *stage = reinterpret_cast<float *>(mine);  // staged variants only
-    float4 *records = reinterpret_cast<float4 *>(kStaged ? mine + kWalkStageBytes : mine);
-    float2 *lattice = reinterpret_cast<float2 *>(mine + kWalkStageBytes);
-    float4 *scratch = reinterpret_cast<float4 *>(mine + kWalkRecordBytes);  // plain Classic variant only
-    uint32_t *locals = reinterpret_cast<uint32_t *>(mine + warp_bytes - kWalkLocalBytes);
-    const uint32_t span = g.range_end - g.range_begin;
-    const uint32_t begin = g.range_begin + static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x) * span / gridDim.x);
-    const uint32_t end =
-        g.range_begin + static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x + 1u) * span / gridDim.x);
-    for (uint32_t batch = begin + static_cast<uint32_t>(warp) * 32u; batch < end;
-         batch += static_cast<uint32_t>(warps) * 32u) {
-        const uint32_t item = batch + static_cast<uint32_t>(lane);
-        const bool valid = item < end;
-        const int in_batch = static_cast<int>(min(32u, end - batch));
-        const WalkRoot wr = walk_setup<NOISE>(g, records, locals, lane, valid ? item : batch, valid,
-                                              static_cast<uint32_t>(P));
-        __syncwarp();
-        if constexpr (CLASSIC && !NOISE) {
-            walk_classic_setup(g, records, lane, valid, locals[lane] & 0x7fffffffu, tvals, offsets, scratch, P);
-            __syncwarp();
-        }
-        if constexpr (kStaged) {
-            walk_base_direct<false, true>(g, records, locals, tvals, rvals, offsets, lane, in_batch, P, stage);
+    const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    unsigned char *mine = reinterpret_cast<unsigned char *>(rvals + padded) + walk_warp_bytes(NOISE, CLASSIC) * warp;
+    const uint32_t begin = static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x) * g.count / gridDim.x);
+    const uint32_t end = static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x + 1u) * g.count / gridDim.x);
+    for (uint32_t batch = begin + warp * g.batch; batch < end; batch += warps * g.batch) {
+        const int in_batch = static_cast<int>(min(g.batch, end - batch));
+        if constexpr (NOISE) {
+            walk_noise_batch<CLASSIC>(g, offsets, mine, smem, tvals, rvals, lane, batch, in_batch);
         } else {
-            walk_base_direct<CLASSIC>(g, records, locals, tvals, rvals, offsets, lane, in_batch, P);
-        }
-        __syncwarp();
-        if constexpr (kWalk) {
-            walk_frame(g.p, wr, lane < in_batch, stage + lane * kWalkRowFloats, lattice + lane, tvals, table, P,
-                       columns);
-            __syncwarp();
-        }
-        if constexpr (kStaged) {
-            if constexpr (CLASSIC) {
-                walk_classic_strand(g, records, stage, locals, lane, in_batch, P);
-                __syncwarp();
-                walk_store8_classic(g, records, stage, locals, rvals, lane, in_batch, P);
-            } else {
-                walk_store8(g, stage, locals, rvals, lane, in_batch, P);
-            }
-            __syncwarp();
-        }
-    }
-}
-
-// Noise on strands of 2..32 CVs without Classic scalars: one producer warp
-// and one consumer warp per 64-thread CTA over the CTA's contiguous range of
-// the strand order, sharing two stage buffers.  The producer runs setup and
-// base (the latency-bound gathers) into one buffer while the consumer runs
-// the noise frame and the stores (the arithmetic) from the other; hardware
-// named barriers hand the buffers over (1, 2: buffer full; 3, 4: buffer
-// empty).  Both warps step through the same batches, so every bar.sync has
-// its matching arrivals.
-__device__ __forceinline__ void named_sync(uint32_t id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ void named_arrive(uint32_t id) {
-    __threadfence_block();  // this warp's shared-memory reads and writes are done before the other warp proceeds
-    asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
-}
-
-__global__ void __launch_bounds__(64, 1) generate_pipe_kernel(LaunchArgs g, const float4 *offsets) {
-    extern __shared__ float4 smem[];
-    const int P = static_cast<int>(g.p.cvs_per_strand);
-    float4 *table = smem;
-    float *tvals = reinterpret_cast<float *>(smem + kTableFloat4);
-    float *rvals = tvals + kWalkMaxCvs;
-    unsigned char *base = reinterpret_cast<unsigned char *>(rvals + kWalkMaxCvs);
-    for (int i = threadIdx.x; i < kTableFloat4; i += blockDim.x) {
-        table[i] = make_float4(__ldg(g.a.gradients + 3 * i), __ldg(g.a.gradients + 3 * i + 1),
-                               __ldg(g.a.gradients + 3 * i + 2), 0.0f);
-    }
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {  // t = cv / (P - 1) (generate.h:295-298)
-        tvals[i] = __fdiv_rn(static_cast<float>(i), static_cast<float>(P - 1));
-        rvals[i] = strand_radius(g.p, tvals[i]);
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const bool producer = threadIdx.x < 32;
-    unsigned char *tail = base + 2 * kPipeBufferBytes;
-    float4 *records = reinterpret_cast<float4 *>(tail);                    // producer
-    float2 *lattice = reinterpret_cast<float2 *>(tail + kWalkRecordBytes);  // consumer
-    const float inv_p = 1.0f / static_cast<float>(P);
-    const uint32_t span = g.range_end - g.range_begin;
-    const uint32_t begin = g.range_begin + static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x) * span / gridDim.x);
-    const uint32_t end =
-        g.range_begin + static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x + 1u) * span / gridDim.x);
-    const uint32_t iterations = (end - begin + 31u) / 32u;
-    for (uint32_t it = 0; it < iterations; ++it) {
-        const uint32_t batch = begin + it * 32u;
-        const int in_batch = static_cast<int>(min(32u, end - batch));
-        const int b = static_cast<int>(it & 1u);
-        unsigned char *buf = base + b * kPipeBufferBytes;
-        float *stage = reinterpret_cast<float *>(buf);
-        float *fr = reinterpret_cast<float *>(buf + kWalkStageBytes);  // 12 x 32: root position, normal, surface_u, domain
-        uint32_t *locals = reinterpret_cast<uint32_t *>(buf + kWalkStageBytes + kPipeFrameBytes);
-        if (producer) {
-            if (it >= 2u) { named_sync(3u + b); }
-            const uint32_t item = batch + static_cast<uint32_t>(lane);
-            const bool valid = item < end;
-            const WalkRoot wr = walk_setup<true>(g, records, locals, lane, valid ? item : batch, valid,
-                                                 static_cast<uint32_t>(P));
-            fr[0 * 32 + lane] = wr.position.x;
-            fr[1 * 32 + lane] = wr.position.y;
-            fr[2 * 32 + lane] = wr.position.z;
-            fr[3 * 32 + lane] = wr.normal.x;
-            fr[4 * 32 + lane] = wr.normal.y;
-            fr[5 * 32 + lane] = wr.normal.z;
-            fr[6 * 32 + lane] = wr.surface_u.x;
-            fr[7 * 32 + lane] = wr.surface_u.y;
-            fr[8 * 32 + lane] = wr.surface_u.z;
-            fr[9 * 32 + lane] = wr.domain.x;
-            fr[10 * 32 + lane] = wr.domain.y;
-            fr[11 * 32 + lane] = wr.domain.z;
-            __syncwarp();
-            walk_base<false>(g, records, stage, locals, tvals, rvals, offsets, lane, in_batch, P, inv_p);
-            named_arrive(1u + b);
-        } else {
-            named_sync(1u + b);
-            WalkRoot wr;
-            wr.position = F3{fr[0 * 32 + lane], fr[1 * 32 + lane], fr[2 * 32 + lane]};
-            wr.normal = F3{fr[3 * 32 + lane], fr[4 * 32 + lane], fr[5 * 32 + lane]};
-            wr.surface_u = F3{fr[6 * 32 + lane], fr[7 * 32 + lane], fr[8 * 32 + lane]};
-            wr.domain = F3{fr[9 * 32 + lane], fr[10 * 32 + lane], fr[11 * 32 + lane]};
-            walk_frame(g.p, wr, lane < in_batch, stage + lane * kWalkRowFloats, lattice + lane, tvals, table, P,
-                       kWalkAxisColumns);
-            __syncwarp();
-            walk_store8(g, stage, locals, rvals, lane, in_batch, P);
-            if (it + 2u < iterations) { named_arrive(3u + b); }
+            walk_plain_batch<CLASSIC>(g, offsets, mine, tvals, rvals, lane, batch, in_batch);
         }
     }
 }
@@ -338,20 +198,17 @@ __global__ void strand_roots_kernel(LaunchArgs g) {
 }
 
 // The frame's guide-offset table (G x P float4) and, after it, the guide
-// frame records (2 float4 per guide) the lane-walk generator reads, then the
-// zero row (kWalkMaxCvs zero entries) its unused stencil slots point at.
+// frame records (2 float4 per guide) the lane-walk generator reads.
 __global__ void guide_offsets_kernel(AssetArgs a, FrameArgs f, uint32_t P, float support_scale, float4 *offsets) {
     const uint64_t n = static_cast<uint64_t>(a.guide_count) * P;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     const uint64_t first = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-    for (uint64_t k = first; k < static_cast<uint64_t>(kWalkMaxCvs); k += stride) {
-        offsets[n + 2u * a.guide_count + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
     for (uint64_t idx = first; idx < n; idx += stride) {
         offsets[idx] = guide_offset_entry(a, f, P, static_cast<uint32_t>(idx / P), static_cast<uint32_t>(idx % P));
     }
     for (uint64_t gi = first; gi < a.guide_count; gi += stride) {
-        guide_frame_entry(a, f, support_scale, static_cast<uint32_t>(gi), offsets + n + 2u * gi);
+        guide_frame_entry(a, f, support_scale, static_cast<uint32_t>(gi),
+                          guide_offset_entry(a, f, P, static_cast<uint32_t>(gi), 0u), offsets + n + 2u * gi);
     }
 }
 
@@ -689,29 +546,41 @@ constexpr uint64_t kWorkspaceAlign = 256u;
 inline uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1u) / a * a; }
 
 struct WorkspaceLayout {
-    uint64_t keys, order, hist, offsets, offset_bytes, total;
+    uint64_t keys, order, hist, offsets, total, wanted;
 };
 
 // Largest guide-offset table the warp-parallel generator stages; beyond it
-// (or beyond 128 CVs) strands take the serial per-thread kernel.
+// strands take the serial per-thread kernel.
 constexpr uint64_t kMaxOffsetTableBytes = uint64_t{1} << 30;
-constexpr uint32_t kMaxParallelCvs = 128u;
+constexpr uint32_t kMaxParallelCvs = 128u;  // of the lane groups, and of what a workspace must hold a table for
 
 bool parallel_path(uint32_t guide_count, uint32_t P) {
     return P <= kMaxParallelCvs && uint64_t{guide_count} * P * 16u <= kMaxOffsetTableBytes;
 }
 
+// Strands of more than kMaxParallelCvs CVs take the lane walk too where the
+// workspace holds their offset table (20,011 strands x 160 CVs with noise, 512
+// guides: 1,214 us on the serial kernel).  The workspace need not: a caller's
+// that holds the order alone stays valid and takes the serial kernel.  The
+// queried size asks for the table when it is no larger than the strands' own
+// points, so it never dominates a caller's memory.
+bool long_walk_path(uint32_t guide_count, uint32_t count, uint32_t P) {
+    return P > kMaxParallelCvs && P <= dev::kWalkMaxCvs && guide_count <= count &&
+           uint64_t{guide_count} * P * 16u <= kMaxOffsetTableBytes;
+}
+
 // keys[count] | order[count] | bins[guides + 1] | offsets[guides * P] (float4)
-// followed by the guide frame records [guides * 2] and the zero row
-// [kWalkMaxCvs] (float4)
+// followed by the guide frame records [guides * 2] (float4).  `total` is what
+// a caller has to provide, `wanted` what the size query asks for.
 WorkspaceLayout workspace_layout(uint32_t guide_count, uint32_t count, uint32_t P) {
     WorkspaceLayout w{};
     w.keys = 0u;
     w.order = align_up(uint64_t{count} * 4u, kWorkspaceAlign);
     w.hist = w.order + align_up(uint64_t{count} * 4u, kWorkspaceAlign);
     w.offsets = w.hist + align_up((uint64_t{guide_count} + 1u) * 4u, kWorkspaceAlign);
-    w.offset_bytes = parallel_path(guide_count, P) ? (uint64_t{guide_count} * (P + 2u) + dev::kWalkMaxCvs) * 16u : 0u;
-    w.total = w.offsets + align_up(w.offset_bytes, kWorkspaceAlign);
+    const uint64_t table = align_up(uint64_t{guide_count} * (P + 2u) * 16u, kWorkspaceAlign);
+    w.total = w.offsets + (parallel_path(guide_count, P) ? table : 0u);
+    w.wanted = w.offsets + (parallel_path(guide_count, P) || long_walk_path(guide_count, count, P) ? table : 0u);
     return w;
 }
 
@@ -819,29 +688,37 @@ KernelFn pick_lanes(int lanes, bool noise, bool classic) {
 // Packed as lanes | ppt << 8 | (block / 32) << 16; 0 means "not set".
 std::atomic<uint32_t> g_tiles[kMaxParallelCvs + 1][2];
 
+// Longest strand a lane-walk tile (lanes 1) can be registered for.  Longer
+// strands take the lane walk unless a lane-group tile is registered for them.
+constexpr uint32_t kMaxLaneWalkTile = 32u;
+
 bool valid_tile(uint32_t P, uint32_t lanes, uint32_t ppt) {
-    if (lanes == 1u) { return ppt == 1u && P >= 2u && P <= static_cast<uint32_t>(dev::kWalkMaxCvs); }
+    if (lanes == 1u) { return ppt == 1u && P >= 2u && P <= kMaxLaneWalkTile; }
     const bool lanes_ok = lanes == 2u || lanes == 4u || lanes == 8u || lanes == 16u || lanes == 32u;
     const bool ppt_ok = ppt == 1u || ppt == 2u || ppt == 4u;
     return lanes_ok && ppt_ok && lanes * ppt >= P && P >= 2u && P <= kMaxParallelCvs;
 }
 
 // Tile shape for P CVs: the registered one, else the lane-walk generator for
-// 2..32 CVs (lanes_per_strand 1; CTAs of 352 threads with noise, 256
+// 2..32 CVs (lanes_per_strand 1; CTAs of 512 threads with noise, 256
 // without), else four CVs per lane on the narrowest power-of-two group that
-// holds the strand.
+// holds the strand (what the autotuner starts from: unregistered, longer
+// strands take the lane walk as well).
+uint32_t registered_tile(uint32_t P, bool noise) {
+    return P <= kMaxParallelCvs ? g_tiles[P][noise ? 1 : 0].load(std::memory_order_relaxed) : 0u;
+}
+
 void default_tile(uint32_t P, bool noise, int *lanes, int *ppt, uint32_t *block) {
-    const uint32_t packed = P <= kMaxParallelCvs ? g_tiles[P][noise ? 1 : 0].load(std::memory_order_relaxed) : 0u;
-    if (packed) {
+    if (const uint32_t packed = registered_tile(P, noise)) {
         *lanes = static_cast<int>(packed & 0xffu);
         *ppt = static_cast<int>((packed >> 8) & 0xffu);
         *block = ((packed >> 16) & 0xffu) * 32u;
         return;
     }
-    if (P >= 2u && P <= static_cast<uint32_t>(dev::kWalkMaxCvs)) {  // the lane-walk generator
+    if (P >= 2u && P <= kMaxLaneWalkTile) {  // the lane-walk generator
         *lanes = 1;
         *ppt = 1;
-        *block = noise ? 352u : 256u;  // with noise: eleven 20 KB warps fill the SM's shared memory
+        *block = noise ? 32u * dev::kWalkNoiseWarps : 256u;
         return;
     }
     *ppt = 4;
@@ -852,10 +729,6 @@ void default_tile(uint32_t P, bool noise, int *lanes, int *ppt, uint32_t *block)
 }
 
 KernelFn pick_kernel(int lanes, int ppt, bool noise, bool classic) {
-    if (lanes == 1) {
-        if (classic) { return noise ? dev::generate_walk_kernel<true, true> : dev::generate_walk_kernel<false, true>; }
-        return noise ? dev::generate_walk_kernel<true, false> : dev::generate_walk_kernel<false, false>;
-    }
     switch (ppt) {
         case 1: return pick_lanes<1>(lanes, noise, classic);
         case 2: return pick_lanes<2>(lanes, noise, classic);
@@ -863,22 +736,14 @@ KernelFn pick_kernel(int lanes, int ppt, bool noise, bool classic) {
     }
 }
 
-// Dynamic shared memory of the generate kernels; for the lane-walk kernel,
-// `staged` says whether its stage is used and `noise` whether it walks the
-// noise frame itself.
 uint32_t launch_kernel(void (*fn)(LaunchArgs, const float4 *), uint32_t grid, uint32_t block, size_t shm,
                        cudaStream_t stream, const LaunchArgs &g, const float4 *offsets) {
     fn<<<grid, block, shm, stream>>>(g, offsets);
     return record_cuda(cudaGetLastError());
 }
 
-
-size_t generate_smem_bytes(uint32_t P, int lanes, int ppt, bool noise, bool staged, uint32_t warps) {
-    if (lanes == 1) {
-        const bool walk = noise && staged;
-        return dev::walk_head_bytes(walk) +
-               dev::walk_warp_bytes(walk, staged, dev::walk_lattice_columns(static_cast<int>(warps))) * warps;
-    }
+// Dynamic shared memory of the lane-group kernels.
+size_t generate_smem_bytes(uint32_t P, int lanes, int ppt, bool noise, uint32_t warps) {
     const size_t per_warp = sizeof(uint32_t) * dev::kRecFields * 32u + sizeof(float4) * 32u / lanes * lanes * ppt +
                             (noise ? sizeof(float2) * 384u : 0u);
     return sizeof(float4) * dev::kTableFloat4 + sizeof(float) * ((P + 3u) & ~3u) + per_warp * warps;
@@ -957,7 +822,8 @@ uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
-                         cudaStream_t stream, float *vec3_points, const nxg_classic_apply_desc *classic) {
+                         uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
+                         const nxg_classic_apply_desc *classic) {
     set_last_cuda_error(0);
     const uint32_t P = params.cvs_per_strand;
     const WorkspaceLayout ws = workspace_layout(asset.header.guide_count, count, P);
@@ -981,7 +847,8 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     }
     const int sms = device_sm_count();
     uint32_t status = NXG_ERROR_NONE;
-    if (!parallel_path(asset.header.guide_count, P)) {
+    const bool parallel = parallel_path(asset.header.guide_count, P);
+    if (!parallel && (!long_walk_path(asset.header.guide_count, count, P) || workspace_bytes < ws.wanted)) {
         const uint32_t threads = 128u;
         const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + threads - 1u) / threads,
                                                                           static_cast<uint64_t>(sms) * 8u));
@@ -992,7 +859,6 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     }
     auto *offsets = reinterpret_cast<float4 *>(wbase + ws.offsets);
     g.guide_frames = offsets + uint64_t{asset.header.guide_count} * P;
-    g.zero_row = asset.header.guide_count * (P + 2u);
     {
         const uint64_t n = uint64_t{asset.header.guide_count} * P;
         const uint32_t threads = 256u;
@@ -1001,29 +867,17 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
         dev::guide_offsets_kernel<<<blocks, threads, 0, stream>>>(g.a, g.f, P, g.p.support_scale, offsets);
         if ((status = record_cuda(cudaGetLastError()))) { return status; }
     }
-    int lanes = 32, ppt = 4;
-    uint32_t tile_block = 0u;
     const bool noise = g.p.noise != 0u;
-    default_tile(P, noise, &lanes, &ppt, &tile_block);
-    if (lanes != 1 && (g.roots || g.root_uvs || g.point_counts)) {  // the lane-walk kernel writes its own
-        const uint32_t threads = 256u;
-        const uint32_t per_block = threads;  // one strand per thread
-        const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + per_block - 1u) / per_block,
-                                                                          static_cast<uint64_t>(sms) * 8u));
-        dev::strand_roots_kernel<<<blocks, threads, 0, stream>>>(g);
-        if ((status = record_cuda(cudaGetLastError()))) { return status; }
-    }
-    g.range_begin = 0u;
-    g.range_end = count;
+    const bool classic_scalars = g.scalars != nullptr;
     int device = 0, smem_optin = 48 * 1024;
     if (cudaGetDevice(&device) == cudaSuccess) {
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     }
-    // Launches `fn` persistently over the order positions [g.range_begin,
-    // g.range_end).  block_size in [1, 1024] is a request: rounded up to whole
-    // warps, then capped at what the kernel's registers and shared memory
-    // (smem(warps) bytes) can launch.
-    auto launch = [&](auto fn, uint32_t requested, auto smem) -> uint32_t {
+    // Launches `fn` persistently over the strand order, `per_warp` strands per
+    // warp at a time.  `requested` threads are rounded up to whole warps, then
+    // capped at what the kernel's registers and shared memory (smem(warps)
+    // bytes) can launch.
+    auto launch = [&](auto fn, uint32_t requested, uint32_t per_warp, auto smem) -> uint32_t {
         cudaFuncAttributes attr{};
         uint32_t st = record_cuda(cudaFuncGetAttributes(&attr, reinterpret_cast<const void *>(fn)));
         if (st) { return st; }
@@ -1043,19 +897,46 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
                                                                        static_cast<int>(block), shm));
         if (st) { return st; }
         per_sm = std::max(per_sm, 1);
-        const uint64_t n = g.range_end - g.range_begin;
-        const uint64_t needed = (n + 32u * warps - 1u) / (32u * warps);
+        const uint64_t needed = (uint64_t{count} + per_warp * warps - 1u) / (uint64_t{per_warp} * warps);
         const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(needed, static_cast<uint64_t>(sms) * per_sm));
         return grid ? launch_kernel(fn, grid, block, shm, stream, g, offsets) : NXG_ERROR_NONE;
     };
-    const uint32_t requested = tile_block ? tile_block : config.block_size;
-    const bool classic_scalars = g.scalars != nullptr;
-    if (lanes == 1 && noise && !classic_scalars && requested <= 64u) {  // producer/consumer warp pairs
-        return launch(dev::generate_pipe_kernel, 64u, [](uint32_t) { return dev::kPipeSmemBytes; });
+    // The lane walk, unless a lane-group tile is registered for these strands.
+    const uint32_t packed = registered_tile(P, noise);
+    if (packed == 0u || (packed & 0xffu) == 1u) {
+        uint32_t warps = packed ? std::max(1u, (packed >> 16) & 0xffu) : (noise ? dev::kWalkNoiseWarps : 8u);
+        g.batch = 32u;
+        if (packed == 0u) {
+            // A call that does not fill the GPU spreads over it: fewer strands
+            // per warp (a warp's time is mostly the walk along one strand,
+            // which they share, plus what it does strand by strand), then
+            // fewer warps per CTA.
+            const uint64_t slots = static_cast<uint64_t>(sms) * 4u;  // one warp per scheduler
+            while (g.batch > 8u && (uint64_t{count} + g.batch - 1u) / g.batch < slots) { g.batch /= 2u; }
+            const uint64_t needed = (uint64_t{count} + g.batch - 1u) / g.batch;
+            warps = static_cast<uint32_t>(std::min<uint64_t>(warps, (needed + sms - 1u) / sms));
+        }
+        const auto fn = noise ? (classic_scalars ? dev::generate_walk_kernel<true, true>
+                                                 : dev::generate_walk_kernel<true, false>)
+                              : (classic_scalars ? dev::generate_walk_kernel<false, true>
+                                                 : dev::generate_walk_kernel<false, false>);
+        return launch(fn, warps * 32u, g.batch, [&](uint32_t w) {
+            return dev::walk_head_bytes(noise, P, w) + dev::walk_warp_bytes(noise, classic_scalars) * w;
+        });
     }
-    const bool staged = lanes == 1 ? noise : (noise || classic_scalars);
-    return launch(pick_kernel(lanes, ppt, noise, classic_scalars), requested,
-                  [&](uint32_t w) { return generate_smem_bytes(P, lanes, ppt, noise, staged, w); });
+    int lanes = 32, ppt = 4;
+    uint32_t tile_block = 0u;
+    default_tile(P, noise, &lanes, &ppt, &tile_block);
+    if (g.roots || g.root_uvs || g.point_counts) {  // the lane-walk kernel writes its own
+        const uint32_t threads = 256u;
+        const uint32_t per_block = threads;  // one strand per thread
+        const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + per_block - 1u) / per_block,
+                                                                          static_cast<uint64_t>(sms) * 8u));
+        dev::strand_roots_kernel<<<blocks, threads, 0, stream>>>(g);
+        if ((status = record_cuda(cudaGetLastError()))) { return status; }
+    }
+    return launch(pick_kernel(lanes, ppt, noise, classic_scalars), tile_block ? tile_block : config.block_size, 32u,
+                  [&](uint32_t w) { return generate_smem_bytes(P, lanes, ppt, noise, w); });
 }
 
 uint32_t validate_range_request(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1094,7 +975,7 @@ extern "C" {
 uint64_t nxg_packed_workspace_size(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
                                    uint32_t strand_count) {
     if (!asset || !params || strand_count == 0u) { return 0u; }
-    return nxg::workspace_layout(asset->header.guide_count, strand_count, params->cvs_per_strand).total;
+    return nxg::workspace_layout(asset->header.guide_count, strand_count, params->cvs_per_strand).wanted;
 }
 
 uint32_t nxg_generate_packed(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1129,8 +1010,8 @@ uint32_t nxg_generate_packed_range(const nxg_device_asset_desc *asset, const nxg
     const nxg_deformed_desc none{};
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
-                                config ? *config : default_config, first_strand, strand_count, workspace, s,
-                                nullptr, nullptr);
+                                config ? *config : default_config, first_strand, strand_count, workspace,
+                                workspace_bytes, s, nullptr, nullptr);
 }
 
 uint32_t nxg_prepare_strand_order(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
@@ -1173,7 +1054,7 @@ uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset, const n
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
-                                static_cast<cudaStream_t>(stream), nullptr, nullptr);
+                                workspace_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr);
 }
 
 uint32_t nxg_query_strand_states(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1225,7 +1106,6 @@ uint32_t nxg_query_walk_states(const nxg_device_asset_desc *asset, const nxg_def
     g.count = 0xffffffffu;  // strand ids are global: every id is a valid order entry
     g.order = strands;
     g.guide_frames = offsets + uint64_t{asset->header.guide_count} * P;
-    g.zero_row = asset->header.guide_count * (P + 2u);
     nxg::set_last_cuda_error(0);
     const uint64_t n = uint64_t{asset->header.guide_count} * P;
     const uint32_t threads = 256u;
@@ -1293,7 +1173,31 @@ uint32_t nxg_autotune_packed(const nxg_device_asset_desc *asset, const nxg_defor
     nxg_tile winner{0u, 0u, 0u};
     float winner_ms = 0.0f;
     const uint32_t reps = std::max(1u, repeats);
-    const uint32_t blocks[5] = {64u, 128u, 256u, 320u, 352u};
+    const auto time = [&](float *ms) -> uint32_t {  // with the tile registered now
+        uint32_t e = NXG_ERROR_NONE;
+        for (uint32_t r = 0; r <= reps; ++r) {  // one to warm up
+            if (r == 1u && (e = nxg::record_cuda(cudaEventRecord(start, s)))) { return e; }
+            if ((e = nxg_generate_packed_ordered(asset, deformed, params, output, &config, first_strand, strand_count,
+                                                 workspace, workspace_bytes, stream))) {
+                return e;
+            }
+        }
+        if ((e = nxg::record_cuda(cudaEventRecord(stop, s))) || (e = nxg::record_cuda(cudaEventSynchronize(stop))) ||
+            (e = nxg::record_cuda(cudaEventElapsedTime(ms, start, stop)))) {
+            return e;
+        }
+        *ms /= static_cast<float>(reps);
+        return NXG_ERROR_NONE;
+    };
+    // Strands too long for a registered lane-walk tile: nothing registered
+    // (the lane walk) is a candidate too.
+    bool unregistered = P > nxg::kMaxLaneWalkTile;
+    if (unregistered) {
+        nxg_set_tile(P, noise ? 1u : 0u, nullptr);
+        error = nxg_get_tile(P, noise ? 1u : 0u, &winner);
+        if (!error) { error = time(&winner_ms); }
+    }
+    const uint32_t blocks[5] = {64u, 128u, 256u, 384u, 512u};
     for (uint32_t lanes = 1u; lanes <= 32u && !error; lanes *= 2u) {
         for (uint32_t ppt = 1u; ppt <= 4u && !error; ppt *= 2u) {
             // tiles that hold the strand without idling half of their lanes
@@ -1301,23 +1205,12 @@ uint32_t nxg_autotune_packed(const nxg_device_asset_desc *asset, const nxg_defor
             for (const uint32_t block : blocks) {
                 const nxg_tile tile{lanes, ppt, block};
                 nxg_set_tile(P, noise ? 1u : 0u, &tile);
-                error = nxg_generate_packed_ordered(asset, deformed, params, output, &config, first_strand,
-                                                    strand_count, workspace, workspace_bytes, stream);
-                if (error) { break; }
-                if ((error = nxg::record_cuda(cudaEventRecord(start, s)))) { break; }
-                for (uint32_t r = 0; r < reps && !error; ++r) {
-                    error = nxg_generate_packed_ordered(asset, deformed, params, output, &config, first_strand,
-                                                        strand_count, workspace, workspace_bytes, stream);
-                }
-                if (error) { break; }
-                if ((error = nxg::record_cuda(cudaEventRecord(stop, s)))) { break; }
-                if ((error = nxg::record_cuda(cudaEventSynchronize(stop)))) { break; }
                 float ms = 0.0f;
-                if ((error = nxg::record_cuda(cudaEventElapsedTime(&ms, start, stop)))) { break; }
-                ms /= static_cast<float>(reps);
+                if ((error = time(&ms))) { break; }
                 if (winner.lanes_per_strand == 0u || ms < winner_ms) {
                     winner = tile;
                     winner_ms = ms;
+                    unregistered = false;
                 }
             }
         }
@@ -1328,7 +1221,7 @@ uint32_t nxg_autotune_packed(const nxg_device_asset_desc *asset, const nxg_defor
         nxg::g_tiles[P][noise ? 1 : 0].store(saved, std::memory_order_relaxed);
         return error ? error : NXG_ERROR_INVALID_ARGUMENT;
     }
-    nxg_set_tile(P, noise ? 1u : 0u, &winner);
+    nxg_set_tile(P, noise ? 1u : 0u, unregistered ? nullptr : &winner);
     if (best) { *best = winner; }
     if (best_ms) { *best_ms = winner_ms; }
     return NXG_ERROR_NONE;
@@ -1390,7 +1283,7 @@ extern "C" uint32_t nxg_generate_motion_packed(const nxg_device_asset_desc *asse
     }
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, outputs[i], cfg, 0u,
-                                     params->strand_count, workspace, s, nullptr, nullptr);
+                                     params->strand_count, workspace, workspace_bytes, s, nullptr, nullptr);
     }
     return error;
 }
@@ -1420,7 +1313,7 @@ extern "C" uint32_t nxg_generate_motion(const nxg_device_asset_desc *asset, cons
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         float *dst = reinterpret_cast<float *>(output->points) + per_sample * i;
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, none, cfg, 0u, params->strand_count,
-                                     workspace, s, dst, nullptr);
+                                     workspace, workspace_bytes, s, dst, nullptr);
     }
     return error;
 }
@@ -1515,7 +1408,8 @@ extern "C" uint32_t nxg_generate_packed_static_scratch(const nxg_device_asset_de
                                                       const nxg_launch_config *config, void *stream) {
     const uint32_t error = nxg_validate_packed_request(asset, deformed, params, output, config);
     if (error != NXG_ERROR_NONE) { return error; }
-    if (nxg_packed_workspace_size(asset, params, params->strand_count) > NXG_STATIC_SCRATCH_BYTES) {
+    if (nxg::workspace_layout(asset->header.guide_count, params->strand_count, params->cvs_per_strand).total >
+        NXG_STATIC_SCRATCH_BYTES) {
         return NXG_ERROR_STATIC_SCRATCH_LIMIT;
     }
     void *scratch = nullptr;

@@ -27,8 +27,7 @@ struct LaunchArgs {
     ParamArgs p;
     uint32_t first_strand;   // global id of output record 0
     uint32_t count;          // strands in this launch
-    uint32_t range_begin;    // lane-walk kernels: positions [range_begin, range_end) of the order
-    uint32_t range_end;
+    uint32_t batch;          // lane-walk kernels: strands a warp takes at a time, at most 32
     float4 *points;
     float *vec3_points;      // when set: sample-major Vec3 output instead of float4 (motion contract)
     uint32_t *roots;         // 12 words per strand, or nullptr
@@ -36,7 +35,6 @@ struct LaunchArgs {
     uint32_t *point_counts;
     const uint32_t *order;   // permutation of [0, count), or nullptr for identity
     const float4 *guide_frames;  // 2 per guide (guide_frame_entry), or nullptr
-    uint32_t zero_row;           // offset-table index of kWalkMaxCvs zero entries (unused lane-walk slots)
     const float2 *scalars;   // Classic per-root (length scale, width), or nullptr
     uint32_t classic_length; // scale each strand about its first point by scalars.x
     uint32_t classic_width;  // radius = 0.5 * max(scalars.y, 0) * radius_scale
@@ -637,6 +635,7 @@ uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
-                         cudaStream_t stream, float *vec3_points, const nxg_classic_apply_desc *classic);
+                         uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
+                         const nxg_classic_apply_desc *classic);
 
 } // namespace nxg

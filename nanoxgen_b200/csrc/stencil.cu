@@ -79,34 +79,7 @@ __device__ __forceinline__ void insert_candidate(Candidate (&best)[kSlots], Cand
 // same differences, so they can differ by rounding only (a few ulps, about
 // 2^-21 relative); the margin is 2^-16, so no guide the host keeps is ever
 // skipped, and a packed value that is too small only lets a group through.
-typedef unsigned long long f32x2;
 constexpr float kFilterMargin = 0.9999847412109375f;  // 1 - 2^-16
-
-__device__ __forceinline__ f32x2 pair(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpair(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 
 struct GuideTile {
     float x[kStencilTile], y[kStencilTile], z[kStencilTile];  // roots, one plane per axis
@@ -162,9 +135,9 @@ __device__ __forceinline__ void begin_triangle(TriangleSearch &t, uint32_t ti, c
             row[1] = make_uint4(kInvalid, kInvalid, kInvalid, kInvalid);
         }
     }
-    t.cx = pair(t.centroid.x, t.centroid.x);
-    t.cy = pair(t.centroid.y, t.centroid.y);
-    t.cz = pair(t.centroid.z, t.centroid.z);
+    t.cx = pair2(t.centroid.x, t.centroid.x);
+    t.cy = pair2(t.centroid.y, t.centroid.y);
+    t.cz = pair2(t.centroid.z, t.centroid.z);
 #pragma unroll
     for (uint32_t k = 0; k < kSlots; ++k) { t.best[k] = {0.0f, kInvalid}; }
 }
@@ -178,8 +151,8 @@ __device__ __forceinline__ void consider_group(TriangleSearch &t, const GuideTil
     const f32x2 dx0 = sub2(t.cx, gx.x), dx1 = sub2(t.cx, gx.y);
     const f32x2 dy0 = sub2(t.cy, gy.x), dy1 = sub2(t.cy, gy.y);
     const f32x2 dz0 = sub2(t.cz, gz.x), dz1 = sub2(t.cz, gz.y);
-    const float2 a = unpair(add2(add2(mul2(dx0, dx0), mul2(dy0, dy0)), mul2(dz0, dz0)));
-    const float2 b = unpair(add2(add2(mul2(dx1, dx1), mul2(dy1, dy1)), mul2(dz1, dz1)));
+    const float2 a = unpair2(add2(add2(mul2(dx0, dx0), mul2(dy0, dy0)), mul2(dz0, dz0)));
+    const float2 b = unpair2(add2(add2(mul2(dx1, dx1), mul2(dy1, dy1)), mul2(dz1, dz1)));
     const float low = fminf(fminf(a.x, a.y), fminf(b.x, b.y));
     if (t.best[kSlots - 1].key < low * kFilterMargin) { return; }
     // The group passed: each guide is checked on its own packed value before

@@ -79,6 +79,43 @@ __device__ __forceinline__ F3 normalize(F3 v) {
     return l2 > 1.0e-20f ? v * rsqrtf(l2) : F3{0.0f, 1.0f, 0.0f};
 }
 
+// Pairs of floats in one 64-bit register pair (sm_100a f32x2 arithmetic): one
+// issued instruction for two IEEE operations.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f32x2 both2(float v) { return pair2(v, v); }
+__device__ __forceinline__ float2 unpair2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ float low2(f32x2 v) { return unpair2(v).x; }
+__device__ __forceinline__ float high2(f32x2 v) { return unpair2(v).y; }
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 __device__ __forceinline__ F3 ld3(const float *p, uint32_t i) {
     const float *q = p + 3u * static_cast<uint64_t>(i);
     return {__ldg(q), __ldg(q + 1), __ldg(q + 2)};
@@ -229,10 +266,14 @@ __device__ __forceinline__ void frame_guide(const AssetArgs &a, const FrameArgs 
 }
 
 // Per-frame guide record for the lane-walk generator: (guide root, support
-// radius * support_scale) and (guide normal, 1), or a zero second word for a
-// corrupt record (first CV past the CV array).
+// radius * support_scale) and (guide normal, flags), the flags zero for a
+// corrupt record (first CV past the CV array).  `lead`: the guide's offset at
+// its first CV, whose being zero means that a strand's first base point is
+// its root exactly.
+enum : uint32_t { kGuideValid = 1u, kGuideLead = 2u };
+
 __device__ __forceinline__ void guide_frame_entry(const AssetArgs &a, const FrameArgs &f, float support_scale,
-                                                  uint32_t gi, float4 *out) {
+                                                  uint32_t gi, float4 lead, float4 *out) {
     const uint32_t *g = a.guides + 14u * static_cast<uint64_t>(gi);
     const uint32_t first = __ldg(g + 0);
     if (first >= a.guide_cv_count) {
@@ -249,7 +290,8 @@ __device__ __forceinline__ void guide_frame_entry(const AssetArgs &a, const Fram
     frame_guide(a, f, first, __ldg(g + 2), __uint_as_float(__ldg(g + 4)), __uint_as_float(__ldg(g + 5)), rest_root,
                 rest_normal, groot, gnormal);
     out[0] = make_float4(groot.x, groot.y, groot.z, __fmul_rn(support, support_scale));
-    out[1] = make_float4(gnormal.x, gnormal.y, gnormal.z, __uint_as_float(1u));
+    const bool zero = lead.x == 0.0f && lead.y == 0.0f && lead.z == 0.0f;
+    out[1] = make_float4(gnormal.x, gnormal.y, gnormal.z, __uint_as_float(kGuideValid | (zero ? 0u : kGuideLead)));
 }
 
 __device__ __forceinline__ Slot eval_slot(const AssetArgs &a, const FrameArgs &f, const ParamArgs &p,
@@ -380,8 +422,9 @@ __device__ __forceinline__ uint32_t temper_index(uint32_t s) {
 __device__ __forceinline__ float s_curve(float t) { return t * t * t * (t * (t * 6.0f - 15.0f) + 10.0f); }
 
 // generate.h:370-402 gradient_noise over a shared-memory copy of the asset's
-// gradient table (float4-padded).
-__device__ __forceinline__ float gradient_noise(const float4 *table, float x, float y, float z) {
+// gradient table (float4-padded, entry e at e << shift).
+__device__ __forceinline__ float gradient_noise(const float4 *table, float x, float y, float z,
+                                                uint32_t shift = 0u) {
     const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
     const int32_t ix = static_cast<int32_t>(fx), iy = static_cast<int32_t>(fy), iz = static_cast<int32_t>(fz);
     const float wx = x - fx, wy = y - fy, wz = z - fz;
@@ -392,7 +435,7 @@ __device__ __forceinline__ float gradient_noise(const float4 *table, float x, fl
     for (uint32_t corner = 0u; corner < 8u; ++corner) {
         const uint32_t ox = corner & 1u, oy = (corner >> 1u) & 1u, oz = (corner >> 2u) & 1u;
         const uint32_t seed = base + (ox ? kLcgA2 : 0u) + (oy ? kLcgA : 0u) + oz;
-        const float4 g = table[temper_index(seed)];
+        const float4 g = table[temper_index(seed) << shift];
         v[corner] = g.x * (wx - static_cast<float>(ox)) + g.y * (wy - static_cast<float>(oy)) +
                     g.z * (wz - static_cast<float>(oz));
     }

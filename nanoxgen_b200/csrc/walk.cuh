@@ -1,30 +1,47 @@
-// walk.cuh -- the lane-walk generator for strands of 2..32 CVs.
+// walk.cuh -- the lane-walk generator, for strands of any CV count whose
+// guide-offset table fits the workspace.
 //
-// A warp takes 32 strands of the strand order at a time, in four steps:
+// A warp takes up to 32 strands of the strand order at a time:
 //
-//   setup  (lane = strand)  root sample, the eight stencil slots and the
-//                           blend mode, folded into one weighted-sum record;
-//   base   (lane = CV)      the base curve from the guide-offset table, read
-//                           as coalesced rows (consecutive lanes on
-//                           consecutive CVs of one guide), into a stage in
-//                           shared memory, one row of 32 xyz slots per strand;
-//   frame  (lane = strand)  with noise: the arc-length prefix, the strand's
-//                           noise lattice, then the reference's cursor walk
-//                           (generate.h:445-502) over the staged row -- the
-//                           transported normal is a serial recurrence, so a
-//                           lane carries it CV by CV with the reference's
-//                           rotation applied as a vector update, and no
-//                           matrix products or cross-lane scans are needed;
-//   store  (8 lanes/strand) the strands' float4s as coalesced streaming
-//                           stores; with per-root Classic scalars, a step
-//                           with lane = strand first takes each strand's
-//                           Classic values (scale, width, drop rule) once.
+//   setup  (lane = strand)   root sample, the eight stencil slots and the
+//                            blend mode, folded into one weighted-sum record;
+//   base   (8 lanes/strand)  the base curve from the guide-offset table, read
+//                            as coalesced rows (consecutive lanes on
+//                            consecutive CVs of one guide): straight to the
+//                            output without noise, else a chunk of 16 CVs per
+//                            strand into a stage in shared memory;
+//   frame  (lane = strand)   with noise: the reference's cursor walk
+//                            (generate.h:445-502) over the staged chunk --
+//                            the transported normal is a serial recurrence,
+//                            so a lane carries it CV by CV with the
+//                            reference's rotation applied as a vector update,
+//                            and no matrix products or cross-lane scans are
+//                            needed; the noise comes from a window of lattice
+//                            columns that moves along the strand;
+//   store  (8 lanes/strand)  the chunk's float4s as coalesced streaming
+//                            stores; preserveLength on strands of more than
+//                            one chunk and Classic scalars are applied to the
+//                            written points afterwards, from L2.
 //
-// Stage rows are 97 words apart and a CV takes 3 words; both strides are odd,
+// What bounds the noisy walk: of 1,000,000 strands x 32 CVs, separately built
+// variants put about 120 us each on the walk itself (near the issue rate),
+// the lattice (shared-memory wavefronts of random table reads) and the base
+// rows (latency of L1 and L2), 60 on the stencil slots and 60 on the stores.
+// So a strand is not staged whole: chunks of 16 CVs and a moving window of
+// five lattice columns keep a warp at 13 KB of shared memory instead of 20,
+// the L1 at 60 KB instead of 28 for the base rows, and any CV count on the
+// same path; the base step requests sixteen rows' entries before it uses one;
+// and the gradient table is held eight times, free of bank conflicts.
+// Twelve warps at 168 registers; sixteen at 128 spilled (729 us).  1,000,000 x
+// 32: 601 us staged whole with all columns, 526 us now; 150,001 x 61: 419 us
+// on lane groups with scans, 228 us; 20,011 x 160: 1,241 us on one thread per
+// strand, 121 us.
+//
+// Stage rows are 49 words apart and a CV takes 3 words; both strides are odd,
 // so a warp reading column c of 32 rows (frame step) and a warp reading one
 // row are free of shared-memory bank conflicts, and the eight-lane base and
 // store steps (four strands of eight CVs per access) meet at most two lanes
-// to a bank (97 = 1 mod 32 shifts each strand's banks by one).
+// to a bank.
 #pragma once
 
 #include "generator_core.cuh"
@@ -32,45 +49,52 @@
 namespace nxg {
 namespace dev {
 
-constexpr int kWalkMaxCvs = 32;
-constexpr int kWalkRowFloats = 3 * kWalkMaxCvs + 1; // a row holds x, y, z per CV (97 words: an odd stride)
-constexpr int kWalkAxisColumns = 12;           // noise lattice columns per axis and strand, at most
-constexpr int kWalkRecords = 8;                // float4 setup records per strand
+constexpr int kWalkChunk = 16;                     // CVs staged at a time
+constexpr int kWalkRowFloats = 3 * kWalkChunk + 1;  // a row holds x, y, z per CV (49 words: an odd stride)
+// Noise lattice columns per axis and strand.  Five cover four lattice cells; a
+// walk crosses a cell every five or six CVs at the sizes grooms use, so a
+// strand refills its window about once (four columns: 533 us against 526 on
+// 1,000,000 strands x 32).
+constexpr int kWalkWindow = 5;
+constexpr int kWalkRecords = 6;                    // float4 setup records per strand
+constexpr int kWalkClassicRecords = 8;             // with the Classic values of walk_classic_setup
+constexpr int kWalkNoiseWarps = 12;                // warps of a full noise CTA
 
-// Shared-memory bytes per warp.  Staged variants (noise or Classic scalars):
-// stage | records (aliased by the lattice once the base step has read them) |
-// output words; the RootSample words use the stage.  The plain variant has no
-// stage -- its base step writes the output directly -- so: records | RootSample
-// words | output words.
+// Copies (log2) of the gradient table in a noise CTA's shared memory, entry e
+// of copy k at (e << copies) + k.  With eight, a lane reads copy lane % 8, so
+// the eight lanes that a 16-byte shared load serves at a time sit in eight
+// different bank groups whatever entries they want (4 wavefronts per warp;
+// with one copy, eight random entries in eight bank groups, 11.6): 1,000,000
+// strands x 32 CVs 574 -> 551 us.  A CTA of a few warps runs too few strands
+// to pay for the copies (2,000 strands x 16: 14.2 us with one, 15.5 with eight).
+__host__ __device__ constexpr uint32_t walk_table_copies(uint32_t warps) { return warps >= 8u ? 3u : 0u; }
+
+// Shared-memory bytes per warp.  With noise: stage | lattice window | records
+// | output words.  Without (the base step writes the output directly):
+// records | output words.
 constexpr size_t kWalkStageBytes = sizeof(float) * 32u * kWalkRowFloats;
+constexpr size_t kWalkLatticeBytes = sizeof(float2) * 3u * kWalkWindow * 32u;
 constexpr size_t kWalkRecordBytes = sizeof(float4) * kWalkRecords * 32u;
-constexpr size_t kWalkLatticeBytes = sizeof(float2) * 3u * kWalkAxisColumns * 32u;
-// Lattice columns per axis and strand for a CTA of `warps` noise warps:
-// twelve up to ten warps; ten for eleven-warp CTAs, whose shared memory holds
-// no more.  A strand needs floor(d + span) - floor(d) + 2 columns on an axis
-// whose noise coordinate starts at d and advances by span over the strand
-// (at most ceil(span) + 2); a warp with a strand that needs more takes direct
-// noise.
-__host__ __device__ constexpr int walk_lattice_columns(int warps) { return warps > 10 ? 10 : kWalkAxisColumns; }
-__host__ __device__ constexpr size_t walk_lattice_bytes(int columns) {
-    return sizeof(float2) * 3u * static_cast<size_t>(columns) * 32u;
-}
-constexpr size_t kWalkRootWordBytes = sizeof(uint32_t) * 12u * 32u;
+constexpr size_t kWalkClassicRecordBytes = sizeof(float4) * kWalkClassicRecords * 32u;
 constexpr size_t kWalkLocalBytes = sizeof(uint32_t) * 32u;
-__host__ __device__ constexpr size_t walk_warp_bytes(bool noise, bool staged, int columns = kWalkAxisColumns) {
-    return staged ? kWalkStageBytes +
-                        (noise && walk_lattice_bytes(columns) > kWalkRecordBytes ? walk_lattice_bytes(columns)
-                                                                                 : kWalkRecordBytes) +
-                        kWalkLocalBytes
-                  : kWalkRecordBytes + kWalkRootWordBytes + kWalkLocalBytes;
+__host__ __device__ constexpr size_t walk_warp_bytes(bool noise, bool classic) {
+    return (noise ? kWalkStageBytes + kWalkLatticeBytes + kWalkRecordBytes
+                  : (classic ? kWalkClassicRecordBytes : kWalkRecordBytes)) +
+           kWalkLocalBytes;
 }
-// Per CTA, before the warps: gradient table (noise) | t values | radii.
-__host__ __device__ constexpr size_t walk_head_bytes(bool noise) {
-    return (noise ? sizeof(float4) * kTableFloat4 : 0u) + 2u * sizeof(float) * kWalkMaxCvs;
+// Per CTA, before the warps: gradient table (noise) | t values | radii, each
+// of P values and padding to a multiple of four (walk_pair reads t in pairs).
+__host__ __device__ constexpr uint32_t walk_padded(uint32_t P) { return (P + 4u) & ~3u; }
+__host__ __device__ constexpr size_t walk_head_bytes(bool noise, uint32_t P, uint32_t warps) {
+    return (noise ? sizeof(float4) * (kTableFloat4 << walk_table_copies(warps)) : 0u) +
+           2u * sizeof(float) * walk_padded(P);
 }
+// Longest strand the walk takes (its t values and radii are in shared memory).
+constexpr uint32_t kWalkMaxCvs = 1024u;
 
 // Record q of strand s lives at records[q * 32 + s]:
-//   q = 0..3  (row of slot 2q, weight, row of slot 2q+1, weight); a row is
+//   q = 0..3  (row of slot 2q, weight, row of slot 2q+1, weight) of the
+//             strand's weighted slots, zeros past its count; a row is
 //             guide * P, the guide's first entry in the offset table
 //   q = 4     (root position, 1 / weight sum)
 //   q = 5     (root normal in normal mode else 0, slot count as bits)
@@ -81,15 +105,24 @@ __host__ __device__ constexpr size_t walk_head_bytes(bool noise) {
 //   base = root + (inv * sum_j w_j offsets[row_j + c] + normal' * t_c) * length_scale.
 // Square root by the PTX approximate instruction (one MUFU operation, no
 // special-case branch); its relative error (below 2^-22) is far inside the
-// position tolerance where it is used (arc lengths, sin(acos x), blend weights).
+// position tolerance where it is used (arc lengths, sin(acos x)), and
+// arguments below 2^-126 (lengths below 2^-63) read as zero.
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// 1 / sqrt(x) by one MUFU operation, for x that is a normal float: the value
+// rsqrtf gives there, without its scaling of subnormal arguments.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
 struct WalkRoot {
     F3 position, normal, surface_u, domain;
+    bool lead;  // the first base point may not be the root exactly (kGuideLead)
 };
 
 // sample_root (generate.h:101-135) plus, with noise, the root's surface_u
@@ -241,9 +274,7 @@ __device__ __forceinline__ void walk_store_root(uint32_t *roots, uint32_t local,
 // the loop of generate.h:214-244 with the frame's guide roots, normals and
 // support radii read from the per-frame guide records.  With `outputs`,
 // also writes the strand's RootSample, root UV and point count.  With
-// `decision` (inspection only), also reports the choices made.  Slots past
-// the strand's count point at the frame's zero row with weight 0, so the
-// base step may read any slot of the four records.
+// `decision` (inspection only), also reports the choices made.
 template <bool NOISE>
 __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *records, uint32_t *locals, int lane,
                                                uint32_t pick, bool valid, uint32_t P, bool outputs = true,
@@ -251,13 +282,14 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
     const AssetArgs &a = g.a;
     const FrameArgs &f = g.f;
     const ParamArgs &p = g.p;
-    uint32_t local = __ldg(g.order + pick);
+    uint32_t local = g.order != nullptr ? __ldg(g.order + pick) : pick;
     if (local >= g.count) {
         local = 0u;
         valid = false;
     }
     WalkRoot r;
     r.surface_u = F3{0.0f, 0.0f, 0.0f};
+    r.lead = false;
     F3 rest_position = {0.0f, 0.0f, 0.0f};
     const Root root = walk_root<NOISE>(a, f, p.seed, g.first_strand + local, r.surface_u, rest_position);
     if (outputs && valid) {  // generate.h:621-623
@@ -265,9 +297,8 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
         if (g.root_uvs) { g.root_uvs[local] = make_float2(root.u, root.v); }
         if (g.point_counts) { g.point_counts[local] = P; }
     }
-    const float zero_row = __uint_as_float(g.zero_row);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) { records[q * 32 + lane] = make_float4(zero_row, 0.0f, zero_row, 0.0f); }
+    for (int q = 0; q < 4; ++q) { records[q * 32 + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
     uint32_t stencil[kSlots];
     const uint32_t *row = a.stencil + static_cast<uint64_t>(root.triangle) * kSlots;
     if ((reinterpret_cast<std::uintptr_t>(a.stencil) & 15u) == 0u) {
@@ -281,9 +312,10 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
     }
     float *slot_words = reinterpret_cast<float *>(records);
     // Guide frame record of slot j (an out-of-range slot reads as a corrupt
-    // record: no slot).  With noise (fewer warps per SM to hide latency) all
-    // eight are requested before any is used; without, one at a time, which
-    // keeps the register count and the occupancy of the plain kernel.
+    // record: no slot).  With noise (fewer warps per SM to hide latency) four
+    // are requested before any is used; without, one at a time, which keeps
+    // the register count and the occupancy of the plain kernel.
+    constexpr uint32_t kAhead = NOISE ? kSlots : 1u;
     float4 gr[kSlots], gn[kSlots];
     auto load_slot = [&](uint32_t j) {
         const bool in_range = stencil[j] != kInvalid && stencil[j] < a.guide_count;
@@ -296,10 +328,6 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
         }
         if (!in_range) { gn[j].w = 0.0f; }
     };
-    if constexpr (NOISE) {
-#pragma unroll
-        for (uint32_t j = 0; j < kSlots; ++j) { load_slot(j); }
-    }
     // Blend weights (1 - d / r)^power in fast arithmetic (they feed positions
     // only); d^2, the rejection test and the radius test that decide which
     // slots count stay in the reference's exact rounding.
@@ -310,8 +338,12 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
     uint32_t blended = 0u;
 #pragma unroll
     for (uint32_t j = 0; j < kSlots; ++j) {
-        if constexpr (!NOISE) { load_slot(j); }
+        if (j % kAhead == 0u) {
+#pragma unroll
+            for (uint32_t k = 0; k < kAhead; ++k) { load_slot(j + k); }
+        }
         if (__float_as_uint(gn[j].w) == 0u) { continue; }  // out of range or corrupt record
+        r.lead = r.lead || (__float_as_uint(gn[j].w) & kGuideLead) != 0u;
         const F3 delta = xsub(root.position, F3{gr[j].x, gr[j].y, gr[j].z});
         const float d2 = xdot(delta, delta);
         if (xdot(root.normal, F3{gn[j].x, gn[j].y, gn[j].z}) < p.rejection_cos) { continue; }
@@ -348,7 +380,7 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
     if (wsum > 1.0e-12f) {
         inv = 1.0f / wsum;
     } else if (nearest != kInvalid) {
-        records[lane] = make_float4(__uint_as_float(nearest * P), 1.0f, zero_row, 0.0f);
+        records[lane] = make_float4(__uint_as_float(nearest * P), 1.0f, 0.0f, 0.0f);
         nb = 1u;
         inv = 1.0f;
         mode = 1u;
@@ -384,8 +416,10 @@ __device__ __forceinline__ WalkRoot walk_setup(const LaunchArgs &g, float4 *reco
 
 // One output point of the strand whose output word is `word` (skipped when
 // the word is marked invalid): float4 (position, radius), or Vec3 positions,
-// 3P consecutive floats per strand (device_contract.h:47-52).
-__device__ __forceinline__ void walk_emit(const LaunchArgs &g, uint32_t word, int P, int c, float4 q) {
+// 3P consecutive floats per strand (device_contract.h:47-52).  `again`: the
+// point is read back soon, so it is stored without the streaming hint.
+__device__ __forceinline__ void walk_emit(const LaunchArgs &g, uint32_t word, int P, int c, float4 q,
+                                          bool again = false) {
     if (word >> 31) { return; }
     const uint64_t index = static_cast<uint64_t>(word) * static_cast<uint32_t>(P) + static_cast<uint32_t>(c);
     if (g.vec3_points) {
@@ -393,6 +427,8 @@ __device__ __forceinline__ void walk_emit(const LaunchArgs &g, uint32_t word, in
         __stcs(out3, q.x);
         __stcs(out3 + 1, q.y);
         __stcs(out3 + 2, q.z);
+    } else if (again) {
+        g.points[index] = q;
     } else {
         __stcs(g.points + index, q);
     }
@@ -406,12 +442,6 @@ __device__ __forceinline__ void stage_put(float *row, int c, F3 v) {
     row[3 * c] = v.x;
     row[3 * c + 1] = v.y;
     row[3 * c + 2] = v.z;
-}
-
-// Strand of a flattened (strand, CV) item: floor((item + 0.5) / P), exact for
-// item < 32 * 32 (the quotient is at least 0.5 / P from an integer).
-__device__ __forceinline__ int walk_strand(int item, float inv_p) {
-    return static_cast<int>((static_cast<float>(item) + 0.5f) * inv_p);
 }
 
 // Base point c of strand s from its records (generate.h:246-267, :300-310).
@@ -440,12 +470,10 @@ __device__ __forceinline__ F3 walk_base_point(const float4 *records, int s, int 
 // Classic scalars without noise (xgen_classic_runtime.cpp:1650-1678,
 // :1827-1858), for this lane's strand before its base step: the first and
 // last base points give the chord; a strand whose scaled chord is near the
-// 1e-4 threshold measures its sampled spline (lanes that need it take turns
-// on `scratch`, 32 float4); a dropped strand gets point count 0.  Leaves
-// records 6 and 7 for walk_base.  Every lane of the warp calls it.
+// 1e-4 threshold measures its sampled spline; a dropped strand gets point
+// count 0.  Leaves records 6 and 7 for walk_base_direct.
 __device__ __forceinline__ void walk_classic_setup(const LaunchArgs &g, float4 *records, int lane, bool valid,
-                                                   uint32_t local, const float *tvals, const float4 *offsets,
-                                                   float4 *scratch, int P) {
+                                                   uint32_t local, const float *tvals, const float4 *offsets, int P) {
     const ParamArgs &p = g.p;
     const float ls = p.length_scale;
     const float2 sc = __ldg(g.scalars + local);
@@ -456,16 +484,10 @@ __device__ __forceinline__ void walk_classic_setup(const LaunchArgs &g, float4 *
         : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
     bool keep = !(raw_width < 1.0e-4f);
     const F3 chord = back - front;
-    const bool measure = keep && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f);
-    for (unsigned todo = __ballot_sync(kFull, measure); todo != 0u; todo &= todo - 1u) {
-        if (lane == __ffs(todo) - 1) {
-            for (int c = 0; c < P; ++c) {
-                const F3 b = walk_base_point(records, lane, c, tvals[c], ls, offsets);
-                scratch[c] = make_float4(b.x, b.y, b.z, 0.0f);
-            }
-            keep = !(__fmul_rn(classic_spline_length(scratch, P), scale) < 1.0e-4f);
-        }
-        __syncwarp();
+    if (keep && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f)) {
+        keep = !(__fmul_rn(classic_spline_length_by(
+                               [&](int c) { return walk_base_point(records, lane, c, tvals[c], ls, offsets); }, P),
+                           scale) < 1.0e-4f);
     }
     const float radius = __fmul_rn(__fmul_rn(0.5f, raw_width < 0.0f ? 0.0f : raw_width), p.radius_scale);
     records[6 * 32 + lane] = make_float4(front.x, front.y, front.z, scale);
@@ -473,124 +495,171 @@ __device__ __forceinline__ void walk_classic_setup(const LaunchArgs &g, float4 *
     if (!keep && valid && g.point_counts != nullptr) { g.point_counts[local] = 0u; }
 }
 
-// Base step: item = s * P + c over the batch, 32 consecutive items per pass,
-// into the stage or (DIRECT) straight to the output; CLASSIC (with DIRECT)
-// applies records 6 and 7: scale about the first point, width override.
-template <bool DIRECT, bool CLASSIC = false>
-__device__ __forceinline__ void walk_base(const LaunchArgs &g, const float4 *records, float *stage,
-                                          const uint32_t *locals, const float *tvals, const float *rvals,
-                                          const float4 *offsets, int lane, int in_batch, int P, float inv_p) {
-    const int items = in_batch * P;
-    const float ls = g.p.length_scale;
-#pragma unroll 2
-    for (int item = lane; item < items; item += 32) {
-        const int s = walk_strand(item, inv_p);
-        const int c = item - s * P;
-        F3 base = walk_base_point(records, s, c, tvals[c], ls, offsets);
-        float radius = rvals[c];
-        if constexpr (CLASSIC) {
-            const float4 front = records[6 * 32 + s];
-            const float4 width = records[7 * 32 + s];
-            if (g.classic_length) { base = xadd(xyz(front), xmul(xsub(base, xyz(front)), front.w)); }
-            if (width.y != 0.0f) { radius = width.x; }
-        }
-        if constexpr (DIRECT) {
-            walk_emit(g, locals[s], P, c, make_float4(base.x, base.y, base.z, radius));
-        } else {
-            stage_put(stage + s * kWalkRowFloats, c, base);  // radii come from the t table at the store
-        }
-    }
+// An offset-table entry as two pairs, (x, y) and (z, unused).
+__device__ __forceinline__ ulonglong2 walk_offset(const float4 *offsets, uint32_t index) {
+    return __ldg(reinterpret_cast<const ulonglong2 *>(offsets) + index);
 }
 
 // Base step straight to the output (no noise).  Eight lanes per strand and
 // four strands per pass: lane (s = pass * 4 + lane / 8, c = lane % 8)
-// computes CVs c + 8m, m < ceil(P / 8).  One address per slot serves the
-// lane's loads (the other CVs sit at fixed distances along the guide's
-// offset row), every load of a warp instruction stays within one 128-byte
-// line per strand, and a lane's t values are fixed for the whole kernel.  A
+// computes CVs c + 8m of a block of 32 CVs, m < 4.  One address per slot
+// serves the lane's loads (the other CVs sit at fixed distances along the
+// guide's offset row), every load of a warp instruction stays within one
+// 128-byte line per strand, and a lane's t values are fixed for the block.  A
 // pass runs as many slot pairs as its strands' largest count; a strand's
 // loads past its own count are predicated off (no memory request), and its
-// records there hold the zero row with weight 0, so the accumulation needs
-// no predicate.  CLASSIC applies records 6 and 7 as walk_base does.  STAGED
-// writes the base points into the strands' stage rows instead of the output
-// (the noise walk reads them there); a stage row of 97 words keeps the
-// four strands of a pass at most two lanes to a bank.  Every lane of the
-// warp calls it.
-template <bool CLASSIC, bool STAGED = false>
+// weights there are zero.
+// CLASSIC applies records 6 and 7.  Every lane of the warp calls it.
+template <bool CLASSIC>
 __device__ __forceinline__ void walk_base_direct(const LaunchArgs &g, const float4 *records, const uint32_t *locals,
                                                  const float *tvals, const float *rvals, const float4 *offsets,
-                                                 int lane, int in_batch, int P, float *stage = nullptr) {
-    static_assert(!(CLASSIC && STAGED), "staged strands take the Classic application at the store");
-    constexpr int kPerLane = kWalkMaxCvs / 8;
-    const int c = lane & 7;
-    const int cpl = (P + 7) >> 3;
-    float tv[kPerLane];
-#pragma unroll
-    for (int m = 0; m < kPerLane; ++m) { tv[m] = tvals[min(c + 8 * m, P - 1)]; }
+                                                 int lane, int in_batch, int P) {
+    constexpr int kPerLane = 4;
     const float ls = g.p.length_scale;
-    const float4 *column = offsets + c;
-    for (int first = 0; first < in_batch; first += 4) {
-        const int s = first + (lane >> 3);
-        const bool live = s < in_batch;
-        const float4 head = records[4 * 32 + s];
-        const float4 tail = records[5 * 32 + s];
-        const uint32_t nb = live ? __float_as_uint(tail.w) : 0u;
-        const uint32_t pairs = __reduce_max_sync(kFull, (nb + 1u) >> 1);
-        F3 acc[kPerLane];
-        float4 da[kPerLane], db[kPerLane];
+    for (int block = 0; block < P; block += 8 * kPerLane) {
+        const int c = block + (lane & 7);
+        const int cpl = min((P - block + 7) >> 3, kPerLane);
+        float tv[kPerLane];
 #pragma unroll
-        for (int m = 0; m < kPerLane; ++m) {
-            acc[m] = F3{0.0f, 0.0f, 0.0f};
-            da[m] = db[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-        for (uint32_t q = 0; q < pairs; ++q) {
-            // A strand loads only its own slots: past its count the registers
-            // keep the last (finite) entries and the weights are zero.
-            const float4 gw = records[q * 32 + s];
-            const float4 *ra = column + __float_as_uint(gw.x);
-            const float4 *rb = column + __float_as_uint(gw.z);
-            const bool la = 2u * q < nb, lb = 2u * q + 1u < nb;
+        for (int m = 0; m < kPerLane; ++m) { tv[m] = tvals[min(c + 8 * m, P - 1)]; }
+        const float4 *column = offsets + c;
+        for (int first = 0; first < in_batch; first += 4) {
+            const int s = first + (lane >> 3);
+            const bool live = s < in_batch;
+            const float4 head = records[4 * 32 + s];
+            const float4 tail = records[5 * 32 + s];
+            const uint32_t nb = live ? __float_as_uint(tail.w) : 0u;
+            const uint32_t pairs = __reduce_max_sync(kFull, (nb + 1u) >> 1);
+            F3 acc[kPerLane];
+            float4 da[kPerLane], db[kPerLane];
 #pragma unroll
             for (int m = 0; m < kPerLane; ++m) {
-                if (m < cpl) {
-                    if (la) { da[m] = __ldg(ra + 8 * m); }
-                    if (lb) { db[m] = __ldg(rb + 8 * m); }
+                acc[m] = F3{0.0f, 0.0f, 0.0f};
+                da[m] = db[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            for (uint32_t q = 0; q < pairs; ++q) {
+                // Past a strand's count the registers keep its last entries
+                // and the weights are zero.
+                const float4 gw = records[q * 32 + s];
+                const float4 *ra = column + __float_as_uint(gw.x);
+                const float4 *rb = column + __float_as_uint(gw.z);
+                const bool la = 2u * q < nb, lb = 2u * q + 1u < nb;
+#pragma unroll
+                for (int m = 0; m < kPerLane; ++m) {
+                    if (m < cpl) {
+                        if (la) { da[m] = __ldg(ra + 8 * m); }
+                        if (lb) { db[m] = __ldg(rb + 8 * m); }
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < kPerLane; ++m) {
+                    if (m < cpl) { acc[m] = acc[m] + xyz(da[m]) * gw.y + xyz(db[m]) * gw.w; }
                 }
             }
-#pragma unroll
-            for (int m = 0; m < kPerLane; ++m) {
-                if (m < cpl) { acc[m] = acc[m] + xyz(da[m]) * gw.y + xyz(db[m]) * gw.w; }
+            const uint32_t word = live ? locals[s] : 0x80000000u;
+            float4 front = {0.0f, 0.0f, 0.0f, 1.0f}, width = {0.0f, 0.0f, 0.0f, 0.0f};
+            if constexpr (CLASSIC) {
+                front = records[6 * 32 + s];
+                width = records[7 * 32 + s];
             }
-        }
-        if constexpr (STAGED) {
-            float *row = stage + s * kWalkRowFloats;
 #pragma unroll
             for (int m = 0; m < kPerLane; ++m) {
                 const int cm = c + 8 * m;
-                if (live && m < cpl && cm < P) {
-                    stage_put(row, cm,
-                              F3{head.x, head.y, head.z} + (acc[m] * head.w + F3{tail.x, tail.y, tail.z} * tv[m]) * ls);
+                if (m < cpl && cm < P) {
+                    F3 base = F3{head.x, head.y, head.z} + (acc[m] * head.w + F3{tail.x, tail.y, tail.z} * tv[m]) * ls;
+                    float radius = rvals[cm];
+                    if constexpr (CLASSIC) {
+                        if (g.classic_length) { base = xadd(xyz(front), xmul(xsub(base, xyz(front)), front.w)); }
+                        if (width.y != 0.0f) { radius = width.x; }
+                    }
+                    walk_emit(g, word, P, cm, make_float4(base.x, base.y, base.z, radius));
                 }
             }
-            continue;
         }
-        const uint32_t word = live ? locals[s] : 0x80000000u;
-        float4 front = {0.0f, 0.0f, 0.0f, 1.0f}, width = {0.0f, 0.0f, 0.0f, 0.0f};
-        if constexpr (CLASSIC) {
-            front = records[6 * 32 + s];
-            width = records[7 * 32 + s];
+    }
+}
+
+// Base step of one chunk with noise: base points a + 1 .. a + n of each
+// strand (the points after CVs a .. a + n - 1) into stage slots 0 .. n - 1,
+// and for an odd n slot n too; past the strand's end they repeat the tip, a
+// zero segment to the walk.  Lanes as in walk_base_direct.  Every lane of the
+// warp calls it.
+__device__ __forceinline__ void walk_base_chunk(const LaunchArgs &g, const float4 *records, float *stage,
+                                                const float *tvals, const float4 *offsets, int lane, int in_batch,
+                                                int a, int n, int P) {
+    constexpr int kPerLane = kWalkChunk / 8;
+    constexpr int kPasses = 2;
+    constexpr uint32_t kTrip = 4u;
+    const int c = lane & 7;
+    const float ls = g.p.length_scale;
+    uint32_t cm[kPerLane];
+    float tv[kPerLane];
+#pragma unroll
+    for (int m = 0; m < kPerLane; ++m) {
+        cm[m] = static_cast<uint32_t>(min(a + 1 + c + 8 * m, P - 1));
+        tv[m] = tvals[cm[m]];
+    }
+    for (int first = 0; first < in_batch; first += 4 * kPasses) {
+        uint32_t nb[kPasses], most = 0u;
+        f32x2 xy[kPasses][kPerLane];
+        float z[kPasses][kPerLane];
+#pragma unroll
+        for (int u = 0; u < kPasses; ++u) {
+            const int s = first + 4 * u + (lane >> 3);
+            nb[u] = s < in_batch ? __float_as_uint(records[5 * 32 + s].w) : 0u;
+            most = max(most, nb[u]);
+#pragma unroll
+            for (int m = 0; m < kPerLane; ++m) {
+                xy[u][m] = 0ull;
+                z[u][m] = 0.0f;
+            }
+        }
+        const uint32_t trips = __reduce_max_sync(kFull, (most + kTrip - 1u) / kTrip);
+        for (uint32_t q = 0; q < trips; ++q) {
+            ulonglong2 d[kPasses][kTrip][kPerLane];
+            float w[kPasses][kTrip];
+#pragma unroll
+            for (int u = 0; u < kPasses; ++u) {
+                const int s = first + 4 * u + (lane >> 3);
+#pragma unroll
+                for (uint32_t j = 0; j < kTrip; j += 2u) {
+                    const float4 gw = records[(q * kTrip + j) / 2u * 32u + s];
+                    const bool la = q * kTrip + j < nb[u], lb = q * kTrip + j + 1u < nb[u];
+                    w[u][j] = gw.y;
+                    w[u][j + 1u] = gw.w;
+#pragma unroll
+                    for (int m = 0; m < kPerLane; ++m) {
+                        d[u][j][m] = d[u][j + 1u][m] = make_ulonglong2(0ull, 0ull);
+                        if (la) { d[u][j][m] = walk_offset(offsets, __float_as_uint(gw.x) + cm[m]); }
+                        if (lb) { d[u][j + 1u][m] = walk_offset(offsets, __float_as_uint(gw.z) + cm[m]); }
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kPasses; ++u) {
+#pragma unroll
+                for (uint32_t j = 0; j < kTrip; ++j) {
+                    const f32x2 ww = both2(w[u][j]);
+#pragma unroll
+                    for (int m = 0; m < kPerLane; ++m) {
+                        xy[u][m] = fma2(d[u][j][m].x, ww, xy[u][m]);
+                        z[u][m] = fmaf(low2(d[u][j][m].y), w[u][j], z[u][m]);
+                    }
+                }
+            }
         }
 #pragma unroll
-        for (int m = 0; m < kPerLane; ++m) {
-            const int cm = c + 8 * m;
-            if (m < cpl && cm < P) {
-                F3 base = F3{head.x, head.y, head.z} + (acc[m] * head.w + F3{tail.x, tail.y, tail.z} * tv[m]) * ls;
-                float radius = rvals[cm];
-                if constexpr (CLASSIC) {
-                    if (g.classic_length) { base = xadd(xyz(front), xmul(xsub(base, xyz(front)), front.w)); }
-                    if (width.y != 0.0f) { radius = width.x; }
-                }
-                walk_emit(g, word, P, cm, make_float4(base.x, base.y, base.z, radius));
+        for (int u = 0; u < kPasses; ++u) {
+            const int s = first + 4 * u + (lane >> 3);
+            if (s >= in_batch) { continue; }
+            const float4 head = records[4 * 32 + s];
+            const float4 tail = records[5 * 32 + s];
+            float *row = stage + s * kWalkRowFloats;
+            const F3 root = {head.x, head.y, head.z}, normal = {tail.x, tail.y, tail.z};
+#pragma unroll
+            for (int m = 0; m < kPerLane; ++m) {
+                stage_put(row, c + 8 * m,
+                          root + (F3{low2(xy[u][m]), high2(xy[u][m]), z[u][m]} * head.w + normal * tv[m]) * ls);
             }
         }
     }
@@ -606,93 +675,96 @@ constexpr float kFloorMagic = 12582912.0f;      // 1.5 * 2^23
 constexpr uint32_t kFloorMagicBits = 0x4b400000u;
 constexpr float kFloorMagicLimit = 4194304.0f;  // 2^22
 
-// 2 (noise - 0.5) along one axis from the strand's lattice columns (the
-// regrouped blend of lattice_noise); the caller folds the 1/2 into the
-// magnitude, a product by an exact power of two.  The axis' columns start at
-// column axis * columns of the strand's lattice; `bias` is the bit pattern
-// of 1.5 * 2^23 plus the axis' first lattice coordinate minus that start, so
-// the sum's bits minus `bias` index the lattice directly, and `kmax` (the
-// axis' last pair) bounds the index (x never lies below the first column:
-// the walk's distances are non-negative; lanes with no strand read some
-// column of their own lattice).
-__device__ __forceinline__ float walk_lattice_delta(const float2 *lat, uint32_t bias, uint32_t kmax, float x) {
-    const float t = __fadd_rd(x, kFloorMagic);
-    const float w = x - (t - kFloorMagic);
-    const uint32_t k = min(__float_as_uint(t) - bias, kmax);
-    const float2 *col = lat + static_cast<int>(k) * 32;
-    const float2 c0 = col[0];
-    const float2 c1 = col[32];
-    const float s = s_curve(w);
-    const float v0 = c0.x * w + c0.y;
-    const float v1 = c1.x * (w - 1.0f) + c1.y;
-    return v0 + s * (v1 - v0);
-}
-
-// Lattice columns (A, B) of the three noise axes for one strand (see
-// lattice_noise): columns lo .. floor(d0 + span) + 1 cover every CV's X and
-// X + 1 (the walk's noise coordinates d0 + arc * f are computed in the same
-// IEEE operations as d0 + span, so none passes it).  `lat` is this lane's
-// column 0 of axis 0; column k of axis a is at lat[(a * columns + k) * 32].
-// fits is false when a strand needs more columns than the lattice holds, or
-// has coordinates beyond the round-down floor's range (it then takes direct
-// noise).  bias and kmax are the per-axis arguments of walk_lattice_delta.
-struct WalkLattice {
-    int lo[3], n[3];
-    uint32_t bias[3], kmax[3];
-    bool fits;
+// A strand's window on its noise lattice: kWalkWindow columns (A, B) per axis
+// (see lattice_noise) from the lattice coordinate the walk had reached when
+// it was filled.  Column k of axis a is at lat[(a * kWalkWindow + k) * 32] of
+// this lane's lattice.  `bias` is per axis the bit pattern of 1.5 * 2^23 plus
+// the first column's coordinate minus the axis' first column index.  The
+// window holds every distance up to `limit`.
+struct WalkWindow {
+    uint32_t bias[3];
+    float limit;
 };
 
-__device__ __forceinline__ WalkLattice walk_fill_lattice(F3 dom, float span, float2 *lat, const float4 *table,
-                                                       int columns) {
-    WalkLattice wl;
-    wl.fits = true;
+// 2 (noise - 0.5) along one axis at two coordinates from the window's columns
+// (the regrouped blend of lattice_noise); the caller folds the 1/2 into the
+// magnitude, a product by an exact power of two.  The round-down sum's bits
+// minus `bias` index the lattice directly, bounded by the axis' last pair of
+// columns whatever the coordinate (lanes with no strand read some column of
+// their own lattice).
+__device__ __forceinline__ f32x2 walk_lattice_pair(const float2 *lat, uint32_t bias, int axis, float xa, float xb) {
+    const uint32_t last = static_cast<uint32_t>(axis * kWalkWindow + kWalkWindow - 2);
+    const float ta = __fadd_rd(xa, kFloorMagic), tb = __fadd_rd(xb, kFloorMagic);
+    const f32x2 w = sub2(pair2(xa, xb), pair2(ta - kFloorMagic, tb - kFloorMagic));
+    const float2 *ca = lat + static_cast<int>(min(__float_as_uint(ta) - bias, last)) * 32;
+    const float2 *cb = lat + static_cast<int>(min(__float_as_uint(tb) - bias, last)) * 32;
+    const float2 a0 = ca[0], a1 = ca[32], b0 = cb[0], b1 = cb[32];
+    const f32x2 w1 = add2(w, both2(-1.0f));
+    const f32x2 s = mul2(mul2(mul2(w, w), w), fma2(w, fma2(w, both2(6.0f), both2(-15.0f)), both2(10.0f)));
+    const f32x2 v0 = pair2(fmaf(a0.x, low2(w), a0.y), fmaf(b0.x, high2(w), b0.y));
+    const f32x2 v1 = pair2(fmaf(a1.x, low2(w1), a1.y), fmaf(b1.x, high2(w1), b1.y));
+    return fma2(s, sub2(v1, v0), v0);
+}
+
+// The window from `distance` on (bias, limit as a uint4), its columns written
+// to `lat`.  Along axis ax the moving coordinate is d_ax + distance, the other
+// two stay at the domain; the eight-corner blend of one column folds into
+// (A, B), and the corner seeds are linear in the moving lattice coordinate X
+// (noise_hash's LCG chain): seed(X + 1) = seed(X) + step.  `limit` keeps every
+// coordinate, rounded, below the last column; it is negative (no distance
+// fits) beyond the round-down floor's range.  A walk that leaves its window at
+// the end starts the next one inside it, so the first two
+// columns are moved there from the old window and only the others are
+// computed (551 -> 533 us on 1,000,000 strands x 32).  Out of line: it is called about twice per strand, and its
+// registers inlined spill the walk's loop.  Every lane of the warp calls it.
+static __device__ __noinline__ uint4 walk_fill_window(F3 dom, float distance, WalkWindow old, float2 *lat,
+                                                      const float4 *table, uint32_t copies) {
+    __builtin_assume(__isShared(lat));
+    __builtin_assume(__isShared(table));
+    uint32_t bias[3], moved[3];
+    float lo[3];
+    bool near = old.limit >= 0.0f;
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-        const float d0 = component(dom, ax);
-        wl.lo[ax] = static_cast<int>(floorf(d0));
-        wl.n[ax] = static_cast<int>(floorf(__fadd_rn(d0, span))) + 2 - wl.lo[ax];
-        wl.fits = wl.fits && wl.n[ax] >= 2 && wl.n[ax] <= columns && fabsf(d0) + span < kFloorMagicLimit;
+        lo[ax] = floorf(__fadd_rn(component(dom, ax), distance));
+        bias[ax] = kFloorMagicBits + static_cast<uint32_t>(static_cast<int>(lo[ax])) -
+                   static_cast<uint32_t>(ax * kWalkWindow);
+        moved[ax] = bias[ax] - old.bias[ax];
+        near = near && moved[ax] <= static_cast<uint32_t>(kWalkWindow) - 2u;
     }
-    if (!wl.fits) {  // lattice reads stay in bounds (column 0 and 1) whatever the strand
-        wl.n[0] = wl.n[1] = wl.n[2] = 2;
-    }
+    int first = 0;
+    if (__all_sync(kFull, near)) {
+        first = 2;
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        wl.bias[ax] = kFloorMagicBits + static_cast<uint32_t>(wl.lo[ax]) - static_cast<uint32_t>(ax * columns);
-        wl.kmax[ax] = static_cast<uint32_t>(ax * columns + wl.n[ax] - 2);
-    }
-    if (!wl.fits) { return wl; }
-    // Columns 0 and 1 of every axis are faces of the unit lattice cube at
-    // floor(dom): its eight corner gradients (corner o = ox + 2 oy + 4 oz)
-    // serve all three axes, the gradients of columns 2.. are looked up.
-    float4 cube[8];
-    {
-        const uint32_t base = static_cast<uint32_t>(wl.lo[0]) * kLcgA2 + static_cast<uint32_t>(wl.lo[1]) * kLcgA +
-                              static_cast<uint32_t>(wl.lo[2]) + kLcgK;
-#pragma unroll
-        for (int o = 0; o < 8; ++o) {
-            cube[o] = table[temper_index(base + ((o & 1) ? kLcgA2 : 0u) + ((o & 2) ? kLcgA : 0u) +
-                                         ((o & 4) ? 1u : 0u))];
+        for (int ax = 0; ax < 3; ++ax) {
+            const float2 *from = lat + (ax * kWalkWindow + static_cast<int>(moved[ax])) * 32;
+            const float2 c0 = from[0], c1 = from[32];
+            lat[ax * kWalkWindow * 32] = c0;
+            lat[(ax * kWalkWindow + 1) * 32] = c1;
         }
     }
+    float limit = FLT_MAX;
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
         const int ib = ax == 0 ? 1 : 0;  // the fixed axes, ascending
         const int ic = ax == 2 ? 1 : 2;
+        const float d0 = component(dom, ax);
+        const int X = static_cast<int>(lo[ax]);
+        const float end = lo[ax] + static_cast<float>(kWalkWindow - 1);
+        // x = d0 + distance rounds by at most 2^-24 of |x|.
+        const float fits = (end - d0) - 4.0e-7f * (fabsf(d0) + fabsf(end));
+        limit = fabsf(d0) + fabsf(end) < kFloorMagicLimit ? fminf(limit, fits) : -1.0f;
         const float db = component(dom, ib), dc = component(dom, ic);
         const float fb = floorf(db), fc = floorf(dc);
         const float wb = db - fb, wc = dc - fc;
         const float sb = s_curve(wb), sc = s_curve(wc);
         const int Yb = static_cast<int>(fb), Zc = static_cast<int>(fc);
-        // The corner seed is linear in the moving coordinate X (noise_hash's
-        // LCG chain): seed(X + 1) = seed(X) + step.
         const uint32_t step = ax == 0 ? kLcgA2 : (ax == 1 ? kLcgA : 1u);
         uint32_t seed[4];
         float wgt[4], wdb[4], wdc[4];
 #pragma unroll
         for (int corner = 0; corner < 4; ++corner) {
             const int ob = corner & 1, oc = corner >> 1;
-            const int X = wl.lo[ax];
             const int cx = ax == 0 ? X : Yb + ob;
             const int cy = ax == 1 ? X : (ax == 0 ? Yb + ob : Zc + oc);
             const int cz = ax == 2 ? X : Zc + oc;
@@ -702,30 +774,26 @@ __device__ __forceinline__ WalkLattice walk_fill_lattice(F3 dom, float span, flo
             wdb[corner] = wgt[corner] * (wb - static_cast<float>(ob));
             wdc[corner] = wgt[corner] * (wc - static_cast<float>(oc));
         }
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
+#pragma unroll 1
+        for (int k = first; k < kWalkWindow; ++k) {
             float A = 0.0f, B = 0.0f;
 #pragma unroll
             for (int corner = 0; corner < 4; ++corner) {
-                const float4 gr = cube[(k << ax) | ((corner & 1) << ib) | ((corner >> 1) << ic)];
+                const float4 gr = table[temper_index(seed[corner] + static_cast<uint32_t>(k) * step) << copies];
                 A += wgt[corner] * component4(gr, ax);
                 B += component4(gr, ib) * wdb[corner] + component4(gr, ic) * wdc[corner];
             }
-            lat[(ax * columns + k) * 32] = make_float2(A, B);
-        }
-#pragma unroll 2
-        for (int k = 2; k < wl.n[ax]; ++k) {
-            float A = 0.0f, B = 0.0f;
-#pragma unroll
-            for (int corner = 0; corner < 4; ++corner) {
-                const float4 gr = table[temper_index(seed[corner] + static_cast<uint32_t>(k) * step)];
-                A += wgt[corner] * component4(gr, ax);
-                B += component4(gr, ib) * wdb[corner] + component4(gr, ic) * wdc[corner];
-            }
-            lat[(ax * columns + k) * 32] = make_float2(A, B);
+            lat[(ax * kWalkWindow + k) * 32] = make_float2(A, B);
         }
     }
-    return wl;
+    return make_uint4(bias[0], bias[1], bias[2], __float_as_uint(limit));
+}
+
+// 2 (noise - 0.5) at a point, for a segment longer than the window.
+static __device__ __noinline__ float walk_direct_noise(const float4 *table, uint32_t copies, float x, float y,
+                                                       float z) {
+    __builtin_assume(__isShared(table));
+    return 2.0f * (gradient_noise(table, x, y, z, copies) - 0.5f);
 }
 
 __device__ __forceinline__ float walk_effective_frequency(const ParamArgs &p, float original_length) {
@@ -739,117 +807,148 @@ __device__ __forceinline__ float walk_segment_length(F3 b, F3 a) {
     return sqrt_approx(__fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x))));
 }
 
-// The cursor walk (generate.h:465-502) over base points base(0..P-1),
-// handing each noisy point to emit(c, point) in CV order; returns the noisy
-// length (generate.h:553-556) when PRESERVE, else 0.  Tangent after CV c: the
-// next segment's direction, carried over zero-length segments and at the
-// tip; the transported normal rotates by rotate_by(axis, acos(cos)) with
-// cos(acos x) = x and sin(acos x) = sqrt(1 - x^2):
-//   M v = cos v + (1 - cos)(axis . v) axis + sin (axis x v),
-// and is left unchanged when the axis is zero (the axis and that test in
-// ordinary arithmetic: where the reference's rounded cross product vanishes
-// for nearly parallel tangents, the rotation left here is within rounding of
-// the identity).  The body has no per-lane branches (each decision is a
-// select), so the compiler can overlap the noise, tangent and frame chains of
-// neighbouring CVs; noise at CV 0 is
-// multiplied by t_0 = 0.  LATTICE: every lane of the warp reads lattice
-// noise (else every lane evaluates gradient_noise).  Base points are
-// requested three CVs before they are used.
-template <bool LATTICE, bool PRESERVE, class Base, class Emit>
-__device__ __forceinline__ float walk_cursor(const ParamArgs &p, const WalkRoot &wr, float f_eff,
-                                             const WalkLattice &wl, const float2 *lat, const float *tvals,
-                                             const float4 *table, int P, Base base, Emit emit) {
-    // Lattice deltas come doubled (walk_lattice_delta): their magnitude takes
-    // the 1/2, which leaves every product bit-identical.
-    const float mscale = LATTICE ? 0.5f * (p.noise_mask * p.noise_amplitude) : p.noise_mask * p.noise_amplitude;
-    const F3 dom = wr.domain;
-    F3 tan = wr.normal;
-    F3 v = wr.surface_u;
-    F3 cur = base(0);
-    F3 nxt = base(1);
-    F3 ahead = P > 2 ? base(2) : nxt;
-    F3 previous_base = cur;
-    F3 previous_point = cur;
-    float noisy = 0.0f;
-    float arc = 0.0f;
-#pragma unroll 2
-    for (int c = 0; c < P; ++c) {
-        // Past the strand's end the look-ahead repeats the last CV, which is
-        // what `ahead` and `nxt` already hold there (the tip's tangent does
-        // not read it).
-        const F3 further = base(min(c + 3, P - 1));
-        arc = __fadd_rn(arc, walk_segment_length(cur, previous_base));
-        // The reference's length_squared(segment) > 0 holds exactly when some
-        // component's square does not round to zero: the same test on the
-        // fused sum (no flush to zero here).
-        const F3 seg = nxt - cur;
-        const F3 ntan = (c + 1 < P && dot(seg, seg) > 0.0f) ? normalize(seg) : tan;
-        const F3 axis = cross(tan, ntan);
-        // A zero axis leaves the normal as it is: cos 1, sin 0 (then k = 0
-        // and the update below is v itself, exactly).
-        const bool turn = dot(axis, axis) > 0.0f;
-        const float d = fminf(fmaxf(dot(tan, ntan), -1.0f), 1.0f);
-        const float cs = turn ? d : 1.0f;
-        const float sn = turn ? sqrt_approx(fmaf(-d, d, 1.0f)) : 0.0f;
-        const float k = (1.0f - cs) * dot(axis, v);
-        const F3 axv = cross(axis, v);
-        v = F3{v.x * cs + axis.x * k + axv.x * sn, v.y * cs + axis.y * k + axv.y * sn,
-               v.z * cs + axis.z * k + axv.z * sn};
-        // The update is linear in v and the reference renormalises after
-        // every step, a positive factor each time: so the transported normal
-        // is the direction of this unnormalised v, which is carried as it is
-        // (each step keeps at least 0.86 of its length, so 32 steps neither
-        // underflow nor overflow) and normalised here for the frame only.
-        const F3 vu = v * rsqrtf(dot(v, v));
-        const F3 bn = cross(vu, ntan);
-        // The frame's third vector cross(bn, vu) is ntan - vu (vu . ntan) for
-        // a unit vu; its part along vu joins vu's coefficient below.
-        const float vn = dot(vu, ntan);
-        const float distance = __fmul_rn(arc, f_eff);
-        const float magnitude = mscale * tvals[c];
-        float gx, gy, gz;
-        if constexpr (LATTICE) {
-            gx = walk_lattice_delta(lat, wl.bias[0], wl.kmax[0], __fadd_rn(dom.x, distance));
-            gy = walk_lattice_delta(lat, wl.bias[1], wl.kmax[1], __fadd_rn(dom.y, distance));
-            gz = walk_lattice_delta(lat, wl.bias[2], wl.kmax[2], __fadd_rn(dom.z, distance));
-        } else {
-            gx = gradient_noise(table, __fadd_rn(dom.x, distance), dom.y, dom.z) - 0.5f;
-            gy = gradient_noise(table, dom.x, __fadd_rn(dom.y, distance), dom.z) - 0.5f;
-            gz = gradient_noise(table, dom.x, dom.y, __fadd_rn(dom.z, distance)) - 0.5f;
-        }
-        const float gzm = gz * magnitude;
-        const F3 q = cur + vu * fmaf(-gzm, vn, gx * magnitude) + bn * (gy * magnitude) + ntan * gzm;
-        if constexpr (PRESERVE) {
-            const F3 e = q - previous_point;
-            noisy += sqrt_approx(dot(e, e));
-            previous_point = q;
-        }
-        emit(c, q);
-        tan = ntan;
-        previous_base = cur;
-        cur = nxt;
-        nxt = ahead;
-        ahead = further;
-    }
-    return noisy;
+// A strand's cursor between two CVs: the tangent after the last CV handled
+// and the transported normal there, the base point of the next CV and the
+// arc length at it.
+struct WalkCursor {
+    F3 tan, v, cur;
+    float arc;
+};
+
+// A vector per half: one of CV c and one of CV c + 1.
+struct F3x2 {
+    f32x2 x, y, z;
+};
+__device__ __forceinline__ f32x2 dot2(const F3x2 &a, const F3x2 &b) {
+    return fma2(a.z, b.z, fma2(a.y, b.y, mul2(a.x, b.x)));
+}
+// a x b; the products' sign is folded into `minus_a` = -a.
+__device__ __forceinline__ F3x2 cross2(const F3x2 &a, const F3x2 &minus_a, const F3x2 &b) {
+    return {fma2(a.y, b.z, mul2(minus_a.z, b.y)), fma2(a.z, b.x, mul2(minus_a.x, b.z)),
+            fma2(a.x, b.y, mul2(minus_a.y, b.x))};
+}
+__device__ __forceinline__ F3x2 scale2(const F3x2 &a, f32x2 s) { return {mul2(a.x, s), mul2(a.y, s), mul2(a.z, s)}; }
+
+// The transported normal over one CV: rotate_by(axis, acos(cos)) applied to v
+// (generate.h:404-418, :475-481) as the vector update
+//   M v = cos v + (1 - cos)(axis . v) axis + sin (axis x v).
+__device__ __forceinline__ F3 walk_turn(F3 v, F3 axis, float cs, float omc, float sn) {
+    const float k = omc * dot(axis, v);
+    const F3 axv = cross(axis, v);
+    return F3{v.x * cs + axis.x * k + axv.x * sn, v.y * cs + axis.y * k + axv.y * sn,
+              v.z * cs + axis.z * k + axv.z * sn};
 }
 
-// walk_cursor with its warp-uniform variant: lattice noise when every lane
-// whose strand counts (`counts`) fits its lattice.  Every lane of the warp
-// calls it.
-template <class Base, class Emit>
-__device__ __forceinline__ float walk_cursor_any(const ParamArgs &p, const WalkRoot &wr, float f_eff,
-                                                 const WalkLattice &wl, bool counts, const float2 *lat,
-                                                 const float *tvals, const float4 *table, int P, Base base,
-                                                 Emit emit) {
-    const bool lattice = __all_sync(kFull, wl.fits || !counts);
-    const bool preserve = p.noise_preserve_length > 0.001f;
-    if (lattice) {
-        return preserve ? walk_cursor<true, true>(p, wr, f_eff, wl, lat, tvals, table, P, base, emit)
-                        : walk_cursor<true, false>(p, wr, f_eff, wl, lat, tvals, table, P, base, emit);
+// Two steps of the cursor walk (generate.h:465-502): the noisy points qa, qb
+// of the CV at the cursor and of the one after it, whose next base points are
+// n0 and n1 (a strand's tip repeats the last base point: a zero segment).
+// Tangent after a CV: the next segment's direction, carried over zero-length
+// segments and at the tip; the transported normal turns by walk_turn with
+// cos(acos x) = x and sin(acos x) = sqrt(1 - x^2), and is left unchanged when
+// the axis is zero (the axis and that test in ordinary arithmetic: where the
+// reference's rounded cross product vanishes for nearly parallel tangents,
+// the rotation left here is within rounding of the identity).
+//
+// What the two CVs do alike runs as packed f32x2 arithmetic, one instruction
+// for both (segments, tangents, rotation axes, frame vectors, the noise
+// blend): the walk is bound by instruction issue and by its dependency
+// chains, and only the turn of v is a chain from CV to CV.  The segment's
+// squared length serves both its direction and the arc length.  `turn` is the
+// CVs' t and `mscale` half the noise magnitude at t = 1 (the noise comes
+// doubled).  The warp refills its windows when a strand that counts has
+// reached the end of its own; a segment that no window holds makes the warp
+// evaluate gradient noise directly.  Every lane of the warp calls it.
+__device__ __forceinline__ void walk_pair(WalkCursor &s, F3 n0, F3 n1, f32x2 t, float mscale, float f_eff, F3 dom,
+                                          bool counts, WalkWindow &wl, float2 *lat, const float4 *table,
+                                          uint32_t copies, F3 &qa, F3 &qb) {
+    const F3 sa = n0 - s.cur, sb = n1 - n0;
+    const F3x2 seg = {pair2(sa.x, sb.x), pair2(sa.y, sb.y), pair2(sa.z, sb.z)};
+    const f32x2 l2 = dot2(seg, seg);
+    const float la = low2(l2), lb = high2(l2);
+    F3x2 tn = scale2(seg, pair2(rsqrt_normal(la), rsqrt_normal(lb)));
+    if (fminf(la, lb) <= 1.0e-20f) {  // a zero segment keeps the tangent; normalize() of a tiny one is (0, 1, 0)
+        F3 ta = la > 1.0e-20f ? F3{low2(tn.x), low2(tn.y), low2(tn.z)} : la > 0.0f ? F3{0.0f, 1.0f, 0.0f} : s.tan;
+        F3 tb = lb > 1.0e-20f ? F3{high2(tn.x), high2(tn.y), high2(tn.z)} : lb > 0.0f ? F3{0.0f, 1.0f, 0.0f} : ta;
+        tn = F3x2{pair2(ta.x, tb.x), pair2(ta.y, tb.y), pair2(ta.z, tb.z)};
     }
-    return preserve ? walk_cursor<false, true>(p, wr, f_eff, wl, lat, tvals, table, P, base, emit)
-                    : walk_cursor<false, false>(p, wr, f_eff, wl, lat, tvals, table, P, base, emit);
+    const float arc_b = __fadd_rn(s.arc, sqrt_approx(la));
+    const f32x2 minus = both2(-1.0f);
+    const F3x2 tp = {pair2(s.tan.x, low2(tn.x)), pair2(s.tan.y, low2(tn.y)), pair2(s.tan.z, low2(tn.z))};
+    const F3x2 axis = cross2(tp, scale2(tp, minus), tn);
+    const f32x2 d = dot2(tp, tn);
+    const f32x2 a2 = dot2(axis, axis);
+    const f32x2 d1 = fma2(d, d, minus);  // cos^2 - 1
+    const float ca = low2(a2) > 0.0f ? low2(d) : 1.0f, cb = high2(a2) > 0.0f ? high2(d) : 1.0f;
+    const f32x2 omc = sub2(both2(1.0f), pair2(ca, cb));
+    const F3 va = walk_turn(s.v, F3{low2(axis.x), low2(axis.y), low2(axis.z)}, ca, low2(omc),
+                            sqrt_approx(fmaxf(-low2(d1), 0.0f)));
+    const F3 vb = walk_turn(va, F3{high2(axis.x), high2(axis.y), high2(axis.z)}, cb, high2(omc),
+                            sqrt_approx(fmaxf(-high2(d1), 0.0f)));
+    // The update is linear in v and the reference renormalises after every
+    // step, a positive factor each time: so the transported normal is the
+    // direction of this unnormalised v, which is carried as it is (each step
+    // keeps at least 0.86 of its length, so 32 steps neither underflow nor
+    // overflow) and normalised here for the frame only.
+    const F3x2 v = {pair2(va.x, vb.x), pair2(va.y, vb.y), pair2(va.z, vb.z)};
+    const f32x2 v2 = dot2(v, v);
+    const F3x2 vu = scale2(v, pair2(rsqrt_normal(low2(v2)), rsqrt_normal(high2(v2))));
+    const F3x2 mv = scale2(vu, minus);
+    const F3x2 bn = cross2(vu, mv, tn);
+    // The frame's third vector cross(bn, vu) is tn - vu (vu . tn) for a unit
+    // vu; its part along vu joins vu's coefficient below.
+    const f32x2 mvn = dot2(mv, tn);
+    const float da = __fmul_rn(s.arc, f_eff), db = __fmul_rn(arc_b, f_eff);
+    bool lattice = true;
+    if (__any_sync(kFull, counts && !(db <= wl.limit))) {
+        const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies);
+        wl = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
+        lattice = __all_sync(kFull, db <= wl.limit || !counts);
+    }
+    f32x2 gx, gy, gz;
+    if (lattice) {
+        gx = walk_lattice_pair(lat, wl.bias[0], 0, __fadd_rn(dom.x, da), __fadd_rn(dom.x, db));
+        gy = walk_lattice_pair(lat, wl.bias[1], 1, __fadd_rn(dom.y, da), __fadd_rn(dom.y, db));
+        gz = walk_lattice_pair(lat, wl.bias[2], 2, __fadd_rn(dom.z, da), __fadd_rn(dom.z, db));
+    } else {
+        gx = pair2(walk_direct_noise(table, copies, __fadd_rn(dom.x, da), dom.y, dom.z),
+                   walk_direct_noise(table, copies, __fadd_rn(dom.x, db), dom.y, dom.z));
+        gy = pair2(walk_direct_noise(table, copies, dom.x, __fadd_rn(dom.y, da), dom.z),
+                   walk_direct_noise(table, copies, dom.x, __fadd_rn(dom.y, db), dom.z));
+        gz = pair2(walk_direct_noise(table, copies, dom.x, dom.y, __fadd_rn(dom.z, da)),
+                   walk_direct_noise(table, copies, dom.x, dom.y, __fadd_rn(dom.z, db)));
+    }
+    const f32x2 magnitude = mul2(both2(mscale), t);  // 0 at CV 0
+    const f32x2 lx = mul2(gx, magnitude), ly = mul2(gy, magnitude), lz = mul2(gz, magnitude);
+    const f32x2 along = fma2(lz, mvn, lx);
+    const f32x2 ox = fma2(tn.x, lz, fma2(bn.x, ly, mul2(vu.x, along)));
+    const f32x2 oy = fma2(tn.y, lz, fma2(bn.y, ly, mul2(vu.y, along)));
+    const f32x2 oz = fma2(tn.z, lz, fma2(bn.z, ly, mul2(vu.z, along)));
+    qa = s.cur + F3{low2(ox), low2(oy), low2(oz)};
+    qb = n0 + F3{high2(ox), high2(oy), high2(oz)};
+    s.tan = F3{high2(tn.x), high2(tn.y), high2(tn.z)};
+    s.v = vb;
+    s.cur = n1;
+    s.arc = __fadd_rn(arc_b, sqrt_approx(lb));
+}
+
+// Fills a CTA's head (every thread calls it; a barrier must follow): the
+// gradient table with noise, t = cv / (P - 1) (generate.h:295-298) and the
+// radii, the padding after the tip repeating it.
+template <bool NOISE>
+__device__ __forceinline__ void walk_fill_head(const LaunchArgs &g, float4 *table, float *tvals, float *rvals) {
+    if constexpr (NOISE) {
+        const uint32_t copies = walk_table_copies(blockDim.x >> 5);
+        for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(kTableFloat4) << copies; i += blockDim.x) {
+            const float *gradient = g.a.gradients + 3u * (i >> copies);
+            table[i] = make_float4(__ldg(gradient), __ldg(gradient + 1), __ldg(gradient + 2), 0.0f);
+        }
+    }
+    const uint32_t P = g.p.cvs_per_strand;
+    for (uint32_t i = threadIdx.x; i < walk_padded(P); i += blockDim.x) {
+        const float t = __fdiv_rn(static_cast<float>(min(i, P - 1u)), static_cast<float>(P - 1u));
+        tvals[i] = t;
+        rvals[i] = strand_radius(g.p, t);
+    }
 }
 
 // preserveLength scale (generate.h:553-563), or 1.
@@ -859,134 +958,244 @@ __device__ __forceinline__ float walk_preserve_scale(const ParamArgs &p, float o
     return fabsf(noisy - target) >= 0.0001f ? target / noisy : 1.0f;
 }
 
-// Frame step for the strand whose staged row is `row` (this lane's strand):
-// the base curve's length, the lattice, then the cursor walk, leaving the
-// noisy points in the row.  The walk reads CV c + 3 after
-// writing CV c, so it never reads a point it has replaced.  Every lane of the
-// warp calls it; lanes whose strand does not count (past the batch) work on
-// whatever their row holds and are ignored.
-__device__ __forceinline__ void walk_frame(const ParamArgs &p, const WalkRoot &wr, bool counts, float *row,
-                                           float2 *lat, const float *tvals, const float4 *table, int P,
-                                           int columns) {
-    // Length of the base curve (generate.h:420-433); the walk accumulates the
-    // same prefix again as its arc length, in the same operations.
-    float original_length = 0.0f;
-    {
-        F3 prev = stage_get(row, 0);
-#pragma unroll 8
-        for (int c = 1; c < P; ++c) {
-            const F3 cur = stage_get(row, c);
-            original_length = __fadd_rn(original_length, walk_segment_length(cur, prev));
-            prev = cur;
-        }
-    }
-    const float f_eff = walk_effective_frequency(p, original_length);
-    const WalkLattice wl = walk_fill_lattice(wr.domain, __fmul_rn(original_length, f_eff), lat, table, columns);
-    const float noisy = walk_cursor_any(
-        p, wr, f_eff, wl, counts, lat, tvals, table, P, [&](int c) { return stage_get(row, c); },
-        [&](int c, F3 q) { stage_put(row, c, q); });
-    const float scale = walk_preserve_scale(p, original_length, noisy);
-    if (scale != 1.0f) {
-        const F3 root = wr.position;
-        for (int c = 0; c < P; ++c) { stage_put(row, c, root + (stage_get(row, c) - root) * scale); }
-    }
-}
-
-// generate_pipe_kernel shared memory: table | t values | radii | two buffers
-// (stage, 12 x 32 frame floats, 32 output words) | producer records |
-// consumer lattice.
-constexpr size_t kPipeFrameBytes = sizeof(float) * 12u * 32u;
-constexpr size_t kPipeBufferBytes = kWalkStageBytes + kPipeFrameBytes + kWalkLocalBytes;
-constexpr size_t kPipeSmemBytes = sizeof(float4) * kTableFloat4 + 2u * sizeof(float) * kWalkMaxCvs +
-                                  2u * kPipeBufferBytes + kWalkRecordBytes + kWalkLatticeBytes;
-
-// Store step without Classic scalars, eight lanes per strand as in
-// walk_base_direct: lane (s = pass * 4 + lane / 8, c = lane % 8) stores CVs
-// c + 8m of its strand's staged row, so each store instruction writes four
-// strands' runs of eight consecutive float4s, and a lane's radii are fixed
-// for the whole kernel.  Every lane of the warp calls it.
-__device__ __forceinline__ void walk_store8(const LaunchArgs &g, const float *stage, const uint32_t *locals,
-                                            const float *rvals, int lane, int in_batch, int P) {
-    constexpr int kPerLane = kWalkMaxCvs / 8;
-    const int c = lane & 7;
-    const int cpl = (P + 7) >> 3;
-    float rv[kPerLane];
-#pragma unroll
-    for (int m = 0; m < kPerLane; ++m) { rv[m] = rvals[min(c + 8 * m, P - 1)]; }
-    for (int first = 0; first < in_batch; first += 4) {
-        const int s = first + (lane >> 3);  // at most 31
-        const uint32_t word = s < in_batch ? locals[s] : 0x80000000u;
-        const float *row = stage + s * kWalkRowFloats;
-#pragma unroll
-        for (int m = 0; m < kPerLane; ++m) {
-            const int cm = c + 8 * m;
-            if (m < cpl && cm < P) {
-                const F3 q = stage_get(row, cm);
-                walk_emit(g, word, P, cm, make_float4(q.x, q.y, q.z, rv[m]));
-            }
-        }
-    }
-}
-
-// The Classic application's per-strand values for the noisy walk, once per
-// strand after the walk (lane = strand; the rules of emit_strand: scale about
-// the first point, width override, the drop rule with its chord bound and
-// sampled-spline measure): records 6 and 7 take (first point, length scale)
-// and (width radius); a dropped strand's point count becomes 0.  The records
-// are free again once the walk is done (the lattice aliased them).  Every
-// lane of the warp calls it.
-__device__ __forceinline__ void walk_classic_strand(const LaunchArgs &g, float4 *records, const float *stage,
-                                                    const uint32_t *locals, int lane, int in_batch, int P) {
-    const ParamArgs &p = g.p;
-    const uint32_t word = locals[lane];
-    if (lane >= in_batch || (word >> 31)) { return; }
+// Length of this lane's base curve (generate.h:420-433), chunk by chunk.
+// Every lane of the warp calls it.
+static __device__ __noinline__ float walk_base_length(const LaunchArgs &g, const float4 *records, float *stage,
+                                                  const float *tvals, const float4 *offsets, int lane, int in_batch,
+                                                  int P, F3 first) {
     const float *row = stage + lane * kWalkRowFloats;
-    const float2 sc = __ldg(g.scalars + word);
-    const F3 front = stage_get(row, 0);
-    const F3 back = stage_get(row, P - 1);
-    const float scale = g.classic_length ? sc.x : 1.0f;
-    const float raw_width = g.classic_width ? sc.y
-        : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
-    bool keep = !(raw_width < 1.0e-4f);
-    const F3 chord = back - front;
-    if (keep && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f)) {
-        keep = !(__fmul_rn(classic_spline_length_by([row](int i) { return stage_get(row, i); }, P), scale) <
-                 1.0e-4f);
+    float length = 0.0f;
+    for (int a = 0; a < P - 1; a += kWalkChunk) {
+        const int n = min(kWalkChunk, P - 1 - a);
+        walk_base_chunk(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+        __syncwarp();
+        for (int i = 0; i < n; ++i) {
+            const F3 next = stage_get(row, i);
+            const F3 d = next - first;
+            length = __fadd_rn(length, sqrt_approx(dot(d, d)));
+            first = next;
+        }
+        __syncwarp();
     }
-    records[6 * 32 + lane] = make_float4(front.x, front.y, front.z, scale);
-    records[7 * 32 + lane] =
-        make_float4(__fmul_rn(__fmul_rn(0.5f, raw_width < 0.0f ? 0.0f : raw_width), p.radius_scale), 0.0f, 0.0f, 0.0f);
-    if (!keep && g.point_counts != nullptr) { g.point_counts[word] = 0u; }
+    return length;
 }
 
-// Store step with the Classic application of records 6 and 7
-// (walk_classic_strand), eight lanes per strand as in walk_store8.  Every
-// lane of the warp calls it.
-__device__ __forceinline__ void walk_store8_classic(const LaunchArgs &g, const float4 *records, const float *stage,
-                                                    const uint32_t *locals, const float *rvals, int lane,
-                                                    int in_batch, int P) {
-    constexpr int kPerLane = kWalkMaxCvs / 8;
+// Store step of one chunk, eight lanes per strand as in walk_base_chunk: each
+// store instruction writes four strands' runs of eight consecutive float4s.
+// Every lane of the warp calls it.
+__device__ __forceinline__ void walk_store_chunk(const LaunchArgs &g, const float *stage, const uint32_t *locals,
+                                                 const float *rvals, int lane, int in_batch, int a, int n, int P,
+                                                 bool again) {
+    constexpr int kPerLane = kWalkChunk / 8;
     const int c = lane & 7;
-    const int cpl = (P + 7) >> 3;
     float rv[kPerLane];
 #pragma unroll
-    for (int m = 0; m < kPerLane; ++m) { rv[m] = rvals[min(c + 8 * m, P - 1)]; }
+    for (int m = 0; m < kPerLane; ++m) { rv[m] = rvals[min(a + c + 8 * m, P - 1)]; }
     for (int first = 0; first < in_batch; first += 4) {
         const int s = first + (lane >> 3);  // at most 31
         const uint32_t word = s < in_batch ? locals[s] : 0x80000000u;
         const float *row = stage + s * kWalkRowFloats;
-        const float4 front = records[6 * 32 + s];
-        const float width = records[7 * 32 + s].x;
 #pragma unroll
         for (int m = 0; m < kPerLane; ++m) {
-            const int cm = c + 8 * m;
-            if (m < cpl && cm < P) {
-                F3 q = stage_get(row, cm);
-                if (g.classic_length) { q = xadd(xyz(front), xmul(xsub(q, xyz(front)), front.w)); }
-                walk_emit(g, word, P, cm, make_float4(q.x, q.y, q.z, g.classic_width ? width : rv[m]));
+            if (c + 8 * m < n) {
+                const F3 q = stage_get(row, c + 8 * m);
+                walk_emit(g, word, P, a + c + 8 * m, make_float4(q.x, q.y, q.z, rv[m]), again);
             }
         }
     }
+}
+
+// Rewrites the written points of the warp's strands: each lane holds its own
+// strand's centre and scale (about `centre`, points to centre + (q - centre)
+// * scale) and radius override (negative: none); lanes over one strand's CVs,
+// so a strand's run is read and written as consecutive float4s.  EXACT: in
+// the uncontracted operations of the Classic application.  The points are
+// this warp's own writes of a moment ago (in L2).  Every lane of the warp
+// calls it, after a __syncwarp.
+template <bool EXACT>
+__device__ __forceinline__ void walk_rescale(const LaunchArgs &g, const uint32_t *locals, F3 centre, float scale,
+                                             float radius, int lane, int in_batch, int P) {
+    for (int s = 0; s < in_batch; ++s) {
+        const uint32_t word = locals[s];
+        const F3 o = {__shfl_sync(kFull, centre.x, s), __shfl_sync(kFull, centre.y, s),
+                      __shfl_sync(kFull, centre.z, s)};
+        const float k = __shfl_sync(kFull, scale, s);
+        const float r = __shfl_sync(kFull, radius, s);
+        const bool move = EXACT ? g.classic_length != 0u : k != 1.0f;
+        if ((word >> 31) || (!move && r < 0.0f)) { continue; }
+        const uint64_t begin = static_cast<uint64_t>(word) * static_cast<uint32_t>(P);
+        if (g.vec3_points) {
+            for (int c = lane; c < P; c += 32) {
+                float *q = g.vec3_points + 3u * (begin + static_cast<uint32_t>(c));
+                const F3 v = o + (F3{q[0], q[1], q[2]} - o) * k;
+                q[0] = v.x;
+                q[1] = v.y;
+                q[2] = v.z;
+            }
+            continue;
+        }
+        float4 *points = g.points + begin;
+#pragma unroll 4
+        for (int c = lane; c < P; c += 32) {
+            const float4 q = points[c];
+            F3 v = xyz(q);
+            if (move) { v = EXACT ? xadd(o, xmul(xsub(v, o), k)) : o + (v - o) * k; }
+            points[c] = make_float4(v.x, v.y, v.z, r < 0.0f ? q.w : r);
+        }
+    }
+}
+
+// The Classic application to noisy strands once their points are written
+// (the rules of emit_strand: scale about the first point, width override, the
+// drop rule with its chord bound and sampled-spline measure); a dropped
+// strand's point count becomes 0.  Every lane of the warp calls it, after a
+// __syncwarp.
+__device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const uint32_t *locals, int lane,
+                                                    int in_batch, int P) {
+    const ParamArgs &p = g.p;
+    const uint32_t word = lane < in_batch ? locals[lane] : 0x80000000u;
+    F3 front = {0.0f, 0.0f, 0.0f};
+    float scale = 1.0f, radius = -1.0f;
+    if (!(word >> 31)) {
+        const float4 *points = g.points + static_cast<uint64_t>(word) * static_cast<uint32_t>(P);
+        const float2 sc = __ldg(g.scalars + word);
+        front = xyz(points[0]);
+        const F3 back = xyz(points[P - 1]);
+        scale = g.classic_length ? sc.x : 1.0f;
+        const float raw_width = g.classic_width ? sc.y
+            : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
+        bool keep = !(raw_width < 1.0e-4f);
+        const F3 chord = back - front;
+        if (keep && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f)) {
+            keep = !(__fmul_rn(classic_spline_length_by([points](int i) { return xyz(points[i]); }, P), scale) <
+                     1.0e-4f);
+        }
+        if (g.classic_width) {
+            radius = __fmul_rn(__fmul_rn(0.5f, raw_width < 0.0f ? 0.0f : raw_width), p.radius_scale);
+        }
+        if (!keep && g.point_counts != nullptr) { g.point_counts[word] = 0u; }
+    }
+    __syncwarp();
+    walk_rescale<true>(g, locals, front, scale, radius, lane, in_batch, P);
+}
+
+// One batch of a warp with noise: strands [batch, batch + in_batch) of the
+// order through setup, base, frame and store.  Every lane of the warp calls
+// it; lanes past in_batch set up its first strand again and are ignored.
+template <bool CLASSIC>
+__device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const float4 *offsets, unsigned char *mine,
+                                                 const float4 *table, const float *tvals, const float *rvals,
+                                                 int lane, uint32_t batch, int in_batch) {
+    float *stage = reinterpret_cast<float *>(mine);
+    float2 *lattice = reinterpret_cast<float2 *>(mine + kWalkStageBytes) + lane;
+    const uint32_t copies = walk_table_copies(blockDim.x >> 5);
+    table += static_cast<uint32_t>(lane) & ((1u << copies) - 1u);
+    float4 *records = reinterpret_cast<float4 *>(mine + kWalkStageBytes + kWalkLatticeBytes);
+    uint32_t *locals = reinterpret_cast<uint32_t *>(mine + kWalkStageBytes + kWalkLatticeBytes + kWalkRecordBytes);
+    const ParamArgs &p = g.p;
+    const int P = static_cast<int>(p.cvs_per_strand);
+    const bool counts = lane < in_batch;
+    const WalkRoot wr = walk_setup<true>(g, records, locals, lane, batch + (counts ? static_cast<uint32_t>(lane) : 0u),
+                                         counts, static_cast<uint32_t>(P));
+    __syncwarp();
+    WalkCursor s{wr.normal, wr.surface_u, wr.position, 0.0f};
+    if (__any_sync(kFull, wr.lead)) { s.cur = walk_base_point(records, lane, 0, tvals[0], p.length_scale, offsets); }
+    float f_eff = p.noise_frequency;
+    const float mscale = 0.5f * (p.noise_mask * p.noise_amplitude);
+    const bool preserve = p.noise_preserve_length > 0.001f;
+    const bool one_chunk = P <= kWalkChunk;
+    const bool again = CLASSIC || (preserve && !one_chunk);
+    float *row = stage + lane * kWalkRowFloats;
+    WalkWindow window;
+    window.limit = -1.0f;
+    F3 previous = s.cur;
+    float noisy = 0.0f;
+    for (int a = 0; a < P; a += kWalkChunk) {
+        const int n = min(kWalkChunk, P - a);
+        walk_base_chunk(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+        __syncwarp();
+        if (a == 0) {
+            // The effective frequency max(0.5 / length, frequency)
+            // (generate.h:543) is the frequency itself for a strand of at
+            // least 0.5 / frequency, which a chord that long from the root to
+            // the chunk's last point or to the tip shows; else the base curve
+            // is measured.
+            const auto sure = [&](F3 point) {
+                const F3 chord = point - s.cur;
+                return sqrt_approx(dot(chord, chord)) * p.noise_frequency * 0.9999f >= 0.5f || !counts;
+            };
+            if (!__all_sync(kFull, sure(stage_get(row, min(n, P - 1) - 1))) &&
+                !__all_sync(kFull, sure(walk_base_point(records, lane, P - 1, tvals[P - 1], p.length_scale,
+                                                        offsets)))) {
+                f_eff = walk_effective_frequency(
+                    p, walk_base_length(g, records, stage, tvals, offsets, lane, in_batch, P, s.cur));
+                walk_base_chunk(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+                __syncwarp();
+            }
+        }
+        F3 n0 = stage_get(row, 0), n1 = stage_get(row, 1);
+#pragma unroll 1
+        for (int i = 0; i < n; i += 2) {
+            // The next pair is requested before this one is replaced (past
+            // the chunk: slots that are not used).
+            const int ahead = min(i + 2, kWalkChunk - 2);
+            const F3 ahead0 = stage_get(row, ahead), ahead1 = stage_get(row, ahead + 1);
+            F3 qa, qb;
+            walk_pair(s, n0, n1, *reinterpret_cast<const f32x2 *>(tvals + a + i), mscale, f_eff, wr.domain, counts,
+                      window, lattice, table, copies, qa, qb);
+            if (preserve) {
+                const F3 e = qa - previous, f = qb - qa;
+                noisy += sqrt_approx(dot(e, e));
+                if (i + 1 < n) { noisy += sqrt_approx(dot(f, f)); }
+                previous = qb;
+            }
+            stage_put(row, i, qa);
+            stage_put(row, i + 1, qb);
+            n0 = ahead0;
+            n1 = ahead1;
+        }
+        if (preserve && one_chunk) {
+            const float scale = walk_preserve_scale(p, s.arc, noisy);
+            if (scale != 1.0f) {
+                for (int c = 0; c < P; ++c) {
+                    stage_put(row, c, wr.position + (stage_get(row, c) - wr.position) * scale);
+                }
+            }
+        }
+        __syncwarp();
+        walk_store_chunk(g, stage, locals, rvals, lane, in_batch, a, n, P, again);
+        __syncwarp();
+    }
+    if (preserve && !one_chunk) {
+        const float scale = counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
+        if (__any_sync(kFull, scale != 1.0f)) {
+            walk_rescale<false>(g, locals, wr.position, scale, -1.0f, lane, in_batch, P);
+            __syncwarp();
+        }
+    }
+    if constexpr (CLASSIC) { walk_classic_finish(g, locals, lane, in_batch, P); }
+    __syncwarp();
+}
+
+// One batch of a warp without noise: setup and the base step straight to the
+// output, with the Classic application.  As walk_noise_batch.
+template <bool CLASSIC>
+__device__ __forceinline__ void walk_plain_batch(const LaunchArgs &g, const float4 *offsets, unsigned char *mine,
+                                                 const float *tvals, const float *rvals, int lane, uint32_t batch,
+                                                 int in_batch) {
+    float4 *records = reinterpret_cast<float4 *>(mine);
+    uint32_t *locals = reinterpret_cast<uint32_t *>(mine + (CLASSIC ? kWalkClassicRecordBytes : kWalkRecordBytes));
+    const int P = static_cast<int>(g.p.cvs_per_strand);
+    const bool counts = lane < in_batch;
+    walk_setup<false>(g, records, locals, lane, batch + (counts ? static_cast<uint32_t>(lane) : 0u), counts,
+                      static_cast<uint32_t>(P));
+    __syncwarp();
+    if constexpr (CLASSIC) {
+        walk_classic_setup(g, records, lane, counts, locals[lane] & 0x7fffffffu, tvals, offsets, P);
+        __syncwarp();
+    }
+    walk_base_direct<CLASSIC>(g, records, locals, tvals, rvals, offsets, lane, in_batch, P);
+    __syncwarp();
 }
 
 } // namespace dev
