@@ -2,22 +2,21 @@
 //
 // A frame of several descriptions (each its own .nxg asset, strand count,
 // CV count, stencil and noise settings) is generated by:
-//   batched_clear      zero the per-description bins and the work counter;
+//   batched_offsets    every description's guide-offset table and guide frame
+//                      records; zeroes the bins and the work counters;
 //   batched_prepare    one pass over every strand of every description:
 //                      root triangle and sort key (first stencil guide)
 //                      with its histogram;
 //   batched_scan       one CTA per description: bin offsets;
 //   batched_scatter    per-description strand-locality orders (ranks in
 //                      shared memory, one global atomic per block and bin);
-//   batched_offsets    every description's guide-offset table and guide
-//                      frame records;
 //   batched_generate   one launch per class of work item -- noisy, noise-free
 //                      -- each with the CTA shape, shared memory and register
 //                      budget of its variant of the lane walk (walk.cuh);
 //                      persistent CTAs pull (description, slice of its strand
 //                      order) items of their class from an atomic counter --
 //                      items of the costliest descriptions first.
-// Six or seven launches per frame whatever the description count, all
+// Five or six chained launches per frame whatever the description count, all
 // enqueue-only and capturable in one CUDA graph.
 #include "generator_core.cuh"
 #include "walk.cuh"
@@ -56,6 +55,7 @@ struct BatchArgs {
     // are k in [desc_first[c], desc_end[c]).
     uint32_t total_items[2];
     uint32_t desc_first[2], desc_end[2];
+    uint32_t first_class;      // the class whose launch comes first
     uint32_t *item_counter;    // one counter per class
     uint64_t total_offsets;
     BatchDesc d[kMaxBatch];
@@ -67,19 +67,11 @@ __device__ __forceinline__ int desc_of_strand(const BatchArgs &b, uint32_t i) {
     return d;
 }
 
-__global__ void batched_clear_kernel(const __grid_constant__ BatchArgs b) {
-    if (blockIdx.x == 0 && threadIdx.x < 2) { b.item_counter[threadIdx.x] = 0u; }
-    for (uint32_t d = 0; d < b.count; ++d) {
-        const uint32_t bins = b.d[d].g.a.guide_count + 1u;
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bins; i += gridDim.x * blockDim.x) {
-            b.d[d].bins[i] = 0u;
-        }
-    }
-}
-
 // One CTA (1024 threads) per description: exclusive scan of its bins.
 __global__ void __launch_bounds__(1024) batched_scan_kernel(const __grid_constant__ BatchArgs b) {
     __shared__ uint32_t warp_sums[32];
+    chain_start();
+    chain_wait();
     const BatchDesc &d = b.d[blockIdx.x];
     uint32_t *data = d.bins;
     const uint32_t n = d.g.a.guide_count + 1u;
@@ -124,6 +116,8 @@ constexpr uint32_t kBatchScatterBins = 8192u;
 __global__ void __launch_bounds__(1024) batched_scatter_blocked_kernel(const __grid_constant__ BatchArgs b,
                                                                        uint32_t chunk) {
     extern __shared__ uint32_t slots[];
+    chain_start();
+    chain_wait();
     const uint32_t begin = blockIdx.x * chunk;
     const uint32_t end = min(b.total_strands, begin + chunk);
     if (begin >= end) { return; }
@@ -156,7 +150,17 @@ __global__ void __launch_bounds__(1024) batched_scatter_blocked_kernel(const __g
     }
 }
 
+// Also clears the work counters and the descriptions' bins.
 __global__ void batched_offsets_kernel(const __grid_constant__ BatchArgs b) {
+    chain_start();
+    chain_wait();
+    if (blockIdx.x == 0 && threadIdx.x < 2) { b.item_counter[threadIdx.x] = 0u; }
+    for (uint32_t d = 0; d < b.count; ++d) {
+        const uint32_t bins = b.d[d].g.a.guide_count + 1u;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bins; i += gridDim.x * blockDim.x) {
+            b.d[d].bins[i] = 0u;
+        }
+    }
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < b.total_offsets;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         int di = 0;
@@ -186,6 +190,8 @@ constexpr uint32_t kBatchPrivateBins = 4096u;
 
 __global__ void __launch_bounds__(256) batched_prepare_kernel(const __grid_constant__ BatchArgs b, uint32_t chunk) {
     __shared__ uint32_t hist[kBatchPrivateBins];
+    chain_start();
+    chain_wait();
     const uint32_t begin = blockIdx.x * chunk;
     const uint32_t end = min(begin + chunk, b.total_strands);
     if (begin >= end) { return; }
@@ -256,11 +262,12 @@ __global__ void __launch_bounds__(CLS == 1 ? 256 : 32 * kWalkNoiseWarps, CLS == 
     const int lane = threadIdx.x & 31;
     const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint32_t per_item = warps * batches_per_warp(CLS);
-    // The next class's launch reads nothing this one writes (its own
-    // descriptions' outputs; the strand order and offset tables were done
-    // before this launch began), so it may start as soon as this launch's
-    // CTAs leave SMs free.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // The strand order and offset tables are complete once this launch may
+    // touch memory.  The next class's launch reads nothing this one writes (its
+    // own descriptions' outputs), so from then on it may start as soon as this
+    // launch's CTAs leave SMs free; it waits at its end only.
+    if (b.first_class == static_cast<uint32_t>(CLS)) { chain_wait(); }
+    chain_start();
     float *tvals = reinterpret_cast<float *>(smem + (CLS == 0 ? kTableFloat4 << walk_table_copies(warps) : 0));
     float *rvals = tvals + walk_padded(kBatchMaxCvs);
     unsigned char *mine = reinterpret_cast<unsigned char *>(rvals + walk_padded(kBatchMaxCvs)) +
@@ -307,6 +314,9 @@ __global__ void __launch_bounds__(CLS == 1 ? 256 : 32 * kWalkNoiseWarps, CLS == 
         }
         __syncthreads();  // the item's batches are done before the next claim resets the counter
     }
+    // The second launch ends no earlier than the first, so what follows on the
+    // stream follows both.
+    if (b.first_class != static_cast<uint32_t>(CLS)) { chain_wait(); }
 }
 
 } // namespace dev
@@ -491,31 +501,25 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
     const auto s = static_cast<cudaStream_t>(stream);
     const int sms = sm_count();
     set_last_cuda_error(0);
-    dev::batched_clear_kernel<<<std::max(1, sms), 256, 0, s>>>(b);
-    if ((status = record_cuda(cudaGetLastError()))) { return status; }
-    {
-        const uint32_t prepare_blocks = static_cast<uint32_t>(std::min<uint64_t>((strands + 255u) / 256u,
-                                                                                 uint64_t(sms) * 8u));
-        const uint32_t chunk = ((strands + prepare_blocks - 1u) / prepare_blocks + 31u) / 32u * 32u;
-        dev::batched_prepare_kernel<<<std::max(1u, prepare_blocks), 256, 0, s>>>(b, chunk);
-        if ((status = record_cuda(cudaGetLastError()))) { return status; }
-    }
-    dev::batched_scan_kernel<<<count, 1024, 0, s>>>(b);
-    if ((status = record_cuda(cudaGetLastError()))) { return status; }
-    {
-        const uint32_t scatter_blocks = static_cast<uint32_t>(std::max(1, sms));
-        const uint32_t chunk = (strands + scatter_blocks - 1u) / scatter_blocks;
-        dev::batched_scatter_blocked_kernel<<<(strands + chunk - 1u) / chunk, 1024,
-                                              dev::kBatchScatterBins * sizeof(uint32_t), s>>>(b, chunk);
-    }
-    if ((status = record_cuda(cudaGetLastError()))) { return status; }
+    b.first_class = items[0] ? 0u : 1u;
     const uint32_t offset_blocks = static_cast<uint32_t>(std::min<uint64_t>((offsets + 255u) / 256u, uint64_t(sms) * 16u));
-    dev::batched_offsets_kernel<<<std::max(1u, offset_blocks), 256, 0, s>>>(b);
-    if ((status = record_cuda(cudaGetLastError()))) { return status; }
+    const uint32_t prepare_blocks = static_cast<uint32_t>(std::min<uint64_t>((strands + 255u) / 256u,
+                                                                             uint64_t(sms) * 8u));
+    const uint32_t prepare_chunk = ((strands + prepare_blocks - 1u) / prepare_blocks + 31u) / 32u * 32u;
+    const uint32_t scatter_chunk = (strands + static_cast<uint32_t>(std::max(1, sms)) - 1u) /
+                                   static_cast<uint32_t>(std::max(1, sms));
+    if ((status = launch_chained(false, dev::batched_offsets_kernel, std::max(1u, offset_blocks), 256u, 0u, s, b)) ||
+        (status = launch_chained(true, dev::batched_prepare_kernel, std::max(1u, prepare_blocks), 256u, 0u, s, b,
+                                 prepare_chunk)) ||
+        (status = launch_chained(true, dev::batched_scan_kernel, count, 1024u, 0u, s, b)) ||
+        (status = launch_chained(true, dev::batched_scatter_blocked_kernel,
+                                 (strands + scatter_chunk - 1u) / scatter_chunk, 1024u,
+                                 dev::kBatchScatterBins * sizeof(uint32_t), s, b, scatter_chunk))) {
+        return status;
+    }
 
     // One generate launch per class with work, in stream order; each runs
     // persistent CTAs at its own occupancy.
-    bool launched = false;
     for (uint32_t c = 0; c < kClasses; ++c) {
         if (items[c] == 0u) { continue; }
         const void *fn = kernel(c);
@@ -533,11 +537,9 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
         const uint32_t grid = static_cast<uint32_t>(
             std::min<uint64_t>(items[c], static_cast<uint64_t>(std::max(1, sms * std::max(per_sm, 1)))));
         void *args[] = {&b};
-        // Every class launch after the first of the frame is a programmatic
-        // dependent of the one before: its CTAs take the SMs that the earlier
-        // class's tail leaves idle.  That is safe because the classes share
-        // no output, and the strand order and offset tables they read were
-        // complete before the first class started.
+        // The first class's launch is chained to the scatter; the second is a
+        // programmatic dependent of the first that does not wait for its end: its
+        // CTAs take the SMs that the first class's tail leaves idle.
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3(grid);
         lc.blockDim = dim3(block);
@@ -545,11 +547,10 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
         lc.stream = s;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = launched ? 1 : 0;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
         lc.attrs = attr;
         lc.numAttrs = 1;
         if ((status = record_cuda(cudaLaunchKernelExC(&lc, fn, args)))) { return status; }
-        launched = true;
     }
     return record_cuda(cudaGetLastError());
 }

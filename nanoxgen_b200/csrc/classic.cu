@@ -151,15 +151,11 @@ uint32_t nxg_generate_packed_classic(const nxg_device_asset_desc *asset, const n
     }
     const auto s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
-    if ((error = nxg::launch_order(*asset, params->seed, first_strand, strand_count, params->cvs_per_strand,
-                                   workspace, s))) {
-        return error;
-    }
     const nxg_deformed_desc none{};
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
-                                workspace_bytes, s, nullptr, classic);
+                                workspace_bytes, s, nullptr, classic, false);
 }
 
 } // extern "C"

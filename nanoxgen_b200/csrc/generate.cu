@@ -2,19 +2,20 @@
 // points (nxg_generate_packed, nxg_generate_packed_range,
 // nxg_packed_workspace_size, nxg_query_strand_states).
 //
-// Pipeline per call, all enqueued on the caller's stream:
-//   1. strand_keys     : alias-sample every strand's root triangle and bin the
+// Pipeline per call, all enqueued on the caller's stream as chained launches
+// (chain_wait); 2 to 4 only where the strand order pays (wants_order):
+//   1. guide_offsets   : the frame's guide-offset table and guide frame
+//                        records;
+//   2. strand_keys     : alias-sample every strand's root triangle and bin the
 //                        strand by its triangle's nearest stencil guide
 //                        (a counting sort's histogram pass);
-//   2. exclusive_scan  : bin offsets;
-//   3. scatter_order   : the permutation that groups strands sharing guides,
+//   3. exclusive_scan  : bin offsets;
+//   4. scatter_order   : the permutation that groups strands sharing guides,
 //                        so one CTA's strands read the same guide CVs from L1
 //                        (ranks in shared memory per block, one global atomic
 //                        per block and bin);
-//   4. guide_offsets   : the frame's guide-offset table and guide frame
-//                        records;
-//   5. generate        : persistent CTAs walk contiguous ranges of the
-//                        permutation with the lane-walk generator
+//   5. generate        : persistent CTAs walk contiguous ranges of the strands
+//                        (in that order) with the lane-walk generator
 //                        (walk.cuh).  Where a lane-group tile is registered
 //                        (nxg_set_tile, up to 128 CVs): a group of L lanes
 //                        owns one strand, the transported frame as prefix
@@ -111,8 +112,10 @@ __global__ void __launch_bounds__(NOISE ? 32 * kWalkNoiseWarps : 256, NOISE ? 1 
     const uint32_t padded = walk_padded(P);
     float *tvals = reinterpret_cast<float *>(smem + (NOISE ? kTableFloat4 << walk_table_copies(blockDim.x >> 5) : 0));
     float *rvals = tvals + padded;
-    walk_fill_head<NOISE>(g, smem, tvals, rvals);
+    walk_fill_head<NOISE>(g, smem, tvals, rvals);  // of the asset and the arguments alone
     __syncthreads();
+    chain_start();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     unsigned char *mine = reinterpret_cast<unsigned char *>(rvals + padded) + walk_warp_bytes(NOISE, CLASSIC) * warp;
@@ -162,6 +165,8 @@ __global__ void classic_serial_apply_kernel(LaunchArgs g) {
 // output order (coalesced), for the frame (generate.h:101-135, :621-623).
 __global__ void strand_roots_kernel(LaunchArgs g) {
     __shared__ uint32_t staged[8][32 * 12];
+    chain_start();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t P = g.p.cvs_per_strand;
@@ -198,11 +203,16 @@ __global__ void strand_roots_kernel(LaunchArgs g) {
 }
 
 // The frame's guide-offset table (G x P float4) and, after it, the guide
-// frame records (2 float4 per guide) the lane-walk generator reads.
-__global__ void guide_offsets_kernel(AssetArgs a, FrameArgs f, uint32_t P, float support_scale, float4 *offsets) {
+// frame records (2 float4 per guide) the lane-walk generator reads; also
+// clears the `bins` words of a strand order that follows.
+__global__ void guide_offsets_kernel(AssetArgs a, FrameArgs f, uint32_t P, float support_scale, float4 *offsets,
+                                     uint32_t *hist, uint32_t bins) {
+    chain_start();
+    chain_wait();
     const uint64_t n = static_cast<uint64_t>(a.guide_count) * P;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     const uint64_t first = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    for (uint64_t k = first; k < bins; k += stride) { hist[k] = 0u; }
     for (uint64_t idx = first; idx < n; idx += stride) {
         offsets[idx] = guide_offset_entry(a, f, P, static_cast<uint32_t>(idx / P), static_cast<uint32_t>(idx % P));
     }
@@ -382,6 +392,8 @@ __global__ void strand_keys_kernel(AssetArgs a, uint32_t seed, uint32_t first, u
                                    uint32_t *hist, uint32_t bins) {
     extern __shared__ uint32_t local_hist[];
     const bool priv = bins <= kPrivateBins;
+    chain_start();
+    chain_wait();
     if (priv) {
         for (uint32_t b = threadIdx.x; b < bins; b += blockDim.x) { local_hist[b] = 0u; }
         __syncthreads();
@@ -409,6 +421,8 @@ __global__ void strand_keys_kernel(AssetArgs a, uint32_t seed, uint32_t first, u
 // Exclusive scan of n words in place, one CTA of 1024 threads.
 __global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t *data, uint32_t n) {
     __shared__ uint32_t warp_sums[32];
+    chain_start();
+    chain_wait();
     const uint32_t tid = threadIdx.x;
     const uint32_t per = (n + blockDim.x - 1u) / blockDim.x;
     const uint32_t lo = min(n, tid * per), hi = min(n, lo + per);
@@ -443,6 +457,8 @@ __global__ void __launch_bounds__(1024) exclusive_scan_kernel(uint32_t *data, ui
 
 __global__ void scatter_order_kernel(const uint32_t *keys, uint32_t *offsets, uint32_t count, uint32_t bins,
                                      uint32_t *order) {
+    chain_start();
+    chain_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t key = min(keys[i], bins - 1u);
         const uint32_t pos = atomicAdd(&offsets[key], 1u);
@@ -462,6 +478,8 @@ __global__ void __launch_bounds__(1024) scatter_order_blocked_kernel(const uint3
     const uint32_t begin = blockIdx.x * chunk;
     const uint32_t end = min(count, begin + chunk);
     for (uint32_t b = threadIdx.x; b < bins; b += blockDim.x) { slots[b] = 0u; }
+    chain_start();
+    chain_wait();
     __syncthreads();
     for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) { atomicAdd(&slots[min(keys[i], bins - 1u)], 1u); }
     __syncthreads();
@@ -736,12 +754,6 @@ KernelFn pick_kernel(int lanes, int ppt, bool noise, bool classic) {
     }
 }
 
-uint32_t launch_kernel(void (*fn)(LaunchArgs, const float4 *), uint32_t grid, uint32_t block, size_t shm,
-                       cudaStream_t stream, const LaunchArgs &g, const float4 *offsets) {
-    fn<<<grid, block, shm, stream>>>(g, offsets);
-    return record_cuda(cudaGetLastError());
-}
-
 // Dynamic shared memory of the lane-group kernels.
 size_t generate_smem_bytes(uint32_t P, int lanes, int ppt, bool noise, uint32_t warps) {
     const size_t per_warp = sizeof(uint32_t) * dev::kRecFields * 32u + sizeof(float4) * 32u / lanes * lanes * ppt +
@@ -779,8 +791,9 @@ uint32_t check_workspace(const nxg_device_asset_desc &asset, uint32_t count, uin
 
 // Counting sort of strands [first, first + count) by their triangle's first
 // stencil guide; leaves the permutation in the workspace's order section.
+// `cleared`: the launch before on the stream has cleared the bins.
 uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_t first, uint32_t count,
-                      uint32_t P, void *workspace, cudaStream_t stream) {
+                      uint32_t P, void *workspace, cudaStream_t stream, bool cleared) {
     const WorkspaceLayout ws = workspace_layout(asset.header.guide_count, count, P);
     auto *wbase = static_cast<unsigned char *>(workspace);
     auto *keys = reinterpret_cast<uint32_t *>(wbase + ws.keys);
@@ -789,41 +802,62 @@ uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_
     const uint32_t bins = asset.header.guide_count + 1u;
     const int sms = device_sm_count();
     const dev::AssetArgs a = resolve_asset(asset);
-    uint32_t status = record_cuda(cudaMemsetAsync(hist, 0, uint64_t{bins} * 4u, stream));
+    uint32_t status = cleared ? uint32_t{NXG_ERROR_NONE}
+                              : record_cuda(cudaMemsetAsync(hist, 0, uint64_t{bins} * 4u, stream));
     if (status) { return status; }
     const uint32_t threads = 256u;
     const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + threads - 1u) / threads,
                                                                       static_cast<uint64_t>(sms) * 4u));
     const size_t shm = bins <= dev::kPrivateBins ? bins * 4u : 0u;
-    dev::strand_keys_kernel<<<blocks, threads, shm, stream>>>(a, seed, first, count, keys, hist, bins);
-    if ((status = record_cuda(cudaGetLastError()))) { return status; }
-    dev::exclusive_scan_kernel<<<1, 1024, 0, stream>>>(hist, bins);
-    if ((status = record_cuda(cudaGetLastError()))) { return status; }
-    if (bins <= dev::kPrivateBins) {  // one block per SM, shared-memory ranks
-        const uint32_t scatter_blocks = static_cast<uint32_t>(std::max(1, sms));
-        const uint32_t chunk = (count + scatter_blocks - 1u) / scatter_blocks;
-        const uint32_t used = (count + chunk - 1u) / chunk;
-        if (bins * 4u > 48u * 1024u) {
-            if ((status = record_cuda(cudaFuncSetAttribute(dev::scatter_order_blocked_kernel,
-                                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           static_cast<int>(bins * 4u))))) {
-                return status;
-            }
-        }
-        dev::scatter_order_blocked_kernel<<<used, 1024, bins * 4u, stream>>>(keys, hist, count, bins, chunk, order);
-    } else {
-        dev::scatter_order_kernel<<<blocks, threads, 0, stream>>>(keys, hist, count, bins, order);
+    if ((status = launch_chained(cleared, dev::strand_keys_kernel, blocks, threads, shm, stream, a, seed, first,
+                                 count, keys, hist, bins)) ||
+        (status = launch_chained(true, dev::exclusive_scan_kernel, 1u, 1024u, 0u, stream, hist, bins))) {
+        return status;
     }
-    return record_cuda(cudaGetLastError());
+    if (bins > dev::kPrivateBins) {
+        return launch_chained(true, dev::scatter_order_kernel, blocks, threads, 0u, stream, keys, hist, count, bins,
+                              order);
+    }
+    // One block per SM, shared-memory ranks.
+    const uint32_t scatter_blocks = static_cast<uint32_t>(std::max(1, sms));
+    const uint32_t chunk = (count + scatter_blocks - 1u) / scatter_blocks;
+    const uint32_t used = (count + chunk - 1u) / chunk;
+    if (bins * 4u > 48u * 1024u) {
+        if ((status = record_cuda(cudaFuncSetAttribute(dev::scatter_order_blocked_kernel,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(bins * 4u))))) {
+            return status;
+        }
+    }
+    return launch_chained(true, dev::scatter_order_blocked_kernel, used, 1024u, bins * 4u, stream, keys, hist, count,
+                          bins, chunk, order);
 }
 
-// The generator over the strand order prepared in `workspace`: the
-// guide-offset table for this frame, then the persistent generate kernel.
+// Whether the lane walk takes its strands in the order of their guides.  The
+// order makes the warps of an SM read the same guide rows from L1, and costs
+// three launches, two passes over a key per strand, and scattered instead of
+// sequential outputs.  It pays where that locality is missing (a table beyond
+// L1) over enough points.  Whole calls, ordered against not, 4,096 guides:
+// with noise 100,000 x 32 86.2 / 78.7 us, 200,000 x 32 142.9 / 143.5, 300,000
+// x 32 198.2 / 207.6, 4,000,000 x 24 2,062 / 2,475; without noise, where more
+// warps hide the rows' latency, 200,000 x 16 61.5 / 51.3, 1,000,000 x 32 242.7
+// / 244.1, 300,000 x 100 200.0 / 203.4, and 2,000,000 x 32 519.6 / 472.1, the
+// root outputs (60 bytes per strand, partial sectors when scattered) no longer
+// fitting L2.
+// A motion call orders its strands once for all samples.
+bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, uint32_t samples) {
+    const uint64_t points = uint64_t{count} * P * samples;
+    if (uint64_t{guide_count} * P * 16u <= (uint64_t{128} << 10)) { return false; }
+    return noise ? points >= 7000000u : points >= 24000000u && count <= 1700000u;
+}
+
+// The guide-offset table for this frame, the strand order where one is wanted
+// and not prepared, then the persistent generate kernel.
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
                          uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
-                         const nxg_classic_apply_desc *classic) {
+                         const nxg_classic_apply_desc *classic, bool prepared, uint32_t samples) {
     set_last_cuda_error(0);
     const uint32_t P = params.cvs_per_strand;
     const WorkspaceLayout ws = workspace_layout(asset.header.guide_count, count, P);
@@ -849,6 +883,10 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     uint32_t status = NXG_ERROR_NONE;
     const bool parallel = parallel_path(asset.header.guide_count, P);
     if (!parallel && (!long_walk_path(asset.header.guide_count, count, P) || workspace_bytes < ws.wanted)) {
+        if (!prepared &&
+            (status = launch_order(asset, params.seed, first, count, P, workspace, stream, false))) {
+            return status;
+        }
         const uint32_t threads = 128u;
         const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + threads - 1u) / threads,
                                                                           static_cast<uint64_t>(sms) * 8u));
@@ -859,15 +897,28 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     }
     auto *offsets = reinterpret_cast<float4 *>(wbase + ws.offsets);
     g.guide_frames = offsets + uint64_t{asset.header.guide_count} * P;
+    const bool noise = g.p.noise != 0u;
+    // The lane walk, unless a lane-group tile is registered for these strands.
+    const uint32_t packed = registered_tile(P, noise);
+    const bool walk = packed == 0u || (packed & 0xffu) == 1u;
+    const bool ordered = !walk || wants_order(asset.header.guide_count, count, P, noise, samples);
     {
         const uint64_t n = uint64_t{asset.header.guide_count} * P;
         const uint32_t threads = 256u;
         const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n + threads - 1u) / threads,
                                                                           static_cast<uint64_t>(sms) * 16u));
-        dev::guide_offsets_kernel<<<blocks, threads, 0, stream>>>(g.a, g.f, P, g.p.support_scale, offsets);
-        if ((status = record_cuda(cudaGetLastError()))) { return status; }
+        const bool sort = ordered && !prepared;
+        // The first launch is an ordinary one.  (Chained to the walk of the
+        // motion sample before, its CTAs and the next walk's took the SMs that
+        // walk still needed: five samples of 250,000 x 24, 791 against 735 us.)
+        if ((status = launch_chained(false, dev::guide_offsets_kernel, blocks, threads, 0u, stream, g.a, g.f, P,
+                                     g.p.support_scale, offsets, reinterpret_cast<uint32_t *>(wbase + ws.hist),
+                                     sort ? asset.header.guide_count + 1u : 0u)) ||
+            (sort && (status = launch_order(asset, params.seed, first, count, P, workspace, stream, true)))) {
+            return status;
+        }
     }
-    const bool noise = g.p.noise != 0u;
+    if (!ordered) { g.order = nullptr; }
     const bool classic_scalars = g.scalars != nullptr;
     int device = 0, smem_optin = 48 * 1024;
     if (cudaGetDevice(&device) == cudaSuccess) {
@@ -899,20 +950,26 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
         per_sm = std::max(per_sm, 1);
         const uint64_t needed = (uint64_t{count} + per_warp * warps - 1u) / (uint64_t{per_warp} * warps);
         const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(needed, static_cast<uint64_t>(sms) * per_sm));
-        return grid ? launch_kernel(fn, grid, block, shm, stream, g, offsets) : NXG_ERROR_NONE;
+        return grid ? launch_chained(walk, fn, grid, block, shm, stream, g, static_cast<const float4 *>(offsets))
+                    : uint32_t{NXG_ERROR_NONE};
     };
-    // The lane walk, unless a lane-group tile is registered for these strands.
-    const uint32_t packed = registered_tile(P, noise);
-    if (packed == 0u || (packed & 0xffu) == 1u) {
+    if (walk) {
         uint32_t warps = packed ? std::max(1u, (packed >> 16) & 0xffu) : (noise ? dev::kWalkNoiseWarps : 8u);
         g.batch = 32u;
         if (packed == 0u) {
-            // A call that does not fill the GPU spreads over it: fewer strands
-            // per warp (a warp's time is mostly the walk along one strand,
-            // which they share, plus what it does strand by strand), then
-            // fewer warps per CTA.
-            const uint64_t slots = static_cast<uint64_t>(sms) * 4u;  // one warp per scheduler
-            while (g.batch > 8u && (uint64_t{count} + g.batch - 1u) / g.batch < slots) { g.batch /= 2u; }
+            // Every warp the GPU holds takes the same number of batches, of
+            // equal size: a multiple of four strands, what a base and a store
+            // pass take.  A warp's time is the walk along one strand, whatever
+            // their number, plus what it does strand by strand, so a call that
+            // leaves warps idle with full batches runs faster with smaller ones
+            // (20,000 strands x 160 CVs with noise 159 -> 113 us, x 100 CVs
+            // without 72 -> 31 us), and the last batches of a larger one are
+            // not nearly empty.  Below a warp per SM the CTAs shrink too.
+            const uint64_t slots = static_cast<uint64_t>(sms) * (noise ? dev::kWalkNoiseWarps
+                                                                       : (classic_scalars ? 16u : 24u));
+            const uint64_t rounds = (count + slots * 32u - 1u) / (slots * 32u);
+            const uint64_t share = (count + slots * rounds - 1u) / (slots * rounds);
+            g.batch = static_cast<uint32_t>(std::clamp<uint64_t>((share + 3u) / 4u * 4u, noise ? 8u : 4u, 32u));
             const uint64_t needed = (uint64_t{count} + g.batch - 1u) / g.batch;
             warps = static_cast<uint32_t>(std::min<uint64_t>(warps, (needed + sms - 1u) / sms));
         }
@@ -1003,15 +1060,11 @@ uint32_t nxg_generate_packed_range(const nxg_device_asset_desc *asset, const nxg
     }
     const auto s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
-    if ((error = nxg::launch_order(*asset, params->seed, first_strand, strand_count, params->cvs_per_strand,
-                                   workspace, s))) {
-        return error;
-    }
     const nxg_deformed_desc none{};
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
-                                workspace_bytes, s, nullptr, nullptr);
+                                workspace_bytes, s, nullptr, nullptr, false);
 }
 
 uint32_t nxg_prepare_strand_order(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
@@ -1033,7 +1086,7 @@ uint32_t nxg_prepare_strand_order(const nxg_device_asset_desc *asset, const nxg_
     }
     nxg::set_last_cuda_error(0);
     return nxg::launch_order(*asset, params->seed, first_strand, strand_count, params->cvs_per_strand, workspace,
-                             static_cast<cudaStream_t>(stream));
+                             static_cast<cudaStream_t>(stream), false);
 }
 
 uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1054,7 +1107,7 @@ uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset, const n
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
-                                workspace_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr);
+                                workspace_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr, true);
 }
 
 uint32_t nxg_query_strand_states(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1111,7 +1164,7 @@ uint32_t nxg_query_walk_states(const nxg_device_asset_desc *asset, const nxg_def
     const uint32_t threads = 256u;
     const uint32_t blocks = static_cast<uint32_t>(std::max<uint64_t>(1u, std::min<uint64_t>(
         (n + threads - 1u) / threads, static_cast<uint64_t>(nxg::device_sm_count()) * 16u)));
-    nxg::dev::guide_offsets_kernel<<<blocks, threads, 0, s>>>(g.a, g.f, P, g.p.support_scale, offsets);
+    nxg::dev::guide_offsets_kernel<<<blocks, threads, 0, s>>>(g.a, g.f, P, g.p.support_scale, offsets, nullptr, 0u);
     if ((error = nxg::record_cuda(cudaGetLastError()))) { return error; }
     nxg::dev::walk_states_kernel<<<(count + 31u) / 32u, 32, 0, s>>>(g, count,
                                                                   reinterpret_cast<nxg::dev::WalkDecision *>(out));
@@ -1277,13 +1330,10 @@ extern "C" uint32_t nxg_generate_motion_packed(const nxg_device_asset_desc *asse
     }
     const auto s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
-    if ((error = nxg::launch_order(*asset, params->seed, 0u, params->strand_count, params->cvs_per_strand,
-                                   workspace, s))) {
-        return error;
-    }
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, outputs[i], cfg, 0u,
-                                     params->strand_count, workspace, workspace_bytes, s, nullptr, nullptr);
+                                     params->strand_count, workspace, workspace_bytes, s, nullptr, nullptr,
+                                     i != 0u, sample_count);
     }
     return error;
 }
@@ -1303,17 +1353,14 @@ extern "C" uint32_t nxg_generate_motion(const nxg_device_asset_desc *asset, cons
     const nxg_launch_config cfg = config ? *config : nxg_launch_config{128u};
     const auto s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
-    if ((error = nxg::launch_order(*asset, params->seed, 0u, params->strand_count, params->cvs_per_strand,
-                                   workspace, s))) {
-        return error;
-    }
     const uint64_t per_sample = uint64_t{params->strand_count} * params->cvs_per_strand * 3u;
     nxg_packed_output_desc none{};
     none.radius_scale = 1.0f;
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         float *dst = reinterpret_cast<float *>(output->points) + per_sample * i;
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, none, cfg, 0u, params->strand_count,
-                                     workspace, workspace_bytes, s, dst, nullptr);
+                                     workspace, workspace_bytes, s, dst, nullptr,
+                                     i != 0u, sample_count);
     }
     return error;
 }

@@ -40,6 +40,14 @@ struct LaunchArgs {
     uint32_t classic_width;  // radius = 0.5 * max(scalars.y, 0) * radius_scale
 };
 
+// Kernels of one call are chained as programmatic dependent launches: each
+// lets the next one's CTAs be set up while it runs (chain_start) and touches
+// memory only once the one before has completed and its writes are visible
+// (chain_wait; a no-op in a kernel launched without the attribute).  That
+// takes the launch gaps out of a chain of short kernels.
+__device__ __forceinline__ void chain_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 constexpr int kTableFloat4 = NXG_NOISE_GRADIENT_COUNT;  // float4 entries of the staged table
 
 __device__ __forceinline__ uint32_t root_word(const Root &r, int w) {
@@ -631,11 +639,31 @@ uint32_t check_launch_inputs(const nxg_device_asset_desc &asset, const nxg_packe
 uint32_t check_workspace(const nxg_device_asset_desc &asset, uint32_t count, uint32_t P, const void *workspace,
                          uint64_t bytes);
 uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_t first, uint32_t count,
-                      uint32_t P, void *workspace, cudaStream_t stream);
+                      uint32_t P, void *workspace, cudaStream_t stream, bool cleared);
+// With `prepared`, the workspace holds the strand order of this range;
+// `samples` frames of it share that order.
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
                          uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
-                         const nxg_classic_apply_desc *classic);
+                         const nxg_classic_apply_desc *classic, bool prepared, uint32_t samples = 1u);
+
+// Launches `fn`; `chained`: as a programmatic dependent of the launch before it
+// on the stream (fn then calls chain_wait before it touches memory).
+template <class... Params, class... Args>
+uint32_t launch_chained(bool chained, void (*fn)(Params...), uint32_t grid, uint32_t block, size_t shm,
+                        cudaStream_t stream, const Args &...args) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(block);
+    config.dynamicSmemBytes = shm;
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attribute;
+    config.numAttrs = chained ? 1u : 0u;
+    return record_cuda(cudaLaunchKernelEx(&config, fn, args...));
+}
 
 } // namespace nxg

@@ -103,3 +103,22 @@ def test_classic_application(cuda, nxg_lib, sphere, cvs, noise):
         dropped = scalars[:, 1] < 1e-4 if width else np.zeros(S, bool)
         counts = out.point_counts.cpu().numpy()
         assert np.array_equal(counts, np.where(dropped, 0, cvs))
+
+
+@pytest.mark.parametrize("noise,strands", [(0.1, 250_000), (0.0, 800_000)])
+def test_ordered_and_unordered_strands_agree(cuda, nxg_lib, noise, strands):
+    """A call large enough to order its strands by guide gives the points and
+    roots of its ranges, which are not ordered, bit for bit."""
+    import torch
+    from nanoxgen_b200 import fixtures
+    from nanoxgen_b200.asset import build_asset
+    from nanoxgen_b200.generator import DeviceAsset, generate_packed
+    w = fixtures.large_sphere(strands=strands, guides=400, n_lon=60, n_rings=41)
+    params = w.params.copy(noise_amplitude=noise, noise_frequency=6.0)
+    d = DeviceAsset(build_asset(w.build_input, w.stencil_slots))
+    full = generate_packed(d, params)
+    for first, count in ((0, 70_001), (strands - 70_001, 70_001)):
+        part = generate_packed(d, params, first_strand=first, count=count)
+        assert torch.equal(part.points, full.points[first * 32:(first + count) * 32])
+        assert torch.equal(part.roots, full.roots[first:first + count])
+        assert torch.equal(part.root_uvs, full.root_uvs[first:first + count])
