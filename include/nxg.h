@@ -306,8 +306,8 @@ void nxg_free(void *pointer);
 int nxg_build_asset_device(const nxg_asset_build_input *input, void *stream, void **out_bytes,
                            uint64_t *out_size, char *message, uint64_t message_capacity);
 
-/* The stencil search alone on device buffers; enqueues one kernel on
- * `stream`.  positions [vertex_count] and triangles [triangle_count] are the
+/* The stencil search alone on device buffers; enqueues one to three kernels
+ * on `stream` (the rows of `stencil` serve as scratch until they are written).  positions [vertex_count] and triangles [triangle_count] are the
  * mesh; guide_roots [guide_count] are the guides' first CVs and
  * guide_normals their root normals normalized as the asset's guide records
  * hold them (nxg_guide_record.root_normal).  Writes stencil [triangle_count

@@ -7,20 +7,32 @@
 // a 200,000-triangle mesh with 4,096 guides), the only super-linear step of
 // the asset build.
 //
-// Layout: one thread per triangle, 128-thread CTAs; the guide roots (one
-// plane per axis) and normals stream through shared memory in tiles of
-// kStencilTile guides, read by every lane at the same address (broadcast).
-// The eight best candidates live in registers.  Scores use the exact
-// helpers of strand_math.cuh (__f*_rn, never contracted), so they equal the
-// host build's bit for bit, and the insertion replays the host's procedure
-// (host.cpp build_stencils), so the rows are identical even for ties and
-// non-finite scores.
+// Two searches, the same rows:
 //
-// Rejection: a candidate whose |centroid - root|^2 alone is above the
-// current eighth score cannot enter (the penalty only adds).  The kernel
-// tests four guides at a time with packed f32x2 arithmetic (about ten
-// issued instructions per candidate instead of twenty-three) and scores the
-// rare group that passes exactly.
+// All pairs (search_all): one thread per triangle, 128-thread CTAs; the guide
+// roots (one plane per axis) and normals stream through shared memory in tiles
+// of kStencilTile guides, read by every lane at the same address (broadcast).
+// The eight best candidates live in registers.  Scores use the exact helpers
+// of strand_math.cuh (__f*_rn, never contracted), so they equal the host
+// build's bit for bit, and the insertion replays the host's procedure
+// (host.cpp build_stencils), so the rows are identical even for ties and
+// non-finite scores.  A candidate whose |centroid - root|^2 alone is above the
+// current eighth score cannot enter (the penalty only adds); four guides at a
+// time are tested with packed f32x2 arithmetic and the rare group that passes
+// is scored exactly.  Bound by FP32 issue: 502 us for 200,000 triangles x
+// 4,096 guides.
+//
+// Clusters (search_clusters), for enough of both: the guides are sorted along
+// a Morton curve into clusters of 32 with bounding boxes, and a warp looks
+// only into clusters that some lane's eighth score does not rule out --
+// a handful of 128, since a mesh's neighbouring triangles share their guides.
+// For finite positions the (score, guide) order is a total one, so the eight
+// smallest do not depend on the order of search; a CTA that meets a wild
+// position (not finite, or beyond kWild) takes all pairs.  167 us at the size
+// above (sorting 21, search 106, the last rows' search partly beside it): bound
+// by the latency of a warp's chain of clusters.  The sorted guides need memory this entry point has no argument
+// for: they are put into the last rows of the output, whose triangles a second
+// kernel searches from its own shared-memory copy and writes last.
 //
 // guide_nearest_kernel, one warp per guide, finds each guide's nearest
 // other root for the automatic support radius (guide_count^2 distances).
@@ -30,6 +42,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cfloat>
+#include <cmath>
 #include <cstdint>
 
 namespace nxg {
@@ -37,7 +51,6 @@ namespace dev {
 namespace {
 
 constexpr uint32_t kStencilThreads = 128u;
-constexpr uint32_t kTrianglesPerThread = 1u;
 constexpr uint32_t kStencilTile = 512u;  // guides per shared-memory tile (14 KB)
 
 struct Candidate {
@@ -111,14 +124,15 @@ __device__ __forceinline__ float root_distance2(F3 centroid, const GuideTile &t,
 struct TriangleSearch {
     F3 centroid, face;
     f32x2 cx, cy, cz;  // the centroid's coordinates, each in both halves
-    bool live;
+    bool live, invalid;  // invalid: out of range, keeps an all-invalid row
     Candidate best[kSlots];
 };
 
 __device__ __forceinline__ void begin_triangle(TriangleSearch &t, uint32_t ti, const nxg_vec3 *__restrict__ positions,
                                                uint32_t vertex_count, const nxg_uint3 *__restrict__ triangles,
-                                               uint32_t triangle_count, uint32_t *__restrict__ stencil) {
+                                               uint32_t triangle_count) {
     t.live = ti < triangle_count;
+    t.invalid = false;
     t.centroid = F3{0.0f, 0.0f, 0.0f};
     t.face = F3{0.0f, 1.0f, 0.0f};
     if (t.live) {
@@ -129,10 +143,8 @@ __device__ __forceinline__ void begin_triangle(TriangleSearch &t, uint32_t ti, c
             t.centroid = xdiv(xadd(xadd(p0, p1), p2), 3.0f);
             t.face = xnormalize(xcross(xsub(p1, p0), xsub(p2, p0)));
         } else {
-            t.live = false;  // an out-of-range triangle keeps an all-invalid row
-            uint4 *row = reinterpret_cast<uint4 *>(stencil + static_cast<size_t>(ti) * kSlots);
-            row[0] = make_uint4(kInvalid, kInvalid, kInvalid, kInvalid);
-            row[1] = make_uint4(kInvalid, kInvalid, kInvalid, kInvalid);
+            t.live = false;
+            t.invalid = true;
         }
     }
     t.cx = pair2(t.centroid.x, t.centroid.x);
@@ -168,13 +180,46 @@ __device__ __forceinline__ void consider_group(TriangleSearch &t, const GuideTil
 
 __device__ __forceinline__ void end_triangle(const TriangleSearch &t, uint32_t ti, uint32_t keep,
                                              uint32_t *__restrict__ stencil) {
-    if (!t.live) { return; }
+    if (!t.live && !t.invalid) { return; }
     uint32_t out[kSlots];
 #pragma unroll
-    for (uint32_t k = 0; k < kSlots; ++k) { out[k] = k < keep ? t.best[k].guide : kInvalid; }
+    for (uint32_t k = 0; k < kSlots; ++k) { out[k] = t.live && k < keep ? t.best[k].guide : kInvalid; }
     uint4 *row = reinterpret_cast<uint4 *>(stencil + static_cast<size_t>(ti) * kSlots);
     row[0] = make_uint4(out[0], out[1], out[2], out[3]);
     row[1] = make_uint4(out[4], out[5], out[6], out[7]);
+}
+
+// The all-pairs search of a CTA's triangles (every thread calls it).
+__device__ __forceinline__ void search_all(TriangleSearch &t, GuideTile &tile, const nxg_vec3 *__restrict__ guide_roots,
+                                           const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count) {
+    const uint32_t count = guide_count < kSlots ? guide_count : kSlots;
+    for (uint32_t base = 0; base < guide_count; base += kStencilTile) {
+        const uint32_t n = guide_count - base < kStencilTile ? guide_count - base : kStencilTile;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const nxg_vec3 r = guide_roots[base + i], m = guide_normals[base + i];
+            tile.x[i] = r.x;
+            tile.y[i] = r.y;
+            tile.z[i] = r.z;
+            tile.normal[i] = make_float4(m.x, m.y, m.z, 0.0f);
+        }
+        __syncthreads();
+        if (!t.live) { continue; }
+        // The first `count` guides fill the lists (tile 0 only; count <= 8).
+        uint32_t j = base == 0u ? count : 0u;
+        for (uint32_t f = 0; f < j; ++f) {
+            consider(t.best, root_distance2(t.centroid, tile, f), f, count, t.face, tile.normal[f]);
+        }
+        for (; j + 4u <= n; j += 4u) {
+            const ulonglong2 gx = *reinterpret_cast<const ulonglong2 *>(&tile.x[j]);
+            const ulonglong2 gy = *reinterpret_cast<const ulonglong2 *>(&tile.y[j]);
+            const ulonglong2 gz = *reinterpret_cast<const ulonglong2 *>(&tile.z[j]);
+            consider_group(t, tile, j, base + j, count, gx, gy, gz);
+        }
+        for (; j < n; ++j) {
+            consider(t.best, root_distance2(t.centroid, tile, j), base + j, count, t.face, tile.normal[j]);
+        }
+    }
 }
 
 // One triangle per thread, 128-thread CTAs (56 registers, 9 CTAs per SM).
@@ -187,62 +232,463 @@ stencil_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count, co
                const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count, uint32_t keep,
                uint32_t *__restrict__ stencil) {
     __shared__ __align__(16) GuideTile tile;
-    const uint32_t first = blockIdx.x * (kStencilThreads * kTrianglesPerThread) + threadIdx.x;
-    TriangleSearch tri[kTrianglesPerThread];
-#pragma unroll
-    for (uint32_t q = 0; q < kTrianglesPerThread; ++q) {
-        begin_triangle(tri[q], first + q * kStencilThreads, positions, vertex_count, triangles, triangle_count,
-                       stencil);
-    }
-    bool any = false;
-#pragma unroll
-    for (uint32_t q = 0; q < kTrianglesPerThread; ++q) { any = any || tri[q].live; }
-    const uint32_t count = guide_count < kSlots ? guide_count : kSlots;
+    const uint32_t ti = blockIdx.x * kStencilThreads + threadIdx.x;
+    TriangleSearch t;
+    begin_triangle(t, ti, positions, vertex_count, triangles, triangle_count);
+    search_all(t, tile, guide_roots, guide_normals, guide_count);
+    end_triangle(t, ti, keep, stencil);
+}
 
-    for (uint32_t base = 0; base < guide_count; base += kStencilTile) {
-        const uint32_t n = guide_count - base < kStencilTile ? guide_count - base : kStencilTile;
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += kStencilThreads) {
-            const nxg_vec3 r = guide_roots[base + i], m = guide_normals[base + i];
-            tile.x[i] = r.x;
-            tile.y[i] = r.y;
-            tile.z[i] = r.z;
-            tile.normal[i] = make_float4(m.x, m.y, m.z, 0.0f);
-        }
-        __syncthreads();
-        if (!any) { continue; }
-        // The first `count` guides fill the lists (tile 0 only; count <= 8).
-        uint32_t j = base == 0u ? count : 0u;
-        for (uint32_t f = 0; f < j; ++f) {
+// ---------------------------------------------------------------------------
+// The cluster search.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kClusterGuides = 32u;
+constexpr uint32_t kClusterWords = 4u * kClusterGuides / 4u;  // float4 per cluster: planes x, y, z, guide index
+constexpr uint32_t kMaxClusters = 160u;    // 92 KB of shared memory in the second kernel
+constexpr uint32_t kTailCtas = 8u;         // CTAs of the second kernel, one thread-block cluster
+constexpr uint32_t kClusterMinGuides = 640u;
+constexpr float kWild = 1.0e15f;           // |coordinate| past it: |d|^2 could overflow
+
+constexpr uint32_t kClusterBoxes = 4u;     // float4 per cluster: roots' box low (and guide count), high, normals' box
+
+// Scratch: kClusterWords float4 per cluster | kClusterBoxes float4 per cluster
+// | one float4 (first word nonzero: a guide is wild).
+__host__ __device__ constexpr uint32_t cluster_scratch_words(uint32_t clusters) {
+    return clusters * (kClusterWords + kClusterBoxes) + 1u;
+}
+// Output rows (two float4 each) the scratch takes.
+__host__ __device__ constexpr uint32_t cluster_scratch_rows(uint32_t clusters) {
+    return (cluster_scratch_words(clusters) + 1u) / 2u;
+}
+
+__device__ __forceinline__ uint32_t spread3(uint32_t v) {  // bits of v three apart
+    uint32_t r = 0u;
 #pragma unroll
-            for (uint32_t q = 0; q < kTrianglesPerThread; ++q) {
-                if (tri[q].live) {
-                    consider(tri[q].best, root_distance2(tri[q].centroid, tile, f), f, count, tri[q].face,
-                             tile.normal[f]);
-                }
-            }
-        }
-        for (; j + 4u <= n; j += 4u) {
-            const ulonglong2 gx = *reinterpret_cast<const ulonglong2 *>(&tile.x[j]);
-            const ulonglong2 gy = *reinterpret_cast<const ulonglong2 *>(&tile.y[j]);
-            const ulonglong2 gz = *reinterpret_cast<const ulonglong2 *>(&tile.z[j]);
+    for (uint32_t k = 0; k < 4u; ++k) { r |= ((v >> k) & 1u) << (3u * k); }
+    return r;
+}
+
+// Sorts the guides by the Morton code of their cell (16 cells per axis of
+// the roots' box) and writes the scratch; one CTA.  The order within a cell is
+// arbitrary.
+__global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restrict__ guide_roots,
+                                                       const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count,
+                                                       uint32_t clusters, float4 *scratch) {
+    constexpr uint32_t kBits = 4u;  // 4,096 cells, of which a surface meets about a fifth
+    constexpr uint32_t bin_count = 1u << (3u * kBits);
+    __shared__ uint32_t bins[bin_count];
+    __shared__ float bounds[6][32];
+    __shared__ uint32_t warp_sums[32];
+    chain_start();
+    chain_wait();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    for (uint32_t i = tid; i < bin_count; i += 1024u) { bins[i] = 0u; }
+    constexpr uint32_t kOwn = (kMaxClusters * kClusterGuides + 1023u) / 1024u;  // guides of a thread
+    nxg_vec3 root[kOwn];
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    bool wild = false;
 #pragma unroll
-            for (uint32_t q = 0; q < kTrianglesPerThread; ++q) {
-                if (tri[q].live) { consider_group(tri[q], tile, j, base + j, count, gx, gy, gz); }
-            }
-        }
-        for (; j < n; ++j) {
+    for (uint32_t q = 0; q < kOwn; ++q) {
+        const uint32_t i = q * 1024u + tid;
+        root[q] = i < guide_count ? guide_roots[i] : nxg_vec3{0.0f, 0.0f, 0.0f};
+    }
 #pragma unroll
-            for (uint32_t q = 0; q < kTrianglesPerThread; ++q) {
-                if (tri[q].live) {
-                    consider(tri[q].best, root_distance2(tri[q].centroid, tile, j), base + j, count, tri[q].face,
-                             tile.normal[j]);
-                }
-            }
+    for (uint32_t q = 0; q < kOwn; ++q) {
+        if (q * 1024u + tid >= guide_count) { continue; }
+        const float v[3] = {root[q].x, root[q].y, root[q].z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            wild = wild || !(fabsf(v[k]) <= kWild);
+            lo[k] = fminf(lo[k], v[k]);
+            hi[k] = fmaxf(hi[k], v[k]);
         }
     }
 #pragma unroll
-    for (uint32_t q = 0; q < kTrianglesPerThread; ++q) { end_triangle(tri[q], first + q * kStencilThreads, keep, stencil); }
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+        }
+        if (lane == 0u) {
+            bounds[k][warp] = lo[k];
+            bounds[3 + k][warp] = hi[k];
+        }
+    }
+    wild = __syncthreads_or(wild);
+    if (tid == 0u) { scratch[clusters * (kClusterWords + kClusterBoxes)] = make_float4(wild ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f); }
+    if (wild) { return; }
+    float extent = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = bounds[k][lane];
+        hi[k] = bounds[3 + k][lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+        }
+        extent = fmaxf(extent, hi[k] - lo[k]);
+    }
+    const float cells = static_cast<float>(1u << kBits);
+    const float scale = extent > 0.0f ? cells / extent : 0.0f;
+    const auto cell = [&](nxg_vec3 r) {
+        const float v[3] = {r.x, r.y, r.z};
+        uint32_t code = 0u;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float q = fminf(fmaxf((v[k] - lo[k]) * scale, 0.0f), cells - 1.0f);
+            code |= spread3(static_cast<uint32_t>(q)) << k;
+        }
+        return min(code, bin_count - 1u);
+    };
+#pragma unroll
+    for (uint32_t q = 0; q < kOwn; ++q) {
+        if (q * 1024u + tid < guide_count) { atomicAdd(&bins[cell(root[q])], 1u); }
+    }
+    __syncthreads();
+    const uint32_t per = (bin_count + 1023u) / 1024u, begin = min(bin_count, tid * per),
+                   end = min(bin_count, begin + per);
+    uint32_t sum = 0u;
+    for (uint32_t i = begin; i < end; ++i) { sum += bins[i]; }
+    uint32_t incl = sum;
+#pragma unroll
+    for (uint32_t o = 1u; o < 32u; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) { incl += u; }
+    }
+    if (lane == 31u) { warp_sums[warp] = incl; }
+    __syncthreads();
+    uint32_t running = incl - sum + __reduce_add_sync(kFull, lane < warp ? warp_sums[lane] : 0u);
+    for (uint32_t i = begin; i < end; ++i) {
+        const uint32_t n = bins[i];
+        bins[i] = running;
+        running += n;
+    }
+    __syncthreads();
+    float *planes = reinterpret_cast<float *>(scratch);
+    const auto put = [planes](uint32_t at, nxg_vec3 r, uint32_t guide) {
+        float *plane = planes + (at / kClusterGuides) * (4u * kClusterWords) + at % kClusterGuides;
+        plane[0] = r.x;
+        plane[kClusterGuides] = r.y;
+        plane[2u * kClusterGuides] = r.z;
+        plane[3u * kClusterGuides] = __uint_as_float(guide);
+    };
+#pragma unroll
+    for (uint32_t q = 0; q < kOwn; ++q) {
+        const uint32_t i = q * 1024u + tid;
+        if (i < guide_count) { put(atomicAdd(&bins[cell(root[q])], 1u), root[q], i); }
+    }
+    // The last cluster's free entries: no guide, further than any.
+    for (uint32_t i = guide_count + tid; i < clusters * kClusterGuides; i += 1024u) {
+        put(i, nxg_vec3{1.0e18f, 1.0e18f, 1.0e18f}, kInvalid);
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (uint32_t c = warp; c < clusters; c += 32u) {
+        const float *plane = planes + c * (4u * kClusterWords) + lane;
+        const bool guide = c * kClusterGuides + lane < guide_count;
+        const uint32_t gi = __float_as_uint(plane[3u * kClusterGuides]);
+        const nxg_vec3 m = guide ? guide_normals[gi] : nxg_vec3{0.0f, 0.0f, 0.0f};
+        const float v[6] = {plane[0], plane[kClusterGuides], plane[2u * kClusterGuides], m.x, m.y, m.z};
+        // A normal that is not finite agrees with every face: a box of all.
+        const bool all = __any_sync(kFull, guide && !(fabsf(m.x) <= kWild && fabsf(m.y) <= kWild && fabsf(m.z) <= kWild));
+        float low[6], high[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            low[k] = guide ? v[k] : FLT_MAX;
+            high[k] = guide ? v[k] : -FLT_MAX;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                low[k] = fminf(low[k], __shfl_xor_sync(kFull, low[k], o));
+                high[k] = fmaxf(high[k], __shfl_xor_sync(kFull, high[k], o));
+            }
+        }
+        if (lane == 0u) {
+            float4 *box = scratch + clusters * kClusterWords + kClusterBoxes * c;
+            box[0] = make_float4(low[0], low[1], low[2],
+                                 static_cast<float>(min(kClusterGuides, guide_count - c * kClusterGuides)));
+            box[1] = make_float4(high[0], high[1], high[2], 0.0f);
+            box[2] = all ? make_float4(-kWild, -kWild, -kWild, 0.0f) : make_float4(low[3], low[4], low[5], 0.0f);
+            box[3] = all ? make_float4(kWild, kWild, kWild, 0.0f) : make_float4(high[3], high[4], high[5], 0.0f);
+        }
+    }
+}
+
+// Squared distance between the boxes [alo, ahi] and [blo, bhi].
+__device__ __forceinline__ float box_distance2(F3 alo, F3 ahi, float4 blo, float4 bhi) {
+    const float x = fmaxf(fmaxf(blo.x - ahi.x, alo.x - bhi.x), 0.0f);
+    const float y = fmaxf(fmaxf(blo.y - ahi.y, alo.y - bhi.y), 0.0f);
+    const float z = fmaxf(fmaxf(blo.z - ahi.z, alo.z - bhi.z), 0.0f);
+    return x * x + y * y + z * z;
+}
+
+// The warp's triangles as one: the middle of their centroids' box and the
+// largest distance of a centroid from it.
+struct WarpBall {
+    F3 middle;
+    float radius;
+};
+
+// A triangle whose nearest guide is penalised (a degenerate one, whose face
+// normal is (0, 1, 0) wherever it lies) has to reach guides that are not, past
+// all the near ones.  For those of a warp that share one face normal, where at
+// least eight guides agree with it, those eight come before every penalised
+// one, so to the end of the search only guides that agree matter to them, and
+// within `reach2` squared distance there are eight.
+constexpr float kPenalty = 1.0e20f;
+struct WarpAim {
+    bool active;   // some triangle of the warp is aimed
+    bool aimed;    // this lane's is
+    F3 face;
+    float reach2;
+};
+
+// What a guide has to be near enough for: the largest eighth score of the
+// other triangles (any guide), and of the aimed ones (one that agrees), there at
+// most their reach; -1 or 0 where there is no such triangle.
+struct WarpWorst {
+    float own, aimed;
+};
+__device__ __forceinline__ WarpWorst worst_scores(const TriangleSearch &t, const WarpAim &aim) {
+    // Non-negative floats order as their bits.
+    const uint32_t key = __float_as_uint(t.best[kSlots - 1].key);
+    WarpWorst w;
+    w.own = __uint_as_float(__reduce_max_sync(kFull, t.live && !aim.aimed ? key : 0u));
+    w.aimed = -1.0f;
+    if (aim.active) {
+        w.aimed = fminf(__uint_as_float(__reduce_max_sync(kFull, aim.aimed ? key : 0u)), aim.reach2);
+    }
+    return w;
+}
+
+// The guides of one cluster for this warp's triangles.  A lane takes one guide;
+// the lanes are sorted by their guides' distance from the warp's middle and
+// hand round, nearest first, those near enough for some triangle: in that
+// order few guides enter any list (a warp pays for an insertion of any of its
+// lanes), and the loop reads no memory.
+__device__ __forceinline__ void consider_cluster(TriangleSearch &t, const WarpBall &ball, const WarpAim &aim,
+                                                 const float4 *cluster, const nxg_vec3 *__restrict__ guide_normals) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float *plane = reinterpret_cast<const float *>(cluster) + lane;
+    const F3 own = {plane[0], plane[kClusterGuides], plane[2u * kClusterGuides]};
+    const uint32_t own_guide = __float_as_uint(plane[3u * kClusterGuides]);
+    const bool guide = own_guide != kInvalid;
+    const nxg_vec3 own_normal = guide ? guide_normals[own_guide] : nxg_vec3{0.0f, 0.0f, 0.0f};
+    const F3 off = own - ball.middle;
+    const float distance = guide ? sqrtf(dot(off, off)) : FLT_MAX;
+    // Bitonic sort of (distance, lane): the low five bits of the distance give
+    // way to the lane, which only blurs the order.
+    uint32_t key = (__float_as_uint(distance) & ~31u) | lane;
+#pragma unroll
+    for (uint32_t k = 2u; k <= 32u; k <<= 1) {
+#pragma unroll
+        for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
+            const uint32_t other = __shfl_xor_sync(kFull, key, j);
+            const bool up = (lane & k) == 0u, low = (lane & j) == 0u;
+            key = up == low ? min(key, other) : max(key, other);
+        }
+    }
+    const int from = static_cast<int>(key & 31u);
+    const F3 root = {__shfl_sync(kFull, own.x, from), __shfl_sync(kFull, own.y, from), __shfl_sync(kFull, own.z, from)};
+    const F3 normal = {__shfl_sync(kFull, own_normal.x, from), __shfl_sync(kFull, own_normal.y, from),
+                       __shfl_sync(kFull, own_normal.z, from)};
+    const uint32_t gi = __shfl_sync(kFull, own_guide, from);
+    // The least |d|^2 of this lane's guide from any of the triangles.
+    const float reach = fmaxf(__shfl_sync(kFull, distance, from) - ball.radius, 0.0f);
+    const float bound = gi != kInvalid ? reach * reach * kFilterMargin : FLT_MAX;
+    const bool agrees = aim.active && !(xdot(aim.face, normal) < -0.25f);
+    const auto near = [&]() {
+        const WarpWorst w = worst_scores(t, aim);
+        return __ballot_sync(kFull, gi != kInvalid && (bound <= w.own || (agrees && bound <= w.aimed)));
+    };
+    for (unsigned mask = near(); mask != 0u; mask &= mask - 1u) {
+        const int i = __ffs(mask) - 1;
+        const F3 d = xsub(t.centroid, F3{__shfl_sync(kFull, root.x, i), __shfl_sync(kFull, root.y, i),
+                                         __shfl_sync(kFull, root.z, i)});
+        const float l2 = xdot(d, d);
+        if (!__any_sync(kFull, t.live && !(t.best[kSlots - 1].key < l2))) { continue; }  // the penalty only adds
+        const F3 m = {__shfl_sync(kFull, normal.x, i), __shfl_sync(kFull, normal.y, i),
+                      __shfl_sync(kFull, normal.z, i)};
+        const Candidate c{__fadd_rn(l2, xdot(t.face, m) < -0.25f ? kPenalty : 0.0f), __shfl_sync(kFull, gi, i)};
+        const bool enters = t.live && candidate_less(c.key, c.guide, t.best[kSlots - 1].key, t.best[kSlots - 1].guide);
+        if (!__any_sync(kFull, enters)) { continue; }
+        if (enters) { insert_candidate(t.best, c, kSlots - 1u); }
+        mask &= near() | (1u << i);
+    }
+}
+
+// The range of dot(face, normal) over a box of normals, widened by more than
+// the rounding of both.
+__device__ __forceinline__ float2 dot_range(F3 face, float4 lo, float4 hi) {
+    const float x0 = face.x * lo.x, x1 = face.x * hi.x, y0 = face.y * lo.y, y1 = face.y * hi.y;
+    const float z0 = face.z * lo.z, z1 = face.z * hi.z;
+    const float slack = 1.0e-5f * (fmaxf(fabsf(x0), fabsf(x1)) + fmaxf(fabsf(y0), fabsf(y1)) + fmaxf(fabsf(z0), fabsf(z1)));
+    return make_float2(fminf(x0, x1) + fminf(y0, y1) + fminf(z0, z1) - slack,
+                       fmaxf(x0, x1) + fmaxf(y0, y1) + fmaxf(z0, z1) + slack);
+}
+
+// Finds the warp's aim for the triangles that the guide of `normal`, the
+// nearest to the warp's middle, is penalised for: the nearest (by its furthest
+// corner) cluster of at least eight guides that all agree with the face of the
+// first of them.  Every lane of the warp calls it.
+__device__ __forceinline__ WarpAim find_aim(const TriangleSearch &t, const WarpBall &ball, F3 normal,
+                                            const float4 *boxes, uint32_t clusters) {
+    WarpAim aim{false, false, F3{0.0f, 0.0f, 0.0f}, 0.0f};
+    const bool open = t.live && xdot(t.face, normal) < -0.25f;
+    const unsigned any = __ballot_sync(kFull, open);
+    if (any == 0u) { return aim; }
+    const int leader = __ffs(any) - 1;
+    aim.face = F3{__shfl_sync(kFull, t.face.x, leader), __shfl_sync(kFull, t.face.y, leader),
+                  __shfl_sync(kFull, t.face.z, leader)};
+    float nearest = FLT_MAX;
+    for (uint32_t c = threadIdx.x & 31u; c < clusters; c += 32u) {
+        const float4 *box = boxes + kClusterBoxes * c;
+        if (box[0].w < static_cast<float>(kSlots) || dot_range(aim.face, box[2], box[3]).x < -0.25f) { continue; }
+        const F3 far = {fmaxf(fabsf(box[0].x - ball.middle.x), fabsf(box[1].x - ball.middle.x)),
+                        fmaxf(fabsf(box[0].y - ball.middle.y), fabsf(box[1].y - ball.middle.y)),
+                        fmaxf(fabsf(box[0].z - ball.middle.z), fabsf(box[1].z - ball.middle.z))};
+        nearest = fminf(nearest, sqrtf(dot(far, far)));
+    }
+    nearest = __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(nearest)));
+    if (nearest == FLT_MAX) { return aim; }
+    const float reach = nearest + ball.radius;
+    aim.reach2 = reach * reach * 1.00002f;
+    aim.active = aim.reach2 < 0.5f * kPenalty;
+    aim.aimed = aim.active && open && t.face.x == aim.face.x && t.face.y == aim.face.y && t.face.z == aim.face.z;
+    return aim;
+}
+
+// The search of this warp's triangles over the scratch's clusters; every lane
+// of the warp calls it.  The nearest cluster first (its guides give bounds
+// near the final ones), then, 32 clusters at a time and nearest first, those
+// whose box is near enough to the box of the warp's centroids.  A box or ball
+// distance is at most the computed |d|^2 of any pair it covers but for
+// rounding, which kFilterMargin covers.
+__device__ __forceinline__ void search_clusters(TriangleSearch &t, const float4 *scratch, uint32_t clusters,
+                                                const nxg_vec3 *__restrict__ guide_normals) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float4 *boxes = scratch + clusters * kClusterWords;
+#pragma unroll
+    for (uint32_t k = 0; k < kSlots; ++k) { t.best[k] = {INFINITY, kInvalid}; }
+    if (__ballot_sync(kFull, t.live) == 0u) { return; }
+    F3 lo = t.live ? t.centroid : F3{FLT_MAX, FLT_MAX, FLT_MAX};
+    F3 hi = t.live ? t.centroid : F3{-FLT_MAX, -FLT_MAX, -FLT_MAX};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = F3{fminf(lo.x, __shfl_xor_sync(kFull, lo.x, o)), fminf(lo.y, __shfl_xor_sync(kFull, lo.y, o)),
+                fminf(lo.z, __shfl_xor_sync(kFull, lo.z, o))};
+        hi = F3{fmaxf(hi.x, __shfl_xor_sync(kFull, hi.x, o)), fmaxf(hi.y, __shfl_xor_sync(kFull, hi.y, o)),
+                fmaxf(hi.z, __shfl_xor_sync(kFull, hi.z, o))};
+    }
+    WarpBall ball;
+    ball.middle = (lo + hi) * 0.5f;
+    const F3 out = t.centroid - ball.middle;
+    // (Rounded up: the radius is subtracted from distances to the middle, whose
+    // own rounding is relative to the coordinates.)
+    const F3 size = {fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y)),
+                     fmaxf(fabsf(lo.z), fabsf(hi.z))};
+    const float slack = 1.0e-6f * (size.x + size.y + size.z);
+    ball.radius = __uint_as_float(__reduce_max_sync(
+                      kFull, t.live ? __float_as_uint(sqrtf(dot(out, out)) * 1.000001f) : 0u)) + slack;
+    float nearest = FLT_MAX;
+    uint32_t first = 0u;
+    for (uint32_t c = lane; c < clusters; c += 32u) {
+        const float d = box_distance2(ball.middle, ball.middle, boxes[kClusterBoxes * c], boxes[kClusterBoxes * c + 1u]);
+        if (d < nearest) {
+            nearest = d;
+            first = c;
+        }
+    }
+    const uint32_t least = __reduce_min_sync(kFull, __float_as_uint(nearest));
+    first = __shfl_sync(kFull, first, __ffs(__ballot_sync(kFull, __float_as_uint(nearest) == least)) - 1);
+    F3 normal;
+    {
+        const float *plane = reinterpret_cast<const float *>(scratch + first * kClusterWords) + lane;
+        const F3 off = F3{plane[0], plane[kClusterGuides], plane[2u * kClusterGuides]} - ball.middle;
+        const uint32_t gi = __float_as_uint(plane[3u * kClusterGuides]);
+        const uint32_t bits = __float_as_uint(gi == kInvalid ? FLT_MAX : dot(off, off));
+        const int lead = __ffs(__ballot_sync(kFull, bits == __reduce_min_sync(kFull, bits))) - 1;
+        const nxg_vec3 m = guide_normals[__shfl_sync(kFull, gi, lead)];
+        normal = F3{m.x, m.y, m.z};
+    }
+    const WarpAim aim = find_aim(t, ball, normal, boxes, clusters);
+    consider_cluster(t, ball, aim, scratch + first * kClusterWords, guide_normals);
+    for (uint32_t base = 0; base < clusters; base += 32u) {
+        const float4 *mine = boxes + kClusterBoxes * (base + lane);
+        float box = FLT_MAX;
+        bool agrees = false;
+        if (base + lane < clusters && base + lane != first) {
+            box = box_distance2(lo, hi, mine[0], mine[1]) * kFilterMargin;
+            agrees = aim.active && !(dot_range(aim.face, mine[2], mine[3]).y < -0.25f);
+        }
+        for (uint32_t guard = 0; guard < 32u; ++guard) {
+            const WarpWorst worst = worst_scores(t, aim);
+            const bool near = box <= worst.own || (agrees && box <= worst.aimed);
+            const uint32_t next = __reduce_min_sync(kFull, __float_as_uint(near ? box : FLT_MAX));
+            if (next == __float_as_uint(FLT_MAX)) { break; }
+            const uint32_t c = static_cast<uint32_t>(__ffs(__ballot_sync(kFull, near && __float_as_uint(box) == next))) - 1u;
+            if (lane == c) { box = FLT_MAX; }
+            consider_cluster(t, ball, aim, scratch + (base + c) * kClusterWords, guide_normals);
+        }
+    }
+}
+
+__device__ __forceinline__ bool wild_triangle(const TriangleSearch &t) {
+    return t.live && !(fabsf(t.centroid.x) <= kWild && fabsf(t.centroid.y) <= kWild && fabsf(t.centroid.z) <= kWild);
+}
+
+// Triangles [0, searched) from the scratch in global memory (the rows from
+// `searched` on).
+__global__ void __launch_bounds__(kStencilThreads)
+stencil_cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
+                       const nxg_uint3 *__restrict__ triangles, uint32_t searched,
+                       const nxg_vec3 *__restrict__ guide_roots, const nxg_vec3 *__restrict__ guide_normals,
+                       uint32_t guide_count, uint32_t clusters, uint32_t keep, uint32_t *stencil) {
+    __shared__ __align__(16) GuideTile tile;
+    chain_wait();
+    chain_start();  // from here on the scratch is complete, which the next kernel relies on
+    const uint32_t ti = blockIdx.x * kStencilThreads + threadIdx.x;
+    TriangleSearch t;
+    begin_triangle(t, ti, positions, vertex_count, triangles, searched);
+    const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(searched) * kSlots);
+    const bool wild = scratch[clusters * (kClusterWords + kClusterBoxes)].x != 0.0f || wild_triangle(t);
+    if (__syncthreads_or(wild)) {
+        search_all(t, tile, guide_roots, guide_normals, guide_count);
+    } else {
+        search_clusters(t, scratch, clusters, guide_normals);
+    }
+    end_triangle(t, ti, keep, stencil);
+}
+
+// The rows the scratch is in: one thread-block cluster, whose CTAs copy the
+// scratch to shared memory before any of them writes a row.  It starts once
+// every CTA of stencil_cluster_kernel has seen the scratch complete, searches
+// beside that kernel's end and writes after it.
+__global__ void __launch_bounds__(1024)
+stencil_tail_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
+                    const nxg_uint3 *__restrict__ triangles, uint32_t searched, uint32_t triangle_count,
+                    const nxg_vec3 *__restrict__ guide_roots, const nxg_vec3 *__restrict__ guide_normals,
+                    uint32_t guide_count, uint32_t clusters, uint32_t keep, uint32_t *stencil) {
+    extern __shared__ float4 copy[];
+    __shared__ __align__(16) GuideTile tile;
+    const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(searched) * kSlots);
+    for (uint32_t i = threadIdx.x; i < cluster_scratch_words(clusters); i += blockDim.x) {
+        copy[i] = __ldcg(scratch + i);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const uint32_t ti = searched + blockIdx.x * blockDim.x + threadIdx.x;
+    TriangleSearch t;
+    begin_triangle(t, ti, positions, vertex_count, triangles, triangle_count);
+    const bool wild = copy[clusters * (kClusterWords + kClusterBoxes)].x != 0.0f || wild_triangle(t);
+    if (__syncthreads_or(wild)) {
+        search_all(t, tile, guide_roots, guide_normals, guide_count);
+    } else {
+        search_clusters(t, copy, clusters, guide_normals);
+    }
+    chain_wait();
+    end_triangle(t, ti, keep, stencil);
 }
 
 // Distance from every guide root to its nearest other root (the automatic
@@ -279,12 +725,55 @@ uint32_t slots_kept(uint32_t guide_count, uint32_t stencil_slots) {
 cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, const nxg_uint3 *triangles,
                          uint32_t triangle_count, const nxg_vec3 *guide_roots, const nxg_vec3 *guide_normals,
                          uint32_t guide_count, uint32_t stencil_slots, uint32_t *stencil, cudaStream_t stream) {
-    const uint32_t per_block = kStencilThreads * kTrianglesPerThread;
-    const uint32_t blocks = (triangle_count + per_block - 1u) / per_block;
-    stencil_kernel<<<blocks, kStencilThreads, 0, stream>>>(positions, vertex_count, triangles, triangle_count,
-                                                           guide_roots, guide_normals, guide_count,
-                                                           slots_kept(guide_count, stencil_slots), stencil);
-    return cudaGetLastError();
+    const uint32_t keep = slots_kept(guide_count, stencil_slots);
+    const uint32_t clusters = (guide_count + kClusterGuides - 1u) / kClusterGuides;
+    const uint32_t rows = cluster_scratch_rows(clusters);
+    // The cluster search where it is faster: enough pairs to pay for the sort
+    // (all pairs against clusters: 20,000 x 1,000 96 / 80 us, 20,000 x 640 72 /
+    // 105, 200,000 x 640 123 / 81), triangles close enough together that a warp
+    // shares its guides (50,000 x 4,096 320 / 190 us, 10,000 x 4,096 297 / 429),
+    // and up to kMaxClusters.
+    if (guide_count < kClusterMinGuides || clusters > kMaxClusters || triangle_count / 12u < guide_count ||
+        uint64_t{triangle_count} * guide_count < 20000000u) {
+        const uint32_t blocks = (triangle_count + kStencilThreads - 1u) / kStencilThreads;
+        stencil_kernel<<<blocks, kStencilThreads, 0, stream>>>(positions, vertex_count, triangles, triangle_count,
+                                                               guide_roots, guide_normals, guide_count, keep, stencil);
+        return cudaGetLastError();
+    }
+    const uint32_t searched = triangle_count - rows;
+    const size_t copy = sizeof(float4) * cluster_scratch_words(clusters);
+    const uint32_t tail_threads = ((rows + kTailCtas - 1u) / kTailCtas + 31u) / 32u * 32u;
+    cudaError_t e = cudaFuncSetAttribute(stencil_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(copy));
+    if (e != cudaSuccess) { return e; }
+    cudaLaunchConfig_t config{};
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = kTailCtas;
+    attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1u;
+    config.stream = stream;
+    config.attrs = attributes;
+    config.gridDim = dim3(1);
+    config.blockDim = dim3(1024);
+    config.dynamicSmemBytes = 0u;
+    e = cudaLaunchKernelEx(&config, cluster_kernel, guide_roots, guide_normals, guide_count, clusters,
+                           reinterpret_cast<float4 *>(stencil + static_cast<size_t>(searched) * kSlots));
+    if (e != cudaSuccess) { return e; }
+    config.numAttrs = 1u;
+    config.gridDim = dim3((searched + kStencilThreads - 1u) / kStencilThreads);
+    config.blockDim = dim3(kStencilThreads);
+    config.dynamicSmemBytes = 0u;
+    e = cudaLaunchKernelEx(&config, stencil_cluster_kernel, positions, vertex_count, triangles, searched, guide_roots,
+                           guide_normals, guide_count, clusters, keep, stencil);
+    if (e != cudaSuccess) { return e; }
+    config.numAttrs = 2u;
+    config.gridDim = dim3(kTailCtas);
+    config.blockDim = dim3(tail_threads);
+    config.dynamicSmemBytes = copy;
+    return cudaLaunchKernelEx(&config, stencil_tail_kernel, positions, vertex_count, triangles, searched,
+                              triangle_count, guide_roots, guide_normals, guide_count, clusters, keep, stencil);
 }
 
 size_t align256(size_t n) { return (n + 255u) & ~size_t{255u}; }
