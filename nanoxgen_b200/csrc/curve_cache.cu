@@ -12,6 +12,7 @@
 // points.  The content hash is a serial chain over 64-bit words (each step
 // multiplies the previous hash), so it has no parallel form and stays on the
 // host.
+#include "launch.cuh"
 #include "nxg.h"
 #include "nxg_cache.h"
 #include "nxg_internal.h"
@@ -281,6 +282,8 @@ struct CheckArgs {
 enum : int { kBadCount = 0, kBadPoint, kBadTexcoord, kBadMotion, kBadPatch, kBadFace };
 
 __global__ void check_init_kernel(nxg_curve_cache_check *r) {
+    dev::chain_start();
+    dev::chain_wait();
     if (threadIdx.x < 8u) { r->first_bad[threadIdx.x] = ~0ull; }
     if (threadIdx.x == 0u) {
         r->error = NXG_CACHE_OK;
@@ -300,84 +303,113 @@ __device__ __forceinline__ bool finite_f(float x) { return isfinite(x); }
 
 // One pass over the device copy: every element check records its first
 // failing index (atomicMin, taken only on a failure); the counts and the bit
-// checksum accumulate per thread across the grid-stride loops and leave as
-// one warp sum and one atomicAdd per warp.
-__global__ void __launch_bounds__(256) check_kernel(const CheckArgs a) {
-    nxg_curve_cache_check *r = a.result;
-    const uint64_t stride = uint64_t{gridDim.x} * blockDim.x;
-    const uint64_t start = uint64_t{blockIdx.x} * blockDim.x + threadIdx.x;
-    uint64_t count_sum = 0u, checksum = 0u;
-    // point counts
-    const uint32_t *counts = reinterpret_cast<const uint32_t *>(a.blob + a.counts_offset);
-    for (uint64_t s = start; s < a.strands; s += stride) {
-        const uint32_t c = __ldcs(counts + s);
-        if (c < 2u) { atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadCount]), s); }
-        count_sum += c;
+// checksum accumulate per thread and leave as one warp sum and one atomicAdd
+// per warp.
+//
+// Bound by HBM: every section is cut into tiles of kCheckTile elements, all
+// tiles dealt round the CTAs, four elements per thread with their loads issued
+// before any is used.  (Section after section over the whole grid, the short
+// sections each cost a latency that nothing else filled: 400,000 x 24 with
+// strand uvs 36 us, in tiles 30 us.)
+constexpr uint32_t kCheckUnroll = 4u;
+constexpr uint32_t kCheckTile = 256u * kCheckUnroll;
+
+__device__ __forceinline__ uint64_t check_tiles(uint64_t n) { return (n + kCheckTile - 1u) / kCheckTile; }
+
+// Flags the first non-finite pair of a float2 section's tile.
+__device__ __forceinline__ void check_pairs(const float2 *v, uint64_t base, uint64_t n, uint64_t *bad) {
+    float2 t[kCheckUnroll];
+#pragma unroll
+    for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+        const uint64_t i = base + u * 256u;
+        t[u] = i < n ? __ldcs(v + i) : make_float2(0.0f, 0.0f);
     }
-    // points (with their texcoords) and the bit checksum: four points per
-    // thread and pass, their loads issued before any is used
-    const float4 *points = reinterpret_cast<const float4 *>(a.blob + a.points_offset);
-    const float2 *tex = a.texcoords_offset ? reinterpret_cast<const float2 *>(a.blob + a.texcoords_offset) : nullptr;
-    constexpr int kUnroll = 4;
-    for (uint64_t base = start; base < a.points; base += kUnroll * stride) {
-        float4 p[kUnroll];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const uint64_t i = base + u * stride;
-            p[u] = i < a.points ? __ldcs(points + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+        if (!finite_f(t[u].x) || !finite_f(t[u].y)) {
+            atomicMin(reinterpret_cast<unsigned long long *>(bad), base + u * 256u);
         }
+    }
+}
+
+__global__ void __launch_bounds__(256) check_kernel(const __grid_constant__ CheckArgs a) {
+    dev::chain_start();
+    dev::chain_wait();
+    nxg_curve_cache_check *r = a.result;
+    uint64_t count_sum = 0u, checksum = 0u;
+    const uint64_t point_tiles = check_tiles(a.points), strand_tiles = check_tiles(a.strands);
+    const uint64_t motion_tiles = check_tiles(a.motion_count);
+    // Tiles: points | texcoords | motion points | counts | patch uvs | face uvs.
+    const uint64_t tex_end = point_tiles + (a.texcoords_offset ? point_tiles : 0u);
+    const uint64_t motion_end = tex_end + motion_tiles;
+    const uint64_t count_end = motion_end + strand_tiles;
+    const uint64_t patch_end = count_end + (a.patch_offset ? strand_tiles : 0u);
+    const uint64_t end = patch_end + (a.face_offset ? strand_tiles : 0u);
+    for (uint64_t tile = blockIdx.x; tile < end; tile += gridDim.x) {
+        if (tile < point_tiles) {  // points and the bit checksum
+            const float4 *points = reinterpret_cast<const float4 *>(a.blob + a.points_offset);
+            const uint64_t base = tile * kCheckTile + threadIdx.x;
+            float4 p[kCheckUnroll];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const uint64_t i = base + u * stride;
-            if (i >= a.points) { break; }
-            if (!finite_f(p[u].x) || !finite_f(p[u].y) || !finite_f(p[u].z) || !finite_f(p[u].w) ||
-                p[u].w < 0.0f) {
-                atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadPoint]), i);
+            for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+                const uint64_t i = base + u * 256u;
+                p[u] = i < a.points ? __ldcs(points + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            if (tex) {
-                const float2 t = __ldcs(tex + i);
-                if (!finite_f(t.x) || !finite_f(t.y)) {
-                    atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadTexcoord]), i);
+#pragma unroll
+            for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+                const uint64_t i = base + u * 256u;
+                if (i >= a.points) { break; }
+                if (!finite_f(p[u].x) || !finite_f(p[u].y) || !finite_f(p[u].z) || !finite_f(p[u].w) ||
+                    p[u].w < 0.0f) {
+                    atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadPoint]), i);
+                }
+                const uint64_t xy = uint64_t{__float_as_uint(p[u].x)} | (uint64_t{__float_as_uint(p[u].y)} << 32u);
+                const uint64_t zw = uint64_t{__float_as_uint(p[u].z)} | (uint64_t{__float_as_uint(p[u].w)} << 32u);
+                checksum += point_term(xy, zw, i);
+            }
+        } else if (tile < tex_end) {
+            check_pairs(reinterpret_cast<const float2 *>(a.blob + a.texcoords_offset),
+                        (tile - point_tiles) * kCheckTile + threadIdx.x, a.points, &r->first_bad[kBadTexcoord]);
+        } else if (tile < motion_end) {  // motion points (xyz, 4-byte aligned)
+            const float *motion = reinterpret_cast<const float *>(a.blob + a.motion_points_offset);
+            const uint64_t base = (tile - tex_end) * kCheckTile + threadIdx.x;
+            float v[kCheckUnroll][3];
+#pragma unroll
+            for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+                const uint64_t i = base + u * 256u;
+#pragma unroll
+                for (uint32_t k = 0; k < 3u; ++k) { v[u][k] = i < a.motion_count ? __ldcs(motion + 3u * i + k) : 0.0f; }
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+                if (!finite_f(v[u][0]) || !finite_f(v[u][1]) || !finite_f(v[u][2])) {
+                    atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadMotion]), base + u * 256u);
                 }
             }
-            const uint64_t xy = uint64_t{__float_as_uint(p[u].x)} | (uint64_t{__float_as_uint(p[u].y)} << 32u);
-            const uint64_t zw = uint64_t{__float_as_uint(p[u].z)} | (uint64_t{__float_as_uint(p[u].w)} << 32u);
-            checksum += point_term(xy, zw, i);
+        } else if (tile < count_end) {
+            const uint32_t *counts = reinterpret_cast<const uint32_t *>(a.blob + a.counts_offset);
+            const uint64_t base = (tile - motion_end) * kCheckTile + threadIdx.x;
+#pragma unroll
+            for (uint32_t u = 0; u < kCheckUnroll; ++u) {
+                const uint64_t s = base + u * 256u;
+                if (s >= a.strands) { break; }
+                const uint32_t c = __ldcs(counts + s);
+                if (c < 2u) { atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadCount]), s); }
+                count_sum += c;
+            }
+        } else if (tile < patch_end) {
+            check_pairs(reinterpret_cast<const float2 *>(a.blob + a.patch_offset),
+                        (tile - count_end) * kCheckTile + threadIdx.x, a.strands, &r->first_bad[kBadPatch]);
+        } else {
+            check_pairs(reinterpret_cast<const float2 *>(a.blob + a.face_offset),
+                        (tile - patch_end) * kCheckTile + threadIdx.x, a.strands, &r->first_bad[kBadFace]);
         }
     }
     count_sum = warp_sum(count_sum);
     checksum = warp_sum(checksum);
     if ((threadIdx.x & 31u) == 0u) {
         if (count_sum) { atomicAdd(reinterpret_cast<unsigned long long *>(&r->point_sum), count_sum); }
-        atomicAdd(reinterpret_cast<unsigned long long *>(&r->checksum), checksum);
-    }
-    const uint64_t first = uint64_t{blockIdx.x} * blockDim.x;
-    // motion points (xyz, 4-byte aligned)
-    const float *motion = reinterpret_cast<const float *>(a.blob + a.motion_points_offset);
-    for (uint64_t i = first + threadIdx.x; i < a.motion_count; i += stride) {
-        const float x = __ldcs(motion + 3u * i), y = __ldcs(motion + 3u * i + 1u), z = __ldcs(motion + 3u * i + 2u);
-        if (!finite_f(x) || !finite_f(y) || !finite_f(z)) {
-            atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadMotion]), i);
-        }
-    }
-    // strand uvs
-    const float2 *patch = a.patch_offset ? reinterpret_cast<const float2 *>(a.blob + a.patch_offset) : nullptr;
-    const float2 *face = a.face_offset ? reinterpret_cast<const float2 *>(a.blob + a.face_offset) : nullptr;
-    if (patch || face) {
-        for (uint64_t s = first + threadIdx.x; s < a.strands; s += stride) {
-            if (patch) {
-                const float2 t = __ldcs(patch + s);
-                if (!finite_f(t.x) || !finite_f(t.y)) {
-                    atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadPatch]), s);
-                }
-            }
-            if (face) {
-                const float2 t = __ldcs(face + s);
-                if (!finite_f(t.x) || !finite_f(t.y)) {
-                    atomicMin(reinterpret_cast<unsigned long long *>(&r->first_bad[kBadFace]), s);
-                }
-            }
-        }
+        if (checksum) { atomicAdd(reinterpret_cast<unsigned long long *>(&r->checksum), checksum); }
     }
 }
 
@@ -386,6 +418,7 @@ __global__ void __launch_bounds__(256) check_kernel(const CheckArgs a) {
 // index), motion times (serial, here), motion points, the strand loop
 // (patch uv before face uv at one index).
 __global__ void check_finish_kernel(const CheckArgs a) {
+    dev::chain_wait();
     nxg_curve_cache_check *r = a.result;
     const uint64_t *b = r->first_bad;
     uint32_t e = NXG_CACHE_OK;
@@ -526,19 +559,21 @@ uint32_t nxg_curve_cache_validate_device(const nxg_curve_cache_header *header, c
     a.samples = h.motion_sample_count;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
-    nxg::cache::check_init_kernel<<<1, 32, 0, s>>>(device_result);
+    if (const uint32_t st = nxg::launch_chained(false, nxg::cache::check_init_kernel, 1u, 32u, 0u, s, device_result)) {
+        return st;
+    }
     int per_sm = 0;
     if (const uint32_t st = nxg::record_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &per_sm, nxg::cache::check_kernel, 256, 0))) {
         return st;
     }
-    const uint64_t largest = std::max<uint64_t>({a.points, a.motion_count, a.strands});
-    const uint64_t needed = (largest + 255u) / 256u;
+    const auto tiles = [](uint64_t n) { return (n + nxg::cache::kCheckTile - 1u) / nxg::cache::kCheckTile; };
+    const uint64_t needed = tiles(a.points) * (a.texcoords_offset ? 2u : 1u) + tiles(a.motion_count) +
+                            tiles(a.strands) * (1u + (a.patch_offset ? 1u : 0u) + (a.face_offset ? 1u : 0u));
     const uint32_t grid = static_cast<uint32_t>(
         std::max<uint64_t>(1u, std::min<uint64_t>(needed, uint64_t(nxg::device_sm_count()) * std::max(per_sm, 1))));
-    nxg::cache::check_kernel<<<grid, 256, 0, s>>>(a);
-    nxg::cache::check_finish_kernel<<<1, 1, 0, s>>>(a);
-    return nxg::record_cuda(cudaGetLastError());
+    if (const uint32_t st = nxg::launch_chained(true, nxg::cache::check_kernel, grid, 256u, 0u, s, a)) { return st; }
+    return nxg::launch_chained(true, nxg::cache::check_finish_kernel, 1u, 1u, 0u, s, a);
 }
 
 } // extern "C"

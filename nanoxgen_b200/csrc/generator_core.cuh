@@ -10,6 +10,7 @@
 // transported frame and the gradient noise, and writes the strand.
 #pragma once
 
+#include "launch.cuh"
 #include "nxg_internal.h"
 #include "nxg_classic.h"
 #include "strand_math.cuh"
@@ -39,14 +40,6 @@ struct LaunchArgs {
     uint32_t classic_length; // scale each strand about its first point by scalars.x
     uint32_t classic_width;  // radius = 0.5 * max(scalars.y, 0) * radius_scale
 };
-
-// Kernels of one call are chained as programmatic dependent launches: each
-// lets the next one's CTAs be set up while it runs (chain_start) and touches
-// memory only once the one before has completed and its writes are visible
-// (chain_wait; a no-op in a kernel launched without the attribute).  That
-// takes the launch gaps out of a chain of short kernels.
-__device__ __forceinline__ void chain_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 constexpr int kTableFloat4 = NXG_NOISE_GRADIENT_COUNT;  // float4 entries of the staged table
 
@@ -630,7 +623,6 @@ __device__ __forceinline__ float4 guide_offset_entry(const AssetArgs &a, const F
 dev::AssetArgs resolve_asset(const nxg_device_asset_desc &desc);
 dev::FrameArgs resolve_frame(const dev::AssetArgs &a, const nxg_deformed_desc &d);
 dev::ParamArgs resolve_params(const nxg_generation_params &p, float radius_scale);
-uint32_t record_cuda(cudaError_t e);
 int device_sm_count();
 uint32_t validate_range_request(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
                                 const nxg_generation_params *params, const nxg_packed_output_desc *output,
@@ -647,23 +639,5 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
                          uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
                          const nxg_classic_apply_desc *classic, bool prepared, uint32_t samples = 1u);
-
-// Launches `fn`; `chained`: as a programmatic dependent of the launch before it
-// on the stream (fn then calls chain_wait before it touches memory).
-template <class... Params, class... Args>
-uint32_t launch_chained(bool chained, void (*fn)(Params...), uint32_t grid, uint32_t block, size_t shm,
-                        cudaStream_t stream, const Args &...args) {
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(grid);
-    config.blockDim = dim3(block);
-    config.dynamicSmemBytes = shm;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attribute;
-    config.numAttrs = chained ? 1u : 0u;
-    return record_cuda(cudaLaunchKernelEx(&config, fn, args...));
-}
 
 } // namespace nxg
