@@ -716,9 +716,9 @@ __device__ __forceinline__ f32x2 walk_lattice_pair(const float2 *lat, uint32_t b
 // the end starts the next one inside it, so the first two
 // columns are moved there from the old window and only the others are
 // computed (551 -> 533 us on 1,000,000 strands x 32).  Out of line: it is called about twice per strand, and its
-// registers inlined spill the walk's loop.  Every lane of the warp calls it.
+// registers inlined spill the walk's loop.  Every one of `lanes` calls it.
 static __device__ __noinline__ uint4 walk_fill_window(F3 dom, float distance, WalkWindow old, float2 *lat,
-                                                      const float4 *table, uint32_t copies) {
+                                                      const float4 *table, uint32_t copies, unsigned lanes) {
     __builtin_assume(__isShared(lat));
     __builtin_assume(__isShared(table));
     uint32_t bias[3], moved[3];
@@ -733,7 +733,7 @@ static __device__ __noinline__ uint4 walk_fill_window(F3 dom, float distance, Wa
         near = near && moved[ax] <= static_cast<uint32_t>(kWalkWindow) - 2u;
     }
     int first = 0;
-    if (__all_sync(kFull, near)) {
+    if (__all_sync(lanes, near)) {
         first = 2;
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
@@ -900,7 +900,7 @@ __device__ __forceinline__ void walk_pair(WalkCursor &s, F3 n0, F3 n1, f32x2 t, 
     const float da = __fmul_rn(s.arc, f_eff), db = __fmul_rn(arc_b, f_eff);
     bool lattice = true;
     if (__any_sync(kFull, counts && !(db <= wl.limit))) {
-        const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies);
+        const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies, kFull);
         wl = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
         lattice = __all_sync(kFull, db <= wl.limit || !counts);
     }
