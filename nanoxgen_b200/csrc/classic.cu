@@ -42,7 +42,13 @@ struct ScalarArgs {
     DeviceExpression width;
 };
 
-__global__ void __launch_bounds__(256) classic_scalars_kernel(const __grid_constant__ ScalarArgs k) {
+// What bounds it: the gathers of a random triangle's vertices (137 of 270 us
+// for 4,000,000 roots of 200,000 triangles; a lookup per lane and load, hence
+// gather3) and their latency, hence 64 warps per SM; then the interpreter
+// (92) and the noise corners (61).  308 us with three loads per vertex and 48
+// warps, 268 now.  Two or four roots per thread and decoded instruction cost
+// more warps than they save instructions (298, 342 us).
+__global__ void __launch_bounds__(256, 8) classic_scalars_kernel(const __grid_constant__ ScalarArgs k) {
     __shared__ float4 table[256];
     __shared__ uint8_t perm[256];
     stage_classic_tables(table, perm);

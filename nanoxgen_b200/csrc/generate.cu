@@ -99,13 +99,14 @@ __global__ void generate_kernel(LaunchArgs g, const float4 *offsets) {
 
 // The lane-walk generator (walk.cuh).  Persistent CTAs over contiguous ranges
 // of the strand order; each warp takes g.batch strands at a time.  Register
-// budgets: the noise variant runs one CTA of up to sixteen warps per SM (at
-// most 128 registers); the plain one three CTAs of eight warps (at most 80
-// registers), the plain Classic one two.  The arguments stay in the constant
+// budgets: the noise variant runs one CTA of up to twelve warps per SM (at
+// most 168 registers), the plain one three CTAs of eight warps (at most 80
+// registers; with Classic scalars on 4,000,000 strands x 24, 902 us, two CTAs
+// 1,037, four 1,135).  The arguments stay in the constant
 // bank (__grid_constant__): an out-of-line call taking them by reference
 // otherwise copies them to every thread's stack first.
 template <bool NOISE, bool CLASSIC>
-__global__ void __launch_bounds__(NOISE ? 32 * kWalkNoiseWarps : 256, NOISE ? 1 : (CLASSIC ? 2 : 3))
+__global__ void __launch_bounds__(NOISE ? 32 * kWalkNoiseWarps : 256, NOISE ? 1 : 3)
     generate_walk_kernel(const __grid_constant__ LaunchArgs g, const float4 *offsets) {
     extern __shared__ float4 smem[];
     const uint32_t P = g.p.cvs_per_strand;
@@ -965,8 +966,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
             // (20,000 strands x 160 CVs with noise 159 -> 113 us, x 100 CVs
             // without 72 -> 31 us), and the last batches of a larger one are
             // not nearly empty.  Below a warp per SM the CTAs shrink too.
-            const uint64_t slots = static_cast<uint64_t>(sms) * (noise ? dev::kWalkNoiseWarps
-                                                                       : (classic_scalars ? 16u : 24u));
+            const uint64_t slots = static_cast<uint64_t>(sms) * (noise ? dev::kWalkNoiseWarps : 24u);
             const uint64_t rounds = (count + slots * 32u - 1u) / (slots * 32u);
             const uint64_t share = (count + slots * rounds - 1u) / (slots * rounds);
             g.batch = static_cast<uint32_t>(std::clamp<uint64_t>((share + 3u) / 4u * 4u, noise ? 8u : 4u, 32u));

@@ -121,6 +121,24 @@ __device__ __forceinline__ F3 ld3(const float *p, uint32_t i) {
     return {__ldg(q), __ldg(q + 1), __ldg(q + 2)};
 }
 
+// Row i of an n x 3 array where each lane reads its own: the aligned two words
+// and the third.  Such a load costs the cache a lookup per lane whatever its
+// width, so two loads instead of three.
+__device__ __forceinline__ F3 gather3(const float *p, uint32_t i) {
+    const float *q = p + 3u * static_cast<uint64_t>(i);
+    const uint32_t odd = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(q) >> 2) & 1u;
+    const float2 two = __ldg(reinterpret_cast<const float2 *>(q + odd));
+    const float one = __ldg(odd ? q : q + 2);
+    return odd ? F3{one, two.x, two.y} : F3{two.x, two.y, one};
+}
+
+// ... of an n x 2 array, which may start at any word.
+__device__ __forceinline__ float2 gather2(const float *p, uint32_t i) {
+    const float *q = p + 2u * static_cast<uint64_t>(i);
+    if ((reinterpret_cast<uintptr_t>(p) & 4u) == 0u) { return __ldg(reinterpret_cast<const float2 *>(q)); }
+    return make_float2(__ldg(q), __ldg(q + 1));
+}
+
 // ---------------------------------------------------------------------------
 // Kernel arguments: device pointers resolved on the host from the validated
 // header mirror, so kernels never read counts or offsets from device memory.
@@ -170,9 +188,10 @@ __device__ __forceinline__ float random01(uint32_t seed, uint32_t strand, uint32
 }
 
 __device__ __forceinline__ uint3 load_triangle(const AssetArgs &a, uint32_t t) {
-    const uint32_t *p = a.triangles + 3u * static_cast<uint64_t>(t);
+    const F3 p = gather3(reinterpret_cast<const float *>(a.triangles), t);
     const uint32_t vmax = a.vertex_count - 1u;
-    return make_uint3(min(__ldg(p), vmax), min(__ldg(p + 1), vmax), min(__ldg(p + 2), vmax));
+    return make_uint3(min(__float_as_uint(p.x), vmax), min(__float_as_uint(p.y), vmax),
+                      min(__float_as_uint(p.z), vmax));
 }
 
 // Alias draw of generate.h:107-112 (the triangle decision alone).
@@ -204,10 +223,10 @@ __device__ __forceinline__ Root sample_root(const AssetArgs &a, const FrameArgs 
     r.b1 = __fmul_rn(s, __fsub_rn(1.0f, r2));
     r.b2 = __fmul_rn(s, r2);
     const uint3 t = load_triangle(a, r.triangle);
-    const F3 p0 = ld3(f.positions, t.x), p1 = ld3(f.positions, t.y), p2 = ld3(f.positions, t.z);
+    const F3 p0 = gather3(f.positions, t.x), p1 = gather3(f.positions, t.y), p2 = gather3(f.positions, t.z);
     r.position = xbary(p0, p1, p2, b0, r.b1, r.b2);
     if (a.flags & NXG_ASSET_HAS_NORMALS) {  // the face normal is replaced by the vertex normals' blend
-        r.normal = xnormalize(xbary(ld3(f.normals, t.x), ld3(f.normals, t.y), ld3(f.normals, t.z),
+        r.normal = xnormalize(xbary(gather3(f.normals, t.x), gather3(f.normals, t.y), gather3(f.normals, t.z),
                                     b0, r.b1, r.b2));
     } else {
         r.normal = xnormalize(xcross(xsub(p1, p0), xsub(p2, p0)));
@@ -215,13 +234,9 @@ __device__ __forceinline__ Root sample_root(const AssetArgs &a, const FrameArgs 
     r.u = 0.0f;
     r.v = 0.0f;
     if ((a.flags & NXG_ASSET_HAS_TEXCOORDS) && a.texcoords) {
-        const float *t0 = a.texcoords + 2u * static_cast<uint64_t>(t.x);
-        const float *t1 = a.texcoords + 2u * static_cast<uint64_t>(t.y);
-        const float *t2 = a.texcoords + 2u * static_cast<uint64_t>(t.z);
-        r.u = __fadd_rn(__fadd_rn(__fmul_rn(__ldg(t0), b0), __fmul_rn(__ldg(t1), r.b1)),
-                        __fmul_rn(__ldg(t2), r.b2));
-        r.v = __fadd_rn(__fadd_rn(__fmul_rn(__ldg(t0 + 1), b0), __fmul_rn(__ldg(t1 + 1), r.b1)),
-                        __fmul_rn(__ldg(t2 + 1), r.b2));
+        const float2 t0 = gather2(a.texcoords, t.x), t1 = gather2(a.texcoords, t.y), t2 = gather2(a.texcoords, t.z);
+        r.u = __fadd_rn(__fadd_rn(__fmul_rn(t0.x, b0), __fmul_rn(t1.x, r.b1)), __fmul_rn(t2.x, r.b2));
+        r.v = __fadd_rn(__fadd_rn(__fmul_rn(t0.y, b0), __fmul_rn(t1.y, r.b1)), __fmul_rn(t2.y, r.b2));
     }
     return r;
 }

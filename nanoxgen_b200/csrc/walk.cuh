@@ -99,7 +99,8 @@ constexpr uint32_t kWalkMaxCvs = 1024u;
 //   q = 4     (root position, 1 / weight sum)
 //   q = 5     (root normal in normal mode else 0, slot count as bits)
 //   q = 6, 7  Classic scalars without noise (walk_classic_setup): (first
-//             point, length scale) and (width radius, width override flag)
+//             point, length scale) and (width radius, width override flag,
+//             width below the drop threshold, chord near it)
 // Nearest mode becomes one slot of weight 1 and normal mode zero slots, so
 // the base step evaluates every strand as
 //   base = root + (inv * sum_j w_j offsets[row_j + c] + normal' * t_c) * length_scale.
@@ -131,6 +132,10 @@ struct WalkRoot {
 template <bool NOISE>
 __device__ __forceinline__ Root walk_root(const AssetArgs &a, const FrameArgs &f, uint32_t seed, uint32_t strand,
                                           F3 &surface_u, F3 &rest_position) {
+    // The noise walk's instructions, not its lookups, bound it (gather3 there:
+    // 706 -> 713 us on 5 samples of 250,000 strands; without noise 1,032 ->
+    // 1,021 us on 4,000,000 x 24).
+    const auto row = [](const float *p, uint32_t i) { return NOISE ? ld3(p, i) : gather3(p, i); };
     Root r;
     r.triangle = sample_triangle(a, seed, strand);
     const float r1 = random01(seed, strand, 2u);
@@ -140,20 +145,20 @@ __device__ __forceinline__ Root walk_root(const AssetArgs &a, const FrameArgs &f
     r.b1 = __fmul_rn(s, __fsub_rn(1.0f, r2));
     r.b2 = __fmul_rn(s, r2);
     const uint3 t = load_triangle(a, r.triangle);
-    const F3 p0 = ld3(f.positions, t.x), p1 = ld3(f.positions, t.y), p2 = ld3(f.positions, t.z);
+    const F3 p0 = row(f.positions, t.x), p1 = row(f.positions, t.y), p2 = row(f.positions, t.z);
     // A deformed frame's noise domain needs the rest-pose vertices too:
     // requested with the frame's, before any arithmetic waits on them.
     F3 q0 = p0, q1 = p1, q2 = p2;
     if (NOISE && f.positions != a.positions) {
-        q0 = ld3(a.positions, t.x);
-        q1 = ld3(a.positions, t.y);
-        q2 = ld3(a.positions, t.z);
+        q0 = row(a.positions, t.x);
+        q1 = row(a.positions, t.y);
+        q2 = row(a.positions, t.z);
     }
     r.position = xbary(p0, p1, p2, b0, r.b1, r.b2);
     // The face normal only where the asset has no vertex normals (the
     // reference computes it first and then replaces it).
     if (a.flags & NXG_ASSET_HAS_NORMALS) {
-        r.normal = xnormalize(xbary(ld3(f.normals, t.x), ld3(f.normals, t.y), ld3(f.normals, t.z),
+        r.normal = xnormalize(xbary(row(f.normals, t.x), row(f.normals, t.y), row(f.normals, t.z),
                                     b0, r.b1, r.b2));
     } else {
         r.normal = xnormalize(xcross(xsub(p1, p0), xsub(p2, p0)));
@@ -163,12 +168,9 @@ __device__ __forceinline__ Root walk_root(const AssetArgs &a, const FrameArgs &f
     const bool uvs = (a.flags & NXG_ASSET_HAS_TEXCOORDS) && a.texcoords;
     float2 uv0 = make_float2(0.0f, 0.0f), uv1 = uv0, uv2 = uv0;
     if (uvs) {
-        uv0 = make_float2(__ldg(a.texcoords + 2u * static_cast<uint64_t>(t.x)),
-                          __ldg(a.texcoords + 2u * static_cast<uint64_t>(t.x) + 1u));
-        uv1 = make_float2(__ldg(a.texcoords + 2u * static_cast<uint64_t>(t.y)),
-                          __ldg(a.texcoords + 2u * static_cast<uint64_t>(t.y) + 1u));
-        uv2 = make_float2(__ldg(a.texcoords + 2u * static_cast<uint64_t>(t.z)),
-                          __ldg(a.texcoords + 2u * static_cast<uint64_t>(t.z) + 1u));
+        uv0 = gather2(a.texcoords, t.x);
+        uv1 = gather2(a.texcoords, t.y);
+        uv2 = gather2(a.texcoords, t.z);
         r.u = __fadd_rn(__fadd_rn(__fmul_rn(uv0.x, b0), __fmul_rn(uv1.x, r.b1)), __fmul_rn(uv2.x, r.b2));
         r.v = __fadd_rn(__fadd_rn(__fmul_rn(uv0.y, b0), __fmul_rn(uv1.y, r.b1)), __fmul_rn(uv2.y, r.b2));
     }
@@ -468,30 +470,45 @@ __device__ __forceinline__ F3 walk_base_point(const float4 *records, int s, int 
 }
 
 // Classic scalars without noise (xgen_classic_runtime.cpp:1650-1678,
-// :1827-1858), for this lane's strand before its base step: the first and
-// last base points give the chord; a strand whose scaled chord is near the
-// 1e-4 threshold measures its sampled spline; a dropped strand gets point
-// count 0.  Leaves records 6 and 7 for walk_base_direct.
-__device__ __forceinline__ void walk_classic_setup(const LaunchArgs &g, float4 *records, int lane, bool valid,
-                                                   uint32_t local, const float *tvals, const float4 *offsets, int P) {
+// :1827-1858), for this lane's strand before its base step: the first base
+// point (the root itself, unless a guide's first offset is not zero), the
+// scale and the radius, left in records 6 and 7 for walk_base_direct.
+__device__ __forceinline__ void walk_classic_setup(const LaunchArgs &g, float4 *records, int lane, const WalkRoot &root,
+                                                   uint32_t local, const float *tvals, const float4 *offsets) {
     const ParamArgs &p = g.p;
-    const float ls = p.length_scale;
     const float2 sc = __ldg(g.scalars + local);
-    const F3 front = walk_base_point(records, lane, 0, tvals[0], ls, offsets);
-    const F3 back = walk_base_point(records, lane, P - 1, tvals[P - 1], ls, offsets);
+    F3 front = root.position;
+    if (root.lead) { front = walk_base_point(records, lane, 0, tvals[0], p.length_scale, offsets); }
     const float scale = g.classic_length ? sc.x : 1.0f;
     const float raw_width = g.classic_width ? sc.y
         : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
-    bool keep = !(raw_width < 1.0e-4f);
-    const F3 chord = back - front;
-    if (keep && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f)) {
-        keep = !(__fmul_rn(classic_spline_length_by(
-                               [&](int c) { return walk_base_point(records, lane, c, tvals[c], ls, offsets); }, P),
-                           scale) < 1.0e-4f);
-    }
     const float radius = __fmul_rn(__fmul_rn(0.5f, raw_width < 0.0f ? 0.0f : raw_width), p.radius_scale);
     records[6 * 32 + lane] = make_float4(front.x, front.y, front.z, scale);
-    records[7 * 32 + lane] = make_float4(radius, g.classic_width ? 1.0f : 0.0f, 0.0f, 0.0f);
+    records[7 * 32 + lane] = make_float4(radius, g.classic_width ? 1.0f : 0.0f, raw_width < 1.0e-4f ? 1.0f : 0.0f, 0.0f);
+}
+
+// The sampled spline's length of this lane's strand.  Out of line: it is rare,
+// and inlined its registers leave room for two CTAs per SM instead of three
+// (1,022 us on 4,000,000 strands x 24; 935 with three).
+static __device__ __noinline__ float walk_spline_length(const float4 *records, int lane, const float *tvals, float ls,
+                                                        const float4 *offsets, int P) {
+    return classic_spline_length_by(
+        [&](int c) { return walk_base_point(records, lane, c, tvals[c], ls, offsets); }, P);
+}
+
+// The drop rule after the base step: a strand of too small a width, or one
+// whose scaled chord walk_base_direct found near the 1e-4 threshold and whose
+// sampled spline is below it, gets point count 0.  (The chord taken in the
+// base step instead of from two points gathered before it: 935 -> 902 us on
+// 4,000,000 strands x 24.)
+__device__ __forceinline__ void walk_classic_drop(const LaunchArgs &g, const float4 *records, int lane, bool valid,
+                                                  uint32_t local, const float *tvals, const float4 *offsets, int P) {
+    const float4 width = records[7 * 32 + lane];
+    bool keep = width.z == 0.0f;
+    if (keep && width.w != 0.0f) {
+        keep = !(__fmul_rn(walk_spline_length(records, lane, tvals, g.p.length_scale, offsets, P),
+                           records[6 * 32 + lane].w) < 1.0e-4f);
+    }
     if (!keep && valid && g.point_counts != nullptr) { g.point_counts[local] = 0u; }
 }
 
@@ -509,9 +526,10 @@ __device__ __forceinline__ ulonglong2 walk_offset(const float4 *offsets, uint32_
 // pass runs as many slot pairs as its strands' largest count; a strand's
 // loads past its own count are predicated off (no memory request), and its
 // weights there are zero.
-// CLASSIC applies records 6 and 7.  Every lane of the warp calls it.
+// CLASSIC applies records 6 and 7, and marks a strand whose scaled chord is
+// near the drop threshold in record 7.  Every lane of the warp calls it.
 template <bool CLASSIC>
-__device__ __forceinline__ void walk_base_direct(const LaunchArgs &g, const float4 *records, const uint32_t *locals,
+__device__ __forceinline__ void walk_base_direct(const LaunchArgs &g, float4 *records, const uint32_t *locals,
                                                  const float *tvals, const float *rvals, const float4 *offsets,
                                                  int lane, int in_batch, int P) {
     constexpr int kPerLane = 4;
@@ -569,6 +587,10 @@ __device__ __forceinline__ void walk_base_direct(const LaunchArgs &g, const floa
                     F3 base = F3{head.x, head.y, head.z} + (acc[m] * head.w + F3{tail.x, tail.y, tail.z} * tv[m]) * ls;
                     float radius = rvals[cm];
                     if constexpr (CLASSIC) {
+                        const F3 chord = base - xyz(front);
+                        if (cm == P - 1 && !(sqrtf(dot(chord, chord)) * front.w > 1.01e-4f)) {
+                            records[7 * 32 + s].w = 1.0f;
+                        }
                         if (g.classic_length) { base = xadd(xyz(front), xmul(xsub(base, xyz(front)), front.w)); }
                         if (width.y != 0.0f) { radius = width.x; }
                     }
@@ -1187,15 +1209,19 @@ __device__ __forceinline__ void walk_plain_batch(const LaunchArgs &g, const floa
     uint32_t *locals = reinterpret_cast<uint32_t *>(mine + (CLASSIC ? kWalkClassicRecordBytes : kWalkRecordBytes));
     const int P = static_cast<int>(g.p.cvs_per_strand);
     const bool counts = lane < in_batch;
-    walk_setup<false>(g, records, locals, lane, batch + (counts ? static_cast<uint32_t>(lane) : 0u), counts,
-                      static_cast<uint32_t>(P));
-    __syncwarp();
+    const WalkRoot root = walk_setup<false>(g, records, locals, lane,
+                                            batch + (counts ? static_cast<uint32_t>(lane) : 0u), counts,
+                                            static_cast<uint32_t>(P));
     if constexpr (CLASSIC) {
-        walk_classic_setup(g, records, lane, counts, locals[lane] & 0x7fffffffu, tvals, offsets, P);
-        __syncwarp();
+        walk_classic_setup(g, records, lane, root, locals[lane] & 0x7fffffffu, tvals, offsets);
     }
+    __syncwarp();
     walk_base_direct<CLASSIC>(g, records, locals, tvals, rvals, offsets, lane, in_batch, P);
     __syncwarp();
+    if constexpr (CLASSIC) {
+        walk_classic_drop(g, records, lane, counts, locals[lane] & 0x7fffffffu, tvals, offsets, P);
+        __syncwarp();
+    }
 }
 
 } // namespace dev
