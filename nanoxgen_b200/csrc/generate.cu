@@ -719,8 +719,9 @@ bool valid_tile(uint32_t P, uint32_t lanes, uint32_t ppt) {
 }
 
 // Tile shape for P CVs: the registered one, else the lane-walk generator for
-// 2..32 CVs (lanes_per_strand 1; CTAs of 512 threads with noise, 256
-// without), else four CVs per lane on the narrowest power-of-two group that
+// 2..32 CVs (lanes_per_strand 1; CTAs of 352 threads with noise, 256
+// without: with noise the size callers have been told, of which the launch of
+// the built-in tile is free, it takes up to kWalkNoiseWarps), else four CVs per lane on the narrowest power-of-two group that
 // holds the strand (what the autotuner starts from: unregistered, longer
 // strands take the lane walk as well).
 uint32_t registered_tile(uint32_t P, bool noise) {
@@ -737,7 +738,7 @@ void default_tile(uint32_t P, bool noise, int *lanes, int *ppt, uint32_t *block)
     if (P >= 2u && P <= kMaxLaneWalkTile) {  // the lane-walk generator
         *lanes = 1;
         *ppt = 1;
-        *block = noise ? 32u * dev::kWalkNoiseWarps : 256u;
+        *block = noise ? 352u : 256u;
         return;
     }
     *ppt = 4;
