@@ -542,7 +542,7 @@ def run_batched(args):
                        "l2": "flushed between timed replays (256 MiB write)"},
             "plain_path": {"ms_per_step": pms, "value": points / (pms / 1e3),
                            "how": "one nxg_generate_packed per description, all in one CUDA graph"},
-            "batched_speedup_vs_plain": pms / ms, "clocks": clocks, "gpu_launches": 7 * args.steps}
+            "batched_speedup_vs_plain": pms / ms, "clocks": clocks, "gpu_launches": 6 * args.steps}
     print(json.dumps(line), flush=True)
 
 
@@ -587,7 +587,7 @@ def run_motion(args):
             "config": {"workload": w.name + "/5-motion-samples", "samples": 5, "strands": S, "cvs_per_strand": P,
                        "tile": tile, "l2": "flushed between timed replays (256 MiB write)"},
             "hbm_gbs": alg / (ms / 1e3) / 1e9, "hbm_frac": alg / (ms / 1e3) / 1e9 / peak, "peak_source": kind,
-            "clocks": clocks, "gpu_launches": (4 + 3 * 5) * args.steps}
+            "clocks": clocks, "gpu_launches": (3 + 2 * 5) * args.steps}
     print(json.dumps(line), flush=True)
 
 
@@ -1146,7 +1146,7 @@ def run_payload(args):
             "config": {"workload": "payload/displaced-sphere-200k-tris/%d-strands-x%d/1-motion-sample" % (S, P),
                        "batches": int(result.batch_first_point.numel() - 1), "max_strands_per_batch": 65536,
                        "transform": transform, "l2": "inputs and outputs larger than L2; flushed between steps"},
-            "roofline": {"bound": "hbm", "kernel": "batches_kernel", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "flat_points_kernel", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind, "traffic": None,
                          "algorithmic_bytes": algorithmic},
             "clocks": clocks, "gpu_launches": args.steps}
@@ -1245,7 +1245,7 @@ def run_asset_build(args):
             "e2e": {"value": em, "unit": "ms per nxg_build_asset_device call",
                     "h2d_bytes_per_step": int(positions.numel() * 4 + triangles.numel() * 4 + 2 * roots.numel() * 4),
                     "d2h_bytes_per_step": int(out.numel() * 4), "blob_equal_host_build": same_blob},
-            "cpu_baseline": cpu, "host_port_build": port, "clocks": clocks, "gpu_launches": args.steps}
+            "cpu_baseline": cpu, "host_port_build": port, "clocks": clocks, "gpu_launches": 3 * args.steps}
     print(json.dumps(line), flush=True)
 
 

@@ -35,7 +35,7 @@
 // Twelve warps at 168 registers; sixteen at 128 spilled (729 us).  1,000,000 x
 // 32: 601 us staged whole with all columns, 526 us now; 150,001 x 61: 419 us
 // on lane groups with scans, 228 us; 20,011 x 160: 1,241 us on one thread per
-// strand, 121 us.
+// strand, 97 us (121 before the equal batches of small calls).
 //
 // Stage rows are 49 words apart and a CV takes 3 words; both strides are odd,
 // so a warp reading column c of 32 rows (frame step) and a warp reading one
@@ -1027,29 +1027,43 @@ __device__ __forceinline__ void walk_store_chunk(const LaunchArgs &g, const floa
     }
 }
 
+__device__ __forceinline__ F3 walk_scaled(F3 centre, F3 q, float k) { return centre + (q - centre) * k; }
+
 // Rewrites the written points of the warp's strands: each lane holds its own
-// strand's centre and scale (about `centre`, points to centre + (q - centre)
-// * scale) and radius override (negative: none); lanes over one strand's CVs,
-// so a strand's run is read and written as consecutive float4s.  EXACT: in
-// the uncontracted operations of the Classic application.  The points are
-// this warp's own writes of a moment ago (in L2).  Every lane of the warp
-// calls it, after a __syncwarp.
-template <bool EXACT>
-__device__ __forceinline__ void walk_rescale(const LaunchArgs &g, const uint32_t *locals, F3 centre, float scale,
-                                             float radius, int lane, int in_batch, int P) {
-    for (int s = 0; s < in_batch; ++s) {
-        const uint32_t word = locals[s];
+// strand's preserveLength scale (points to centre + (q - centre) * keep) and,
+// CLASSIC, the Classic one (about `front`, in its uncontracted operations) and
+// radius override (negative: none).  The points are this warp's own writes of
+// a moment ago, so what bounds it is the latency of L2: eight lanes per strand
+// and four strands at a time as in the store step, a lane's loads requested
+// together, both scales in one pass.  500,000 strands x 24 with noise, one
+// strand at a time and now: Classic scalars 424 -> 356 us, preserveLength 398
+// -> 340, both 524 -> 361.  (Longer runs in flight, or out of line, the walk's
+// own registers spill.)  Every lane of the warp calls it, after a __syncwarp.
+template <bool CLASSIC>
+__device__ __forceinline__ void walk_rescale(const LaunchArgs &g, const uint32_t *locals, F3 centre, float keep,
+                                             F3 front, float scale, float radius, int lane, int in_batch, int P) {
+    const bool length = CLASSIC && g.classic_length != 0u;
+    constexpr int kPerLane = 4;
+#pragma unroll 1
+    for (int first = 0; first < in_batch; first += 4) {
+        const int s = first + (lane >> 3);  // at most 31
+        const uint32_t word = s < in_batch ? locals[s] : 0x80000000u;
         const F3 o = {__shfl_sync(kFull, centre.x, s), __shfl_sync(kFull, centre.y, s),
                       __shfl_sync(kFull, centre.z, s)};
-        const float k = __shfl_sync(kFull, scale, s);
-        const float r = __shfl_sync(kFull, radius, s);
-        const bool move = EXACT ? g.classic_length != 0u : k != 1.0f;
-        if ((word >> 31) || (!move && r < 0.0f)) { continue; }
+        const float k = __shfl_sync(kFull, keep, s);
+        F3 f = {0.0f, 0.0f, 0.0f};
+        float by = 1.0f, r = -1.0f;
+        if constexpr (CLASSIC) {
+            f = F3{__shfl_sync(kFull, front.x, s), __shfl_sync(kFull, front.y, s), __shfl_sync(kFull, front.z, s)};
+            by = __shfl_sync(kFull, scale, s);
+            r = __shfl_sync(kFull, radius, s);
+        }
+        if ((word >> 31) || (k == 1.0f && !length && r < 0.0f)) { continue; }
         const uint64_t begin = static_cast<uint64_t>(word) * static_cast<uint32_t>(P);
         if (g.vec3_points) {
-            for (int c = lane; c < P; c += 32) {
+            for (int c = lane & 7; c < P; c += 8) {
                 float *q = g.vec3_points + 3u * (begin + static_cast<uint32_t>(c));
-                const F3 v = o + (F3{q[0], q[1], q[2]} - o) * k;
+                const F3 v = walk_scaled(o, F3{q[0], q[1], q[2]}, k);
                 q[0] = v.x;
                 q[1] = v.y;
                 q[2] = v.z;
@@ -1057,23 +1071,30 @@ __device__ __forceinline__ void walk_rescale(const LaunchArgs &g, const uint32_t
             continue;
         }
         float4 *points = g.points + begin;
-#pragma unroll 4
-        for (int c = lane; c < P; c += 32) {
-            const float4 q = points[c];
-            F3 v = xyz(q);
-            if (move) { v = EXACT ? xadd(o, xmul(xsub(v, o), k)) : o + (v - o) * k; }
-            points[c] = make_float4(v.x, v.y, v.z, r < 0.0f ? q.w : r);
+#pragma unroll 1
+        for (int c = lane & 7; c < P; c += 8 * kPerLane) {
+            float4 q[kPerLane];
+#pragma unroll
+            for (int m = 0; m < kPerLane; ++m) { q[m] = points[min(c + 8 * m, P - 1)]; }
+#pragma unroll
+            for (int m = 0; m < kPerLane; ++m) {
+                F3 v = xyz(q[m]);
+                if (k != 1.0f) { v = walk_scaled(o, v, k); }
+                if (length) { v = xadd(f, xmul(xsub(v, f), by)); }
+                if (c + 8 * m < P) { points[c + 8 * m] = make_float4(v.x, v.y, v.z, r < 0.0f ? q[m].w : r); }
+            }
         }
     }
 }
 
 // The Classic application to noisy strands once their points are written
 // (the rules of emit_strand: scale about the first point, width override, the
-// drop rule with its chord bound and sampled-spline measure); a dropped
-// strand's point count becomes 0.  Every lane of the warp calls it, after a
+// drop rule with its chord bound and sampled-spline measure), after their
+// preserveLength scale `kept` about `centre`; a dropped strand's point count
+// becomes 0.  Every lane of the warp calls it, after a
 // __syncwarp.
-__device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const uint32_t *locals, int lane,
-                                                    int in_batch, int P) {
+__device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const uint32_t *locals, F3 centre,
+                                                    float kept, int lane, int in_batch, int P) {
     const ParamArgs &p = g.p;
     const uint32_t word = lane < in_batch ? locals[lane] : 0x80000000u;
     F3 front = {0.0f, 0.0f, 0.0f};
@@ -1081,15 +1102,19 @@ __device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const u
     if (!(word >> 31)) {
         const float4 *points = g.points + static_cast<uint64_t>(word) * static_cast<uint32_t>(P);
         const float2 sc = __ldg(g.scalars + word);
-        front = xyz(points[0]);
-        const F3 back = xyz(points[P - 1]);
+        const auto point = [=](int i) {
+            const F3 q = xyz(points[i]);
+            return kept != 1.0f ? walk_scaled(centre, q, kept) : q;
+        };
+        front = point(0);
+        const F3 back = point(P - 1);
         scale = g.classic_length ? sc.x : 1.0f;
         const float raw_width = g.classic_width ? sc.y
             : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
         bool keep = !(raw_width < 1.0e-4f);
         const F3 chord = back - front;
         if (keep && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f)) {
-            keep = !(__fmul_rn(classic_spline_length_by([points](int i) { return xyz(points[i]); }, P), scale) <
+            keep = !(__fmul_rn(classic_spline_length_by(point, P), scale) <
                      1.0e-4f);
         }
         if (g.classic_width) {
@@ -1098,7 +1123,7 @@ __device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const u
         if (!keep && g.point_counts != nullptr) { g.point_counts[word] = 0u; }
     }
     __syncwarp();
-    walk_rescale<true>(g, locals, front, scale, radius, lane, in_batch, P);
+    walk_rescale<true>(g, locals, centre, kept, front, scale, radius, lane, in_batch, P);
 }
 
 // One batch of a warp with noise: strands [batch, batch + in_batch) of the
@@ -1188,14 +1213,12 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
         walk_store_chunk(g, stage, locals, rvals, lane, in_batch, a, n, P, again);
         __syncwarp();
     }
-    if (preserve && !one_chunk) {
-        const float scale = counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
-        if (__any_sync(kFull, scale != 1.0f)) {
-            walk_rescale<false>(g, locals, wr.position, scale, -1.0f, lane, in_batch, P);
-            __syncwarp();
-        }
+    const float kept = preserve && !one_chunk && counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
+    if constexpr (CLASSIC) {
+        walk_classic_finish(g, locals, wr.position, kept, lane, in_batch, P);
+    } else if (__any_sync(kFull, kept != 1.0f)) {
+        walk_rescale<false>(g, locals, wr.position, kept, wr.position, 1.0f, -1.0f, lane, in_batch, P);
     }
-    if constexpr (CLASSIC) { walk_classic_finish(g, locals, lane, in_batch, P); }
     __syncwarp();
 }
 
