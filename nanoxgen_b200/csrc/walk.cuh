@@ -505,7 +505,7 @@ __device__ __forceinline__ void walk_classic_drop(const LaunchArgs &g, const flo
                                                   uint32_t local, const float *tvals, const float4 *offsets, int P) {
     const float4 width = records[7 * 32 + lane];
     bool keep = width.z == 0.0f;
-    if (keep && width.w != 0.0f) {
+    if (valid && keep && width.w != 0.0f) {
         keep = !(__fmul_rn(walk_spline_length(records, lane, tvals, g.p.length_scale, offsets, P),
                            records[6 * 32 + lane].w) < 1.0e-4f);
     }
@@ -588,7 +588,7 @@ __device__ __forceinline__ void walk_base_direct(const LaunchArgs &g, float4 *re
                     float radius = rvals[cm];
                     if constexpr (CLASSIC) {
                         const F3 chord = base - xyz(front);
-                        if (cm == P - 1 && !(sqrtf(dot(chord, chord)) * front.w > 1.01e-4f)) {
+                        if (live && cm == P - 1 && !(sqrtf(dot(chord, chord)) * front.w > 1.01e-4f)) {
                             records[7 * 32 + s].w = 1.0f;
                         }
                         if (g.classic_length) { base = xadd(xyz(front), xmul(xsub(base, xyz(front)), front.w)); }
@@ -1090,11 +1090,12 @@ __device__ __forceinline__ void walk_rescale(const LaunchArgs &g, const uint32_t
 // The Classic application to noisy strands once their points are written
 // (the rules of emit_strand: scale about the first point, width override, the
 // drop rule with its chord bound and sampled-spline measure), after their
-// preserveLength scale `kept` about `centre`; a dropped strand's point count
-// becomes 0.  Every lane of the warp calls it, after a
+// preserveLength scale `kept` about the root `centre`, which is the first point
+// too unless `lead`; `back` is the tip as written.  A dropped strand's point
+// count becomes 0.  Every lane of the warp calls it, after a
 // __syncwarp.
 __device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const uint32_t *locals, F3 centre,
-                                                    float kept, int lane, int in_batch, int P) {
+                                                    float kept, bool lead, F3 back, int lane, int in_batch, int P) {
     const ParamArgs &p = g.p;
     const uint32_t word = lane < in_batch ? locals[lane] : 0x80000000u;
     F3 front = {0.0f, 0.0f, 0.0f};
@@ -1106,8 +1107,8 @@ __device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const u
             const F3 q = xyz(points[i]);
             return kept != 1.0f ? walk_scaled(centre, q, kept) : q;
         };
-        front = point(0);
-        const F3 back = point(P - 1);
+        front = lead ? point(0) : centre;  // its displacement is 0
+        if (kept != 1.0f) { back = walk_scaled(centre, back, kept); }
         scale = g.classic_length ? sc.x : 1.0f;
         const float raw_width = g.classic_width ? sc.y
             : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
@@ -1215,7 +1216,8 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
     }
     const float kept = preserve && !one_chunk && counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
     if constexpr (CLASSIC) {
-        walk_classic_finish(g, locals, wr.position, kept, lane, in_batch, P);
+        walk_classic_finish(g, locals, wr.position, kept, wr.lead, stage_get(row, (P - 1) % kWalkChunk), lane, in_batch,
+                            P);
     } else if (__any_sync(kFull, kept != 1.0f)) {
         walk_rescale<false>(g, locals, wr.position, kept, wr.position, 1.0f, -1.0f, lane, in_batch, P);
     }
