@@ -907,24 +907,41 @@ __device__ __forceinline__ void walk_pair(WalkCursor &s, F3 n0, F3 n1, f32x2 t, 
     const F3 vb = walk_turn(va, F3{high2(axis.x), high2(axis.y), high2(axis.z)}, cb, high2(omc),
                             sqrt_approx(fmaxf(-high2(d1), 0.0f)));
     // The update is linear in v and the reference renormalises after every
-    // step, a positive factor each time: so the transported normal is the
-    // direction of this unnormalised v, which is carried as it is (each step
-    // keeps at least 0.86 of its length, so 32 steps neither underflow nor
-    // overflow) and normalised here for the frame only.
+    // step, a positive factor each time; here both steps' directions come from
+    // one pair of roots, and the second goes on to the next pair.  (Carried
+    // unnormalised over a whole strand, v underflows: a turn by theta, axis of
+    // length sin theta, shortens it to sqrt(1 - c^2 + c^4) across the axis,
+    // 0.866 at 45 degrees, and to |c + (1 - c)(1 - c^2)| along it, c = cos
+    // theta, which vanishes near 139 degrees.)  No step lengthens v, so where
+    // the second leaves some of it the first did too; where nothing is left
+    // (`lost`), the second step is taken again with the reference's
+    // normalisation of each, (0, 1, 0) below 1e-20.
     const F3x2 v = {pair2(va.x, vb.x), pair2(va.y, vb.y), pair2(va.z, vb.z)};
     const f32x2 v2 = dot2(v, v);
-    const F3x2 vu = scale2(v, pair2(rsqrt_normal(low2(v2)), rsqrt_normal(high2(v2))));
-    const F3x2 mv = scale2(vu, minus);
-    const F3x2 bn = cross2(vu, mv, tn);
+    F3x2 vu = scale2(v, pair2(rsqrt_normal(low2(v2)), rsqrt_normal(high2(v2))));
+    F3x2 mv = scale2(vu, minus);
+    F3x2 bn = cross2(vu, mv, tn);
     // The frame's third vector cross(bn, vu) is tn - vu (vu . tn) for a unit
     // vu; its part along vu joins vu's coefficient below.
-    const f32x2 mvn = dot2(mv, tn);
+    f32x2 mvn = dot2(mv, tn);
     const float da = __fmul_rn(s.arc, f_eff), db = __fmul_rn(arc_b, f_eff);
+    const bool lost = !(high2(v2) > 1.0e-20f);
     bool lattice = true;
-    if (__any_sync(kFull, counts && !(db <= wl.limit))) {
-        const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies, kFull);
-        wl = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
-        lattice = __all_sync(kFull, db <= wl.limit || !counts);
+    if (__any_sync(kFull, counts && (lost || !(db <= wl.limit)))) {
+        if (lost) {
+            const F3 ua = normalize(va);
+            const F3 ub = normalize(walk_turn(ua, F3{high2(axis.x), high2(axis.y), high2(axis.z)}, cb, high2(omc),
+                                              sqrt_approx(fmaxf(-high2(d1), 0.0f))));
+            vu = F3x2{pair2(ua.x, ub.x), pair2(ua.y, ub.y), pair2(ua.z, ub.z)};
+            mv = scale2(vu, minus);
+            bn = cross2(vu, mv, tn);
+            mvn = dot2(mv, tn);
+        }
+        if (__any_sync(kFull, counts && !(db <= wl.limit))) {
+            const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies, kFull);
+            wl = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
+            lattice = __all_sync(kFull, db <= wl.limit || !counts);
+        }
     }
     f32x2 gx, gy, gz;
     if (lattice) {
@@ -948,7 +965,7 @@ __device__ __forceinline__ void walk_pair(WalkCursor &s, F3 n0, F3 n1, f32x2 t, 
     qa = s.cur + F3{low2(ox), low2(oy), low2(oz)};
     qb = n0 + F3{high2(ox), high2(oy), high2(oz)};
     s.tan = F3{high2(tn.x), high2(tn.y), high2(tn.z)};
-    s.v = vb;
+    s.v = F3{high2(vu.x), high2(vu.y), high2(vu.z)};
     s.cur = n1;
     s.arc = __fadd_rn(arc_b, sqrt_approx(lb));
 }
