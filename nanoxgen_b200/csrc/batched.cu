@@ -426,8 +426,9 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
     if (cudaGetDevice(&device) == cudaSuccess) {
         cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     }
-    // CTA size per class.
+    // CTA size and static shared memory per class.
     uint32_t class_block[kClasses] = {0u, 0u};
+    size_t class_static[kClasses] = {0u, 0u};
     for (uint32_t c = 0; c < kClasses; ++c) {
         cudaFuncAttributes attr{};
         if ((status = record_cuda(cudaFuncGetAttributes(&attr, kernel(c))))) { return status; }
@@ -439,6 +440,7 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
             block -= 32u;
         }
         class_block[c] = block;
+        class_static[c] = attr.sharedSizeBytes;
     }
 
     auto *w = static_cast<unsigned char *>(workspace);
@@ -525,10 +527,7 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
         const void *fn = kernel(c);
         const uint32_t block = class_block[c];
         const size_t shm = dev::batch_smem_bytes(static_cast<int>(c), any_classic, block / 32u);
-        if ((status = record_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(shm))))) {
-            return status;
-        }
+        if ((status = allow_shared(fn, class_static[c], smem_optin))) { return status; }
         int per_sm = 0;
         if ((status = record_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(block),
                                                                                 shm)))) {

@@ -824,13 +824,6 @@ uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_
     const uint32_t scatter_blocks = static_cast<uint32_t>(std::max(1, sms));
     const uint32_t chunk = (count + scatter_blocks - 1u) / scatter_blocks;
     const uint32_t used = (count + chunk - 1u) / chunk;
-    if (bins * 4u > 48u * 1024u) {
-        if ((status = record_cuda(cudaFuncSetAttribute(dev::scatter_order_blocked_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(bins * 4u))))) {
-            return status;
-        }
-    }
     return launch_chained(true, dev::scatter_order_blocked_kernel, used, 1024u, bins * 4u, stream, keys, hist, count,
                           bins, chunk, order);
 }
@@ -941,8 +934,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
         const uint32_t warps = block / 32u;
         const size_t shm = smem(warps);
         if (shm > 48u * 1024u) {
-            st = record_cuda(cudaFuncSetAttribute(reinterpret_cast<const void *>(fn),
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shm)));
+            st = allow_shared(reinterpret_cast<const void *>(fn), attr.sharedSizeBytes, smem_optin);
             if (st) { return st; }
         }
         int per_sm = 0;

@@ -40,4 +40,13 @@ uint32_t launch_chained(bool chained, void (*fn)(Params...), uint32_t grid, uint
     return record_cuda(cudaLaunchKernelEx(&config, fn, args...));
 }
 
+// Lets `fn` (of `fixed` bytes of static shared memory) be launched with any
+// dynamic shared memory that a block may have, `optin` bytes in all.  The limit
+// is the process's, so every call sets the same one: set to a call's own size,
+// it could fall between another thread's setting and its launch.
+inline uint32_t allow_shared(const void *fn, size_t fixed, int optin) {
+    return record_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            optin - static_cast<int>(fixed)));
+}
+
 } // namespace nxg

@@ -743,8 +743,9 @@ cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, co
     const uint32_t searched = triangle_count - rows;
     const size_t copy = sizeof(float4) * cluster_scratch_words(clusters);
     const uint32_t tail_threads = ((rows + kTailCtas - 1u) / kTailCtas + 31u) / 32u * 32u;
+    // The largest copy, whatever this call's: the limit is the process's.
     cudaError_t e = cudaFuncSetAttribute(stencil_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(copy));
+                                         static_cast<int>(sizeof(float4) * cluster_scratch_words(kMaxClusters)));
     if (e != cudaSuccess) { return e; }
     cudaLaunchConfig_t config{};
     cudaLaunchAttribute attributes[2];
