@@ -724,6 +724,8 @@ bool valid_tile(uint32_t P, uint32_t lanes, uint32_t ppt) {
 // the built-in tile is free, it takes up to kWalkNoiseWarps), else four CVs per lane on the narrowest power-of-two group that
 // holds the strand (what the autotuner starts from: unregistered, longer
 // strands take the lane walk as well).
+bool lane_groups(uint32_t packed) { return packed != 0u && (packed & 0xffu) != 1u; }
+
 uint32_t registered_tile(uint32_t P, bool noise) {
     return P <= kMaxParallelCvs ? g_tiles[P][noise ? 1 : 0].load(std::memory_order_relaxed) : 0u;
 }
@@ -828,6 +830,8 @@ uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_
                           bins, chunk, order);
 }
 
+namespace {
+
 // Whether the lane walk takes its strands in the order of their guides.  The
 // order makes the warps of an SM read the same guide rows from L1, and costs
 // three launches, two passes over a key per strand, and scattered instead of
@@ -846,13 +850,24 @@ bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, u
     return noise ? points >= 7000000u : points >= 24000000u && count <= 1700000u;
 }
 
+} // namespace
+
+LaunchForm launch_form(uint32_t guide_count, const nxg_generation_params &params, uint32_t count, uint32_t samples) {
+    const uint32_t P = params.cvs_per_strand;
+    const bool noise = resolve_params(params, 1.0f).noise != 0u;
+    LaunchForm form;
+    form.tile = registered_tile(P, noise);
+    form.ordered = lane_groups(form.tile) || wants_order(guide_count, count, P, noise, samples);
+    return form;
+}
+
 // The guide-offset table for this frame, the strand order where one is wanted
-// and not prepared, then the persistent generate kernel.
+// and not ready, then the persistent generate kernel.
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
                          uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
-                         const nxg_classic_apply_desc *classic, bool prepared, uint32_t samples) {
+                         const nxg_classic_apply_desc *classic, LaunchForm form, bool order_ready) {
     set_last_cuda_error(0);
     const uint32_t P = params.cvs_per_strand;
     const WorkspaceLayout ws = workspace_layout(asset.header.guide_count, count, P);
@@ -878,7 +893,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     uint32_t status = NXG_ERROR_NONE;
     const bool parallel = parallel_path(asset.header.guide_count, P);
     if (!parallel && (!long_walk_path(asset.header.guide_count, count, P) || workspace_bytes < ws.wanted)) {
-        if (!prepared &&
+        if (!order_ready &&
             (status = launch_order(asset, params.seed, first, count, P, workspace, stream, false))) {
             return status;
         }
@@ -894,15 +909,14 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     g.guide_frames = offsets + uint64_t{asset.header.guide_count} * P;
     const bool noise = g.p.noise != 0u;
     // The lane walk, unless a lane-group tile is registered for these strands.
-    const uint32_t packed = registered_tile(P, noise);
-    const bool walk = packed == 0u || (packed & 0xffu) == 1u;
-    const bool ordered = !walk || wants_order(asset.header.guide_count, count, P, noise, samples);
+    const uint32_t packed = form.tile;
+    const bool walk = !lane_groups(packed);
     {
         const uint64_t n = uint64_t{asset.header.guide_count} * P;
         const uint32_t threads = 256u;
         const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n + threads - 1u) / threads,
                                                                           static_cast<uint64_t>(sms) * 16u));
-        const bool sort = ordered && !prepared;
+        const bool sort = form.ordered && !order_ready;
         // The first launch is an ordinary one.  (Chained to the walk of the
         // motion sample before, its CTAs and the next walk's took the SMs that
         // walk still needed: five samples of 250,000 x 24, 791 against 735 us.)
@@ -913,7 +927,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
             return status;
         }
     }
-    if (!ordered) { g.order = nullptr; }
+    if (!form.ordered) { g.order = nullptr; }
     const bool classic_scalars = g.scalars != nullptr;
     int device = 0, smem_optin = 48 * 1024;
     if (cudaGetDevice(&device) == cudaSuccess) {
@@ -974,9 +988,8 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
             return dev::walk_head_bytes(noise, P, w) + dev::walk_warp_bytes(noise, classic_scalars) * w;
         });
     }
-    int lanes = 32, ppt = 4;
-    uint32_t tile_block = 0u;
-    default_tile(P, noise, &lanes, &ppt, &tile_block);
+    const int lanes = static_cast<int>(packed & 0xffu), ppt = static_cast<int>((packed >> 8) & 0xffu);
+    const uint32_t tile_block = ((packed >> 16) & 0xffu) * 32u;
     if (g.roots || g.root_uvs || g.point_counts) {  // the lane-walk kernel writes its own
         const uint32_t threads = 256u;
         const uint32_t per_block = threads;  // one strand per thread
@@ -1057,7 +1070,8 @@ uint32_t nxg_generate_packed_range(const nxg_device_asset_desc *asset, const nxg
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
-                                workspace_bytes, s, nullptr, nullptr, false);
+                                workspace_bytes, s, nullptr, nullptr,
+                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u), false);
 }
 
 uint32_t nxg_prepare_strand_order(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
@@ -1100,7 +1114,8 @@ uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset, const n
     const nxg_launch_config default_config{128u};
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
-                                workspace_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr, true);
+                                workspace_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr,
+                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u), true);
 }
 
 uint32_t nxg_query_strand_states(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1323,10 +1338,12 @@ extern "C" uint32_t nxg_generate_motion_packed(const nxg_device_asset_desc *asse
     }
     const auto s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
+    const nxg::LaunchForm form =
+        nxg::launch_form(asset->header.guide_count, *params, params->strand_count, sample_count);
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, outputs[i], cfg, 0u,
-                                     params->strand_count, workspace, workspace_bytes, s, nullptr, nullptr,
-                                     i != 0u, sample_count);
+                                     params->strand_count, workspace, workspace_bytes, s, nullptr, nullptr, form,
+                                     i != 0u);
     }
     return error;
 }
@@ -1349,11 +1366,12 @@ extern "C" uint32_t nxg_generate_motion(const nxg_device_asset_desc *asset, cons
     const uint64_t per_sample = uint64_t{params->strand_count} * params->cvs_per_strand * 3u;
     nxg_packed_output_desc none{};
     none.radius_scale = 1.0f;
+    const nxg::LaunchForm form =
+        nxg::launch_form(asset->header.guide_count, *params, params->strand_count, sample_count);
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         float *dst = reinterpret_cast<float *>(output->points) + per_sample * i;
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, none, cfg, 0u, params->strand_count,
-                                     workspace, workspace_bytes, s, dst, nullptr,
-                                     i != 0u, sample_count);
+                                     workspace, workspace_bytes, s, dst, nullptr, form, i != 0u);
     }
     return error;
 }

@@ -632,12 +632,20 @@ uint32_t check_workspace(const nxg_device_asset_desc &asset, uint32_t count, uin
                          uint64_t bytes);
 uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_t first, uint32_t count,
                       uint32_t P, void *workspace, cudaStream_t stream, bool cleared);
-// With `prepared`, the workspace holds the strand order of this range;
-// `samples` frames of it share that order.
+// How a call's strands are generated, decided once per call: the tile
+// registered for them (which another thread may change meanwhile) and whether
+// they are taken in the strand order.
+struct LaunchForm {
+    uint32_t tile;
+    bool ordered;
+};
+// `samples`: frames that share one strand order.
+LaunchForm launch_form(uint32_t guide_count, const nxg_generation_params &params, uint32_t count, uint32_t samples);
+// `order_ready`: the workspace holds the strand order of this range.
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
                          const nxg_launch_config &config, uint32_t first, uint32_t count, void *workspace,
                          uint64_t workspace_bytes, cudaStream_t stream, float *vec3_points,
-                         const nxg_classic_apply_desc *classic, bool prepared, uint32_t samples = 1u);
+                         const nxg_classic_apply_desc *classic, LaunchForm form, bool order_ready);
 
 } // namespace nxg

@@ -76,3 +76,52 @@ def test_small_and_large_calls_at_once(cuda, nxg_lib):
         return body
 
     run_threads(*[generating(p) for p in calls], *[searching(m) for m in meshes])
+
+
+def test_motion_call_keeps_its_form(cuda, nxg_lib):
+    """Lane-group tiles registered and withdrawn by another thread while a
+    motion call is enqueued: every sample holds every strand (the lane groups
+    read a strand order, which a call of this size writes only if its first
+    sample takes them)."""
+    import torch
+    from nanoxgen_b200 import fixtures
+    from nanoxgen_b200.asset import build_asset
+    from nanoxgen_b200.generator import (DeformedGeometry, DeviceAsset, allocate_outputs, generate_motion_packed,
+                                         set_tile)
+    w = fixtures.plain_sphere(strands=3000)
+    asset = build_asset(w.build_input, w.stencil_slots)
+    d, params, samples = DeviceAsset(asset), w.params.copy(cvs_per_strand=24), 6
+    rest = torch.from_numpy(np.ascontiguousarray(asset.positions())).cuda()
+    frames = [DeformedGeometry(positions=rest * (1.0 + 0.01 * k)) for k in range(samples)]
+    times = np.linspace(0.0, 1.0, samples).astype(np.float32)
+    outputs = [allocate_outputs(3000, 24, "cuda") for _ in frames]
+    want = [c.points.clone() for c in generate_motion_packed(d, params, frames, times, outputs=outputs)]
+    torch.cuda.synchronize()
+    done = threading.Event()
+
+    def toggling():
+        while not done.is_set():
+            set_tile(24, True, 8, 4, 128)
+            set_tile(24, True)
+
+    def generating():
+        try:
+            stream = torch.cuda.Stream()
+            for _ in range(300):
+                with torch.cuda.stream(stream):
+                    d.workspace(params, 3000).fill_(255)
+                    for o in outputs:
+                        o[0].fill_(float("nan"))
+                    generate_motion_packed(d, params, frames, times, outputs=outputs, stream=stream)
+                    # lane groups and lane walk agree to the generator's bar
+                    near = [((o[0][:, :3] - p[:, :3]).norm(dim=1).max() <= 1e-5 * asset.bbox_diagonal())
+                            for o, p in zip(outputs, want)]
+                stream.synchronize()
+                assert all(bool(n) for n in near)
+        finally:
+            done.set()
+
+    try:
+        run_threads(toggling, generating)
+    finally:
+        set_tile(24, True)
