@@ -639,8 +639,10 @@ struct LaunchForm {
     uint32_t tile;
     bool ordered;
 };
-// `samples`: frames that share one strand order.
-LaunchForm launch_form(uint32_t guide_count, const nxg_generation_params &params, uint32_t count, uint32_t samples);
+// `samples`: frames that share one strand order; `prepared`: the caller has
+// prepared it.
+LaunchForm launch_form(uint32_t guide_count, const nxg_generation_params &params, uint32_t count, uint32_t samples,
+                       bool prepared);
 // `order_ready`: the workspace holds the strand order of this range.
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,
