@@ -417,11 +417,11 @@ uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset,
  * (2, 4, 8, 16 or 32) owns one strand, each lane `cvs_per_lane` consecutive
  * CVs (1, 2 or 4; lanes * cvs <= 128 and >= the strand's CVs); a CTA has
  * `block_size` threads (0: take nxg_launch_config::block_size).
- * lanes_per_strand 1 (with cvs_per_lane 1, strands of 2..32 CVs) selects the
- * lane-walk generator: base curve and stores lane-parallel, one lane walking
- * each strand's noise frame; its block_size is an upper bound (at most 384
- * threads with noise, 256 without).  It is the built-in choice for 2..32
- * CVs, and longer strands take it too while no tile is registered for them. */
+ * lanes_per_strand 1 selects the lane-walk generator, the built-in choice (base
+ * curve and stores lane-parallel, one lane walking each strand's noise frame);
+ * its cvs_per_lane is 1 for strands of 2..32 CVs and the CV count for longer
+ * ones, and its block_size is an upper bound (at most 384 threads with noise,
+ * 256 without). */
 typedef struct nxg_tile {
     uint32_t lanes_per_strand;
     uint32_t cvs_per_lane;
@@ -433,18 +433,16 @@ typedef struct nxg_tile {
  * built-in choice.  Thread-safe; takes effect at the next launch. */
 uint32_t nxg_set_tile(uint32_t cvs_per_strand, uint32_t noise, const nxg_tile *tile);
 
-/* The tile registered for this CV count and noise setting, else the built-in
- * one (for more than 32 CVs the lane-group tile the autotuner starts from;
- * while none is registered such strands take the lane walk, and a call that
- * does not fill the GPU takes smaller CTAs). */
+/* The tile the next launch for this CV count and noise setting will use: the
+ * registered one, else the built-in one.  Registering the built-in one again
+ * changes nothing.  (A call that does not fill the GPU takes smaller CTAs.) */
 uint32_t nxg_get_tile(uint32_t cvs_per_strand, uint32_t noise, nxg_tile *tile);
 
-/* Autotuner: prepares the strand order, then times every admissible tile
- * (lane groups and CVs per lane that hold the strand, CTAs of
- * 64/128/256/384/512 threads) over `repeats` launches of nxg_generate_packed_ordered with CUDA
+/* Autotuner: prepares the strand order, then times the built-in tile and every
+ * other admissible one (lane groups and CVs per lane that hold the strand, CTAs
+ * of 64/128/256/384/512 threads) over `repeats` launches of nxg_generate_packed_ordered with CUDA
  * events on `stream`, registers the fastest with nxg_set_tile and returns
- * it (for more than 32 CVs nothing stays registered when the lane walk is
- * fastest, and the tile returned is nxg_get_tile's).  It writes the outputs and synchronises the stream, so it is a
+ * it (nothing stays registered when the built-in one is fastest).  It writes the outputs and synchronises the stream, so it is a
  * set-up call, not part of the enqueue-only path. */
 uint32_t nxg_autotune_packed(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
                              const nxg_generation_params *params, const nxg_packed_output_desc *output,

@@ -707,47 +707,32 @@ KernelFn pick_lanes(int lanes, bool noise, bool classic) {
 // Packed as lanes | ppt << 8 | (block / 32) << 16; 0 means "not set".
 std::atomic<uint32_t> g_tiles[kMaxParallelCvs + 1][2];
 
-// Longest strand a lane-walk tile (lanes 1) can be registered for.  Longer
-// strands take the lane walk unless a lane-group tile is registered for them.
-constexpr uint32_t kMaxLaneWalkTile = 32u;
-
-bool valid_tile(uint32_t P, uint32_t lanes, uint32_t ppt) {
-    if (lanes == 1u) { return ppt == 1u && P >= 2u && P <= kMaxLaneWalkTile; }
-    const bool lanes_ok = lanes == 2u || lanes == 4u || lanes == 8u || lanes == 16u || lanes == 32u;
-    const bool ppt_ok = ppt == 1u || ppt == 2u || ppt == 4u;
-    return lanes_ok && ppt_ok && lanes * ppt >= P && P >= 2u && P <= kMaxParallelCvs;
+uint32_t packed_tile(const nxg_tile &t) {
+    return t.lanes_per_strand | (t.cvs_per_lane << 8) | ((t.block_size + 31u) / 32u << 16);
 }
-
-// Tile shape for P CVs: the registered one, else the lane-walk generator for
-// 2..32 CVs (lanes_per_strand 1; CTAs of 352 threads with noise, 256
-// without: with noise the size callers have been told, of which the launch of
-// the built-in tile is free, it takes up to kWalkNoiseWarps), else four CVs per lane on the narrowest power-of-two group that
-// holds the strand (what the autotuner starts from: unregistered, longer
-// strands take the lane walk as well).
-bool lane_groups(uint32_t packed) { return packed != 0u && (packed & 0xffu) != 1u; }
 
 uint32_t registered_tile(uint32_t P, bool noise) {
     return P <= kMaxParallelCvs ? g_tiles[P][noise ? 1 : 0].load(std::memory_order_relaxed) : 0u;
 }
 
-void default_tile(uint32_t P, bool noise, int *lanes, int *ppt, uint32_t *block) {
-    if (const uint32_t packed = registered_tile(P, noise)) {
-        *lanes = static_cast<int>(packed & 0xffu);
-        *ppt = static_cast<int>((packed >> 8) & 0xffu);
-        *block = ((packed >> 16) & 0xffu) * 32u;
-        return;
-    }
-    if (P >= 2u && P <= kMaxLaneWalkTile) {  // the lane-walk generator
-        *lanes = 1;
-        *ppt = 1;
-        *block = noise ? 352u : 256u;
-        return;
-    }
-    *ppt = 4;
-    int l = 2;
-    while (l < 32 && static_cast<uint32_t>(l * 4) < P) { l *= 2; }
-    *lanes = l;
-    *block = 0u;
+bool lane_groups(uint32_t packed) { return packed != 0u && (packed & 0xffu) != 1u; }
+
+// The lane walk's tile has one lane per strand.  Its CVs per lane read 1 up to
+// 32 CVs, and the strand's CV count past them.
+uint32_t lane_walk_ppt(uint32_t P) { return P <= 32u ? 1u : P; }
+
+bool valid_tile(uint32_t P, uint32_t lanes, uint32_t ppt) {
+    if (lanes == 1u) { return ppt == lane_walk_ppt(P) && P >= 2u && P <= kMaxParallelCvs; }
+    const bool lanes_ok = lanes == 2u || lanes == 4u || lanes == 8u || lanes == 16u || lanes == 32u;
+    const bool ppt_ok = ppt == 1u || ppt == 2u || ppt == 4u;
+    return lanes_ok && ppt_ok && lanes * ppt >= P && P >= 2u && P <= kMaxParallelCvs;
+}
+
+// The tile of strands without a registered one: the lane walk.  Registering it
+// registers none.  (Up to 32 CVs with noise the launch is free to take CTAs of
+// up to kWalkNoiseWarps, more than the 352 threads its callers have been told.)
+nxg_tile builtin_tile(uint32_t P, bool noise) {
+    return {1u, lane_walk_ppt(P), !noise ? 256u : (P <= 32u ? 352u : 32u * static_cast<uint32_t>(dev::kWalkNoiseWarps))};
 }
 
 KernelFn pick_kernel(int lanes, int ppt, bool noise, bool classic) {
@@ -967,9 +952,12 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
                     : uint32_t{NXG_ERROR_NONE};
     };
     if (walk) {
-        uint32_t warps = packed ? std::max(1u, (packed >> 16) & 0xffu) : (noise ? dev::kWalkNoiseWarps : 8u);
-        g.batch = 32u;
-        if (packed == 0u) {
+        uint32_t warps = noise ? dev::kWalkNoiseWarps : 8u;
+        if (packed) {  // a registered CTA size is a bound
+            const uint32_t tile_warps = (packed >> 16) & 0xffu;
+            warps = std::min(warps, tile_warps ? tile_warps : (config.block_size + 31u) / 32u);
+        }
+        {
             // Every warp the GPU holds takes the same number of batches, of
             // equal size: a multiple of four strands, what a base and a store
             // pass take.  A warp's time is the walk along one strand, whatever
@@ -1187,6 +1175,7 @@ uint32_t nxg_query_walk_states(const nxg_device_asset_desc *asset, const nxg_def
 uint32_t nxg_set_tile(uint32_t cvs_per_strand, uint32_t noise, const nxg_tile *tile) {
     if (cvs_per_strand < 2u || cvs_per_strand > nxg::kMaxParallelCvs) { return NXG_ERROR_INVALID_ARGUMENT; }
     std::atomic<uint32_t> &slot = nxg::g_tiles[cvs_per_strand][noise ? 1 : 0];
+    const uint32_t builtin = nxg::packed_tile(nxg::builtin_tile(cvs_per_strand, noise != 0u));
     if (!tile) {
         slot.store(0u, std::memory_order_relaxed);
         return NXG_ERROR_NONE;
@@ -1194,19 +1183,16 @@ uint32_t nxg_set_tile(uint32_t cvs_per_strand, uint32_t noise, const nxg_tile *t
     if (!nxg::valid_tile(cvs_per_strand, tile->lanes_per_strand, tile->cvs_per_lane) || tile->block_size > 1024u) {
         return NXG_ERROR_INVALID_ARGUMENT;
     }
-    const uint32_t warps = (tile->block_size + 31u) / 32u;
-    slot.store(tile->lanes_per_strand | (tile->cvs_per_lane << 8) | (warps << 16), std::memory_order_relaxed);
+    const uint32_t packed = nxg::packed_tile(*tile);
+    slot.store(packed == builtin ? 0u : packed, std::memory_order_relaxed);
     return NXG_ERROR_NONE;
 }
 
 uint32_t nxg_get_tile(uint32_t cvs_per_strand, uint32_t noise, nxg_tile *tile) {
     if (!tile || cvs_per_strand < 2u || cvs_per_strand > nxg::kMaxParallelCvs) { return NXG_ERROR_INVALID_ARGUMENT; }
-    int lanes = 0, ppt = 0;
-    uint32_t block = 0u;
-    nxg::default_tile(cvs_per_strand, noise != 0u, &lanes, &ppt, &block);
-    tile->lanes_per_strand = static_cast<uint32_t>(lanes);
-    tile->cvs_per_lane = static_cast<uint32_t>(ppt);
-    tile->block_size = block;
+    const uint32_t packed = nxg::registered_tile(cvs_per_strand, noise != 0u);
+    *tile = packed ? nxg_tile{packed & 0xffu, (packed >> 8) & 0xffu, (packed >> 16) * 32u}
+                   : nxg::builtin_tile(cvs_per_strand, noise != 0u);
     return NXG_ERROR_NONE;
 }
 
@@ -1255,39 +1241,35 @@ uint32_t nxg_autotune_packed(const nxg_device_asset_desc *asset, const nxg_defor
         *ms /= static_cast<float>(reps);
         return NXG_ERROR_NONE;
     };
-    // Strands too long for a registered lane-walk tile: nothing registered
-    // (the lane walk) is a candidate too.
-    bool unregistered = P > nxg::kMaxLaneWalkTile;
-    if (unregistered) {
-        nxg_set_tile(P, noise ? 1u : 0u, nullptr);
-        error = nxg_get_tile(P, noise ? 1u : 0u, &winner);
-        if (!error) { error = time(&winner_ms); }
-    }
+    // Nothing registered is the first candidate, and stays unless another is faster.
+    winner = nxg::builtin_tile(P, noise);
+    nxg_set_tile(P, noise ? 1u : 0u, nullptr);
+    error = time(&winner_ms);
     const uint32_t blocks[5] = {64u, 128u, 256u, 384u, 512u};
     for (uint32_t lanes = 1u; lanes <= 32u && !error; lanes *= 2u) {
         for (uint32_t ppt = 1u; ppt <= 4u && !error; ppt *= 2u) {
             // tiles that hold the strand without idling half of their lanes
             if (!nxg::valid_tile(P, lanes, ppt) || (lanes > 2u && lanes * ppt >= 2u * P)) { continue; }
             for (const uint32_t block : blocks) {
+                if (lanes == 1u && block >= nxg::builtin_tile(P, noise).block_size) { break; }  // no bound
                 const nxg_tile tile{lanes, ppt, block};
                 nxg_set_tile(P, noise ? 1u : 0u, &tile);
                 float ms = 0.0f;
                 if ((error = time(&ms))) { break; }
-                if (winner.lanes_per_strand == 0u || ms < winner_ms) {
+                if (ms < winner_ms) {
                     winner = tile;
                     winner_ms = ms;
-                    unregistered = false;
                 }
             }
         }
     }
     cudaEventDestroy(start);
     cudaEventDestroy(stop);
-    if (error || winner.lanes_per_strand == 0u) {
+    if (error) {
         nxg::g_tiles[P][noise ? 1 : 0].store(saved, std::memory_order_relaxed);
-        return error ? error : NXG_ERROR_INVALID_ARGUMENT;
+        return error;
     }
-    nxg_set_tile(P, noise ? 1u : 0u, unregistered ? nullptr : &winner);
+    nxg_set_tile(P, noise ? 1u : 0u, &winner);
     if (best) { *best = winner; }
     if (best_ms) { *best_ms = winner_ms; }
     return NXG_ERROR_NONE;

@@ -38,3 +38,32 @@ def test_a_prepared_order_is_taken(sphere, strands, cvs, noise):
     left_out[order[::3].long()] = True
     assert bool(got[left_out].isnan().all())
     assert torch.equal(got[~left_out], want[~left_out])
+
+
+@pytest.mark.parametrize("noise", [False, True])
+@pytest.mark.parametrize("cvs", [2, 16, 32, 33, 64, 128])
+def test_tiles_read_and_registered_again(sphere, cvs, noise):
+    """The tile that is read is the one in use: registered again, points are
+    the same bits (a lane-group kernel's differ), and it reads the same.  A
+    lane-walk tile of any CTA size leaves the bits alone; the autotuner
+    returns what it leaves in use."""
+    import torch
+    from nanoxgen_b200.generator import autotune, generate_packed, get_tile, set_tile
+    d, params = sphere
+    params = params.copy(strand_count=401, cvs_per_strand=cvs, noise_amplitude=0.1 if noise else 0.0)
+    try:
+        want = generate_packed(d, params).points
+        builtin = get_tile(cvs, noise)
+        set_tile(cvs, noise, *builtin)
+        assert get_tile(cvs, noise) == builtin and builtin[0] == 1
+        assert torch.equal(generate_packed(d, params).points, want)
+        for block in (0, 32, 96, 1024):
+            set_tile(cvs, noise, builtin[0], builtin[1], block)
+            assert torch.equal(generate_packed(d, params).points, want)
+        set_tile(cvs, noise, 32, 4, 64)
+        assert get_tile(cvs, noise) == (32, 4, 64)
+        tile, _ = autotune(d, params, torch.empty_like(want), repeats=1)
+        assert get_tile(cvs, noise) == tile
+    finally:
+        set_tile(cvs, noise)
+    assert get_tile(cvs, noise) == builtin
