@@ -361,9 +361,10 @@ uint32_t nxg_validate_motion_request(const nxg_device_asset_desc *asset,
  * strands of this asset at params->cvs_per_strand CVs: the strand-locality
  * sort (keys, permutation, per-guide bins) and the per-frame guide-offset
  * table (guide_count x cvs_per_strand float4, then 2 guide records per guide).
- * Past 128 CVs the table is included up to 1,024 CVs while there are no more
- * guides than strands, and optional: a workspace without room for it is
- * accepted and takes a slower kernel.  The workspace must be 256-byte
+ * Past 128 CVs the table is included up to 1,024 CVs while the asset has no
+ * more guides than the description (params->strand_count) strands, and
+ * optional: a workspace without room for it is accepted and takes a slower
+ * kernel, whose points differ in rounding.  The workspace must be 256-byte
  * aligned; its contents need no initialisation. */
 uint64_t nxg_packed_workspace_size(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
                                    uint32_t strand_count);

@@ -565,7 +565,7 @@ constexpr uint64_t kWorkspaceAlign = 256u;
 inline uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1u) / a * a; }
 
 struct WorkspaceLayout {
-    uint64_t keys, order, hist, offsets, total, wanted;
+    uint64_t keys, order, hist, offsets, total, walked;
 };
 
 // Largest guide-offset table the warp-parallel generator stages; beyond it
@@ -580,17 +580,14 @@ bool parallel_path(uint32_t guide_count, uint32_t P) {
 // Strands of more than kMaxParallelCvs CVs take the lane walk too where the
 // workspace holds their offset table (20,011 strands x 160 CVs with noise, 512
 // guides: 1,214 us on the serial kernel).  The workspace need not: a caller's
-// that holds the order alone stays valid and takes the serial kernel.  The
-// queried size asks for the table when it is no larger than the strands' own
-// points, so it never dominates a caller's memory.
-bool long_walk_path(uint32_t guide_count, uint32_t count, uint32_t P) {
-    return P > kMaxParallelCvs && P <= dev::kWalkMaxCvs && guide_count <= count &&
-           uint64_t{guide_count} * P * 16u <= kMaxOffsetTableBytes;
+// that holds the order alone stays valid and takes the serial kernel.
+bool long_walk_path(uint32_t guide_count, uint32_t P) {
+    return P > kMaxParallelCvs && P <= dev::kWalkMaxCvs && uint64_t{guide_count} * P * 16u <= kMaxOffsetTableBytes;
 }
 
 // keys[count] | order[count] | bins[guides + 1] | offsets[guides * P] (float4)
 // followed by the guide frame records [guides * 2] (float4).  `total` is what
-// a caller has to provide, `wanted` what the size query asks for.
+// a caller has to provide, `walked` what the lane walk needs.
 WorkspaceLayout workspace_layout(uint32_t guide_count, uint32_t count, uint32_t P) {
     WorkspaceLayout w{};
     w.keys = 0u;
@@ -599,7 +596,7 @@ WorkspaceLayout workspace_layout(uint32_t guide_count, uint32_t count, uint32_t 
     w.offsets = w.hist + align_up((uint64_t{guide_count} + 1u) * 4u, kWorkspaceAlign);
     const uint64_t table = align_up(uint64_t{guide_count} * (P + 2u) * 16u, kWorkspaceAlign);
     w.total = w.offsets + (parallel_path(guide_count, P) ? table : 0u);
-    w.wanted = w.offsets + (parallel_path(guide_count, P) || long_walk_path(guide_count, count, P) ? table : 0u);
+    w.walked = w.offsets + (parallel_path(guide_count, P) || long_walk_path(guide_count, P) ? table : 0u);
     return w;
 }
 
@@ -882,7 +879,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     const int sms = device_sm_count();
     uint32_t status = NXG_ERROR_NONE;
     const bool parallel = parallel_path(asset.header.guide_count, P);
-    if (!parallel && (!long_walk_path(asset.header.guide_count, count, P) || workspace_bytes < ws.wanted)) {
+    if (!parallel && (!long_walk_path(asset.header.guide_count, P) || workspace_bytes < ws.walked)) {
         if (!order_ready &&
             (status = launch_order(asset, params.seed, first, count, P, workspace, stream, false))) {
             return status;
@@ -1031,7 +1028,11 @@ extern "C" {
 uint64_t nxg_packed_workspace_size(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
                                    uint32_t strand_count) {
     if (!asset || !params || strand_count == 0u) { return 0u; }
-    return nxg::workspace_layout(asset->header.guide_count, strand_count, params->cvs_per_strand).wanted;
+    // The optional table (past 128 CVs) is asked for while it is no larger than
+    // the description's own points, so it never dominates a caller's memory:
+    // by the whole description, whose ranges are then all generated alike.
+    const auto ws = nxg::workspace_layout(asset->header.guide_count, strand_count, params->cvs_per_strand);
+    return asset->header.guide_count <= std::max(strand_count, params->strand_count) ? ws.walked : ws.total;
 }
 
 uint32_t nxg_generate_packed(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,

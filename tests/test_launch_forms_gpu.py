@@ -67,3 +67,18 @@ def test_tiles_read_and_registered_again(sphere, cvs, noise):
     finally:
         set_tile(cvs, noise)
     assert get_tile(cvs, noise) == builtin
+
+
+@pytest.mark.parametrize("cvs", [129, 200])
+def test_short_ranges_of_long_strands(sphere, cvs):
+    """Ranges of fewer strands than guides, past 128 CVs, have the whole
+    call's points bit for bit (the walk's; the serial kernel's differ)."""
+    import torch
+    from nanoxgen_b200.generator import generate_packed
+    d, params = sphere
+    guides = d.header.guide_count
+    params = params.copy(strand_count=3 * guides, cvs_per_strand=cvs)
+    want = generate_packed(d, params).points.view(-1, cvs, 4)
+    for first, count in ((0, guides - 1), (guides, 1), (2 * guides + 1, guides - 1)):
+        got = generate_packed(d, params, first_strand=first, count=count).points.view(-1, cvs, 4)
+        assert torch.equal(got, want[first:first + count])
