@@ -237,6 +237,18 @@ __device__ inline F3 fx_fallback_surface_u(F3 n) {
     return xnormalize(xcross(n, axis));
 }
 
+// 2 (noise - 0.5) of the three axes at one distance along a strand, each value
+// in the reference's rounding.  Out of line: only a magnitude with a ramp or a
+// segment longer than a lattice window takes it.
+static __device__ __noinline__ F3 fx_noise_at(const float4 *table, F3 domain, float distance) {
+    const auto value = [table](float x, float y, float z) {
+        return 2.0f * __fsub_rn(classic_noise(table, x, y, z), 0.5f);
+    };
+    return F3{value(__fadd_rn(domain.x, distance), domain.y, domain.z),
+              value(domain.x, __fadd_rn(domain.y, distance), domain.z),
+              value(domain.x, domain.y, __fadd_rn(domain.z, distance))};
+}
+
 // apply_noise (xgen_classic_runtime.cpp:897-1040) on one strand: the
 // module's parameters, then the SgCurve frame transported from the surface
 // normal along the current curve with gradient-noise displacement of every
@@ -331,17 +343,16 @@ __device__ inline bool fx_noise(FxCurve &k, int P, const DeviceExpression *m, co
             const float distance = __fmul_rn(travelled, effective_frequency);
             F3 noise = later;
             if (per_cv) {
-                noise.x = walk_direct_noise(table, 0u, __fadd_rn(domain.x, distance), domain.y, domain.z);
-                noise.y = walk_direct_noise(table, 0u, domain.x, __fadd_rn(domain.y, distance), domain.z);
-                noise.z = walk_direct_noise(table, 0u, domain.x, domain.y, __fadd_rn(domain.z, distance));
+                noise = fx_noise_at(table, domain, distance);
             } else if ((cv & 1) != 0) {
                 float after = distance;
                 if (cv + 1 < P) {
                     const F3 d = xsub(next_base, current_base);
                     after = __fmul_rn(__fadd_rn(travelled, __fsqrt_rn(xdot(d, d))), effective_frequency);
                 }
-                bool lattice = true;
-                if (__any_sync(lanes, !(after <= window.limit))) {
+                // The last CV alone is not worth another window.
+                bool lattice = after <= window.limit;
+                if (cv + 1 < P && __any_sync(lanes, !lattice)) {
                     const uint4 w = walk_fill_window(domain, distance, window, lat, table, 0u, lanes);
                     window = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
                     lattice = after <= window.limit;
@@ -356,13 +367,8 @@ __device__ inline bool fx_noise(FxCurve &k, int P, const DeviceExpression *m, co
                     noise = F3{low2(x), low2(y), low2(z)};
                     later = F3{high2(x), high2(y), high2(z)};
                 } else {
-                    const auto at = [&](float d) {
-                        return F3{walk_direct_noise(table, 0u, __fadd_rn(domain.x, d), domain.y, domain.z),
-                                  walk_direct_noise(table, 0u, domain.x, __fadd_rn(domain.y, d), domain.z),
-                                  walk_direct_noise(table, 0u, domain.x, domain.y, __fadd_rn(domain.z, d))};
-                    };
-                    noise = at(distance);
-                    later = at(after);
+                    noise = fx_noise_at(table, domain, distance);
+                    later = fx_noise_at(table, domain, after);
                 }
             }
             const float lx = __fmul_rn(0.5f * noise.x, magnitude);
