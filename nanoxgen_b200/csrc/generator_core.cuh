@@ -579,8 +579,13 @@ __device__ __forceinline__ void emit_strand(const LaunchArgs &g, const Records &
     __syncwarp();
 }
 
-// offsets[g*P + cv] = sample_guide(g, cv/(P-1)) - guide_root(g) for the frame,
-// in the reference's exact (uncontracted) arithmetic (generate.h:137-205).
+// offsets[g*P + cv] = sample_guide(g, cv/(P-1)) - guide_root(g) for the frame
+// (generate.h:137-205), up to kExactTableCvs CVs in the reference's exact
+// (uncontracted) arithmetic.  Longer strands' points are held to what the
+// serial kernel gives them, whose sample has a rounding less: rms against 64
+// bits of 40,000 strands x 160 without noise 6.79e-8, 7.00e-8 uncontracted.
+constexpr uint32_t kExactTableCvs = 128u;
+
 __device__ __forceinline__ float4 guide_offset_entry(const AssetArgs &a, const FrameArgs &f, uint32_t P, uint32_t gi,
                                                      uint32_t cv) {
     const uint32_t *rec = a.guides + 14u * static_cast<uint64_t>(gi);
@@ -610,7 +615,14 @@ __device__ __forceinline__ float4 guide_offset_entry(const AssetArgs &a, const F
         uint32_t i = static_cast<uint32_t>(x);
         if (i >= count - 1u) { i = count - 2u; }
         const float fr = __fsub_rn(x, static_cast<float>(i));
-        v = xadd(xmul(ld3(f.guide_cvs, first + i), __fsub_rn(1.0f, fr)), xmul(ld3(f.guide_cvs, first + i + 1u), fr));
+        const F3 va = ld3(f.guide_cvs, first + i), vb = ld3(f.guide_cvs, first + i + 1u);
+        const float fa = __fsub_rn(1.0f, fr);
+        if (P <= kExactTableCvs) {
+            v = xadd(xmul(va, fa), xmul(vb, fr));
+        } else {
+            v = F3{__fmaf_rn(va.x, fa, __fmul_rn(vb.x, fr)), __fmaf_rn(va.y, fa, __fmul_rn(vb.y, fr)),
+                   __fmaf_rn(va.z, fa, __fmul_rn(vb.z, fr))};
+        }
     }
     if (!f.deformed_guide_cvs && f.deformed_positions && bound) { v = xsub(xadd(v, groot), rest_root); }
     const F3 d = xsub(v, groot);

@@ -82,3 +82,34 @@ def test_short_ranges_of_long_strands(sphere, cvs):
     for first, count in ((0, guides - 1), (guides, 1), (2 * guides + 1, guides - 1)):
         got = generate_packed(d, params, first_strand=first, count=count).points.view(-1, cvs, 4)
         assert torch.equal(got, want[first:first + count])
+
+
+def test_base_points_past_128_cvs(sphere):
+    """The offset table samples guides for strands past 128 CVs with a fused
+    multiply-add, as the serial kernel does: nearest-guide points are nearer to
+    64 bits than from the reference's three roundings."""
+    import torch
+    from nanoxgen_b200.generator import generate_packed
+    d, params = sphere
+    cvs = 160
+    params = params.copy(strand_count=400, cvs_per_strand=cvs, noise_amplitude=0.0, guide_support_scale=1e-6)
+    out = generate_packed(d, params)
+    got = out.points.cpu().numpy()[:, :3].reshape(-1, cvs, 3)
+    roots = out.roots_numpy()
+    g, F = d.asset.guides(), np.float32
+    curves = d.asset.guide_cvs().reshape(len(g), -1, 3)
+    # The nearest eligible guide, and its curve, at the strand's parameters.
+    near = d.asset.stencil()[roots["triangle_index"]].astype(np.int64)
+    ok = near < len(g)
+    d2 = np.where(ok, ((roots["position"][:, None] - curves[np.where(ok, near, 0), 0]) ** 2).sum(-1), np.inf)
+    guide = curves[near[np.arange(len(near)), d2.argmin(1)]]
+    x = (np.arange(cvs, dtype=F) / F(cvs - 1)) * F(guide.shape[1] - 1)
+    i = np.minimum(x.astype(np.int64), guide.shape[1] - 2)
+    f = (x - i.astype(F))[None, :, None]
+    a, b = guide[:, i], guide[:, i + 1]
+    root = roots["position"][:, None]
+    thrice = root + ((a * (F(1) - f) + b * f) - guide[:, :1])
+    wide = root + (a.astype(np.float64) * (1.0 - f.astype(np.float64)) + b.astype(np.float64) * f - guide[:, :1])
+    rms = lambda e: float(np.sqrt((e.astype(np.float64) ** 2).mean()))
+    assert np.abs(got - wide).max() <= 8 * 2.0 ** -24 * np.abs(wide).max()
+    assert rms(got - wide) < 0.97 * rms(thrice - wide)
