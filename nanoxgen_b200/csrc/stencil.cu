@@ -28,7 +28,12 @@
 // a handful of 128, since a mesh's neighbouring triangles share their guides.
 // For finite positions the (score, guide) order is a total one, so the eight
 // smallest do not depend on the order of search; a CTA that meets a wild
-// position (not finite, or beyond kWild) takes all pairs.  167 us at the size
+// position (not finite, or beyond kWild) takes all pairs.  So does one whose
+// warps' triangles lie scattered over too many clusters, and the whole call
+// where the sort finds a sample of the warps scattered over the mesh: a visit
+// to a cluster costs a warp as much as all pairs cost it over six to eight
+// clusters' guides (200,000 x 4,096 in random triangle order 3,609 us by
+// clusters, 1,200 by all pairs).  155 us at the size
 // above (sorting 21, search 106, the last rows' search partly beside it): bound
 // by the latency of a warp's chain of clusters.  The sorted guides need memory this entry point has no argument
 // for: they are put into the last rows of the output, whose triangles a second
@@ -246,13 +251,15 @@ constexpr uint32_t kClusterGuides = 32u;
 constexpr uint32_t kClusterWords = 4u * kClusterGuides / 4u;  // float4 per cluster: planes x, y, z, guide index
 constexpr uint32_t kMaxClusters = 160u;    // 92 KB of shared memory in the second kernel
 constexpr uint32_t kTailCtas = 8u;         // CTAs of the second kernel, one thread-block cluster
+constexpr uint32_t kTailMaxThreads = 384u;
 constexpr uint32_t kClusterMinGuides = 640u;
 constexpr float kWild = 1.0e15f;           // |coordinate| past it: |d|^2 could overflow
 
 constexpr uint32_t kClusterBoxes = 4u;     // float4 per cluster: roots' box low (and guide count), high, normals' box
 
 // Scratch: kClusterWords float4 per cluster | kClusterBoxes float4 per cluster
-// | one float4 (first word nonzero: a guide is wild).
+// | one float4, in the last row of all: its first word nonzero where every
+// triangle takes all pairs, its second where that is because a guide is wild.
 __host__ __device__ constexpr uint32_t cluster_scratch_words(uint32_t clusters) {
     return clusters * (kClusterWords + kClusterBoxes) + 1u;
 }
@@ -268,16 +275,43 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {  // bits of v three ap
     return r;
 }
 
+// A warp of the sample is scattered where its triangles reach further than 1.7
+// clusters would if they shared out the mesh as squares: neighbours reach
+// 0.07 to 0.15 of a mesh of 50,000 to 200,000 triangles (0.8 to 1.3 of 32 to
+// 128 clusters), a quarter of a ring of 64 quads 0.34 (1.9 of 32, where all
+// pairs are level), two patches of sixteen triangles 0.56 (2.5 of 20).
+constexpr float kScattered = 1.7f * 1.7f;
+
+// The box of the warp's triangles.
+struct WarpBox {
+    F3 lo, hi;
+};
+__device__ __forceinline__ WarpBox warp_box(const TriangleSearch &t) {
+    WarpBox b;
+    b.lo = t.live ? t.centroid : F3{FLT_MAX, FLT_MAX, FLT_MAX};
+    b.hi = t.live ? t.centroid : F3{-FLT_MAX, -FLT_MAX, -FLT_MAX};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        b.lo = F3{fminf(b.lo.x, __shfl_xor_sync(kFull, b.lo.x, o)), fminf(b.lo.y, __shfl_xor_sync(kFull, b.lo.y, o)),
+                  fminf(b.lo.z, __shfl_xor_sync(kFull, b.lo.z, o))};
+        b.hi = F3{fmaxf(b.hi.x, __shfl_xor_sync(kFull, b.hi.x, o)), fmaxf(b.hi.y, __shfl_xor_sync(kFull, b.hi.y, o)),
+                  fmaxf(b.hi.z, __shfl_xor_sync(kFull, b.hi.z, o))};
+    }
+    return b;
+}
+
 // Sorts the guides by the Morton code of their cell (16 cells per axis of
 // the roots' box) and writes the scratch; one CTA.  The order within a cell is
-// arbitrary.
-__global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restrict__ guide_roots,
+// arbitrary.  Each warp also looks at the triangles of one warp of the search.
+__global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
+                                                       const nxg_uint3 *__restrict__ triangles, uint32_t searched,
+                                                       const nxg_vec3 *__restrict__ guide_roots,
                                                        const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count,
                                                        uint32_t clusters, float4 *scratch) {
     constexpr uint32_t kBits = 4u;  // 4,096 cells, of which a surface meets about a fifth
     constexpr uint32_t bin_count = 1u << (3u * kBits);
     __shared__ uint32_t bins[bin_count];
-    __shared__ float bounds[6][32];
+    __shared__ float bounds[6][32], mesh[6][32];
     __shared__ uint32_t warp_sums[32];
     chain_start();
     chain_wait();
@@ -287,6 +321,8 @@ __global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restric
     nxg_vec3 root[kOwn];
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     bool wild = false;
+    TriangleSearch sample;
+    begin_triangle(sample, warp * (searched / 1024u) * 32u + lane, positions, vertex_count, triangles, searched);
 #pragma unroll
     for (uint32_t q = 0; q < kOwn; ++q) {
         const uint32_t i = q * 1024u + tid;
@@ -315,9 +351,35 @@ __global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restric
             bounds[3 + k][warp] = hi[k];
         }
     }
+    const WarpBox box = warp_box(sample);
+    if (lane == 0u) {
+        mesh[0][warp] = box.lo.x;
+        mesh[1][warp] = box.lo.y;
+        mesh[2][warp] = box.lo.z;
+        mesh[3][warp] = box.hi.x;
+        mesh[4][warp] = box.hi.y;
+        mesh[5][warp] = box.hi.z;
+    }
     wild = __syncthreads_or(wild);
-    if (tid == 0u) { scratch[clusters * (kClusterWords + kClusterBoxes)] = make_float4(wild ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f); }
-    if (wild) { return; }
+    // Most of the sample scattered: all pairs (every warp counts alike).
+    float across = 0.0f, own = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float low = mesh[k][lane], high = mesh[3 + k][lane];
+        own = fmaxf(own, high - low);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            low = fminf(low, __shfl_xor_sync(kFull, low, o));
+            high = fmaxf(high, __shfl_xor_sync(kFull, high, o));
+        }
+        across = fmaxf(across, high - low);
+    }
+    const bool all = wild ||
+        __popc(__ballot_sync(kFull, own * own * static_cast<float>(clusters) > kScattered * across * across)) > 16;
+    if (tid == 0u) {
+        scratch[clusters * (kClusterWords + kClusterBoxes)] = make_float4(all ? 1.0f : 0.0f, wild ? 1.0f : 0.0f, 0.0f, 0.0f);
+    }
+    if (all) { return; }
     float extent = 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -565,22 +627,14 @@ __device__ __forceinline__ WarpAim find_aim(const TriangleSearch &t, const WarpB
 // whose box is near enough to the box of the warp's centroids.  A box or ball
 // distance is at most the computed |d|^2 of any pair it covers but for
 // rounding, which kFilterMargin covers.
-__device__ __forceinline__ void search_clusters(TriangleSearch &t, const float4 *scratch, uint32_t clusters,
-                                                const nxg_vec3 *__restrict__ guide_normals) {
+__device__ __forceinline__ void search_clusters(TriangleSearch &t, const WarpBox &bounds, const float4 *scratch,
+                                                uint32_t clusters, const nxg_vec3 *__restrict__ guide_normals) {
     const uint32_t lane = threadIdx.x & 31u;
     const float4 *boxes = scratch + clusters * kClusterWords;
 #pragma unroll
     for (uint32_t k = 0; k < kSlots; ++k) { t.best[k] = {INFINITY, kInvalid}; }
     if (__ballot_sync(kFull, t.live) == 0u) { return; }
-    F3 lo = t.live ? t.centroid : F3{FLT_MAX, FLT_MAX, FLT_MAX};
-    F3 hi = t.live ? t.centroid : F3{-FLT_MAX, -FLT_MAX, -FLT_MAX};
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = F3{fminf(lo.x, __shfl_xor_sync(kFull, lo.x, o)), fminf(lo.y, __shfl_xor_sync(kFull, lo.y, o)),
-                fminf(lo.z, __shfl_xor_sync(kFull, lo.z, o))};
-        hi = F3{fmaxf(hi.x, __shfl_xor_sync(kFull, hi.x, o)), fmaxf(hi.y, __shfl_xor_sync(kFull, hi.y, o)),
-                fmaxf(hi.z, __shfl_xor_sync(kFull, hi.z, o))};
-    }
+    const F3 lo = bounds.lo, hi = bounds.hi;
     WarpBall ball;
     ball.middle = (lo + hi) * 0.5f;
     const F3 out = t.centroid - ball.middle;
@@ -638,25 +692,84 @@ __device__ __forceinline__ bool wild_triangle(const TriangleSearch &t) {
     return t.live && !(fabsf(t.centroid.x) <= kWild && fabsf(t.centroid.y) <= kWild && fabsf(t.centroid.z) <= kWild);
 }
 
+// Whether the CTA's triangles lie scattered over too many clusters: whether its
+// warps' boxes touch more than a twentieth of the clusters and 2.5 on average
+// (neighbours touch 2.3 to 4, two patches of sixteen 8 of 20, 19 of 128; all
+// pairs cost as much as visits to a seventh of them).  Every thread of the CTA
+// calls it.
+__device__ __forceinline__ bool scattered_triangles(const WarpBox &bounds, const float4 *scratch, uint32_t clusters) {
+    const float4 *boxes = scratch + clusters * kClusterWords;
+    uint32_t touched = 0u;
+    for (uint32_t c = threadIdx.x & 31u; c < clusters; c += 32u) {
+        touched += box_distance2(bounds.lo, bounds.hi, boxes[kClusterBoxes * c], boxes[kClusterBoxes * c + 1u]) == 0.0f;
+    }
+    __shared__ uint32_t sum;
+    if (threadIdx.x == 0u) { sum = 0u; }
+    __syncthreads();
+    touched = __reduce_add_sync(kFull, touched);
+    if ((threadIdx.x & 31u) == 0u) { atomicAdd(&sum, touched); }
+    __syncthreads();
+    return sum * 20u > (blockDim.x >> 5) * (clusters + 50u);
+}
+
+// The all-pairs search of one triangle, which every thread of the CTA holds, for
+// finite positions: each takes every blockDim-th guide, and the CTA picks the
+// least (score, guide) eight times.  (By one thread, a triangle that every
+// guide is penalised for takes 70 us of 1,024 guides.)
+__device__ __forceinline__ void share_triangle(TriangleSearch &t, const nxg_vec3 *__restrict__ guide_roots,
+                                               const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count) {
+    constexpr unsigned long long kNone = ~0ull;
+    __shared__ unsigned long long least[2], row[kSlots];
+    unsigned long long last = 0ull;
+    if (threadIdx.x < 2u) { least[threadIdx.x] = kNone; }
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t k = 0; k < kSlots; ++k) {
+        unsigned long long mine = kNone;
+        for (uint32_t gi = threadIdx.x; gi < guide_count; gi += blockDim.x) {
+            const nxg_vec3 r = guide_roots[gi], m = guide_normals[gi];
+            const F3 d = xsub(t.centroid, F3{r.x, r.y, r.z});
+            const float key = __fadd_rn(xdot(d, d), xdot(t.face, F3{m.x, m.y, m.z}) < -0.25f ? kPenalty : 0.0f);
+            const unsigned long long c = static_cast<unsigned long long>(__float_as_uint(key)) << 32 | gi;
+            if ((k == 0u || c > last) && c < mine) { mine = c; }
+        }
+        if (mine != kNone) { atomicMin(&least[k & 1u], mine); }
+        __syncthreads();
+        last = least[k & 1u];
+        if (threadIdx.x == 0u) {
+            least[(k + 1u) & 1u] = kNone;
+            row[k] = last;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kSlots; ++k) {
+        t.best[k] = {__uint_as_float(static_cast<uint32_t>(row[k] >> 32)), static_cast<uint32_t>(row[k])};
+    }
+}
+
 // Triangles [0, searched) from the scratch in global memory (the rows from
-// `searched` on).
-__global__ void __launch_bounds__(kStencilThreads)
+// `searched` on); where every triangle takes all pairs, those of the scratch's
+// rows too but for the last row, which says so.
+__global__ void __launch_bounds__(kStencilThreads, 8)
 stencil_cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
-                       const nxg_uint3 *__restrict__ triangles, uint32_t searched,
+                       const nxg_uint3 *__restrict__ triangles, uint32_t searched, uint32_t triangle_count,
                        const nxg_vec3 *__restrict__ guide_roots, const nxg_vec3 *__restrict__ guide_normals,
                        uint32_t guide_count, uint32_t clusters, uint32_t keep, uint32_t *stencil) {
     __shared__ __align__(16) GuideTile tile;
     chain_wait();
     chain_start();  // from here on the scratch is complete, which the next kernel relies on
     const uint32_t ti = blockIdx.x * kStencilThreads + threadIdx.x;
-    TriangleSearch t;
-    begin_triangle(t, ti, positions, vertex_count, triangles, searched);
     const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(searched) * kSlots);
-    const bool wild = scratch[clusters * (kClusterWords + kClusterBoxes)].x != 0.0f || wild_triangle(t);
-    if (__syncthreads_or(wild)) {
+    const bool all = __ldcg(&scratch[clusters * (kClusterWords + kClusterBoxes)].x) != 0.0f;
+    if (!all && blockIdx.x * kStencilThreads >= searched) { return; }
+    TriangleSearch t;
+    begin_triangle(t, ti, positions, vertex_count, triangles, all ? triangle_count - 1u : searched);
+    const WarpBox bounds = warp_box(t);
+    if (__syncthreads_or(all || wild_triangle(t)) || scattered_triangles(bounds, scratch, clusters)) {
         search_all(t, tile, guide_roots, guide_normals, guide_count);
     } else {
-        search_clusters(t, scratch, clusters, guide_normals);
+        search_clusters(t, bounds, scratch, clusters, guide_normals);
     }
     end_triangle(t, ti, keep, stencil);
 }
@@ -664,8 +777,10 @@ stencil_cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_c
 // The rows the scratch is in: one thread-block cluster, whose CTAs copy the
 // scratch to shared memory before any of them writes a row.  It starts once
 // every CTA of stencil_cluster_kernel has seen the scratch complete, searches
-// beside that kernel's end and writes after it.
-__global__ void __launch_bounds__(1024)
+// beside that kernel's end and writes after it.  Where every triangle takes all
+// pairs (the last row, which nobody else writes, says so) it has that row
+// alone, and one CTA shares its guides out to its threads unless one is wild.
+__global__ void __launch_bounds__(kTailMaxThreads)
 stencil_tail_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
                     const nxg_uint3 *__restrict__ triangles, uint32_t searched, uint32_t triangle_count,
                     const nxg_vec3 *__restrict__ guide_roots, const nxg_vec3 *__restrict__ guide_normals,
@@ -678,14 +793,28 @@ stencil_tail_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_coun
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const float4 flags = copy[clusters * (kClusterWords + kClusterBoxes)];
+    const bool all = flags.x != 0.0f;
     const uint32_t ti = searched + blockIdx.x * blockDim.x + threadIdx.x;
     TriangleSearch t;
+    if (all && flags.y == 0.0f) {
+        begin_triangle(t, triangle_count - 1u, positions, vertex_count, triangles, triangle_count);
+        if (!wild_triangle(t)) {  // the same triangle in every thread
+            if (blockIdx.x != 0u) { return; }
+            if (t.live) { share_triangle(t, guide_roots, guide_normals, guide_count); }
+            chain_wait();
+            if (threadIdx.x == 0u) { end_triangle(t, triangle_count - 1u, keep, stencil); }
+            return;
+        }
+    }
     begin_triangle(t, ti, positions, vertex_count, triangles, triangle_count);
-    const bool wild = copy[clusters * (kClusterWords + kClusterBoxes)].x != 0.0f || wild_triangle(t);
-    if (__syncthreads_or(wild)) {
+    if (all && ti != triangle_count - 1u) { t.live = t.invalid = false; }
+    const WarpBox bounds = warp_box(t);
+    if (__syncthreads_or(all || wild_triangle(t))) {
+        if (!__syncthreads_or(t.live || t.invalid)) { return; }
         search_all(t, tile, guide_roots, guide_normals, guide_count);
     } else {
-        search_clusters(t, copy, clusters, guide_normals);
+        search_clusters(t, bounds, copy, clusters, guide_normals);
     }
     chain_wait();
     end_triangle(t, ti, keep, stencil);
@@ -722,6 +851,8 @@ uint32_t slots_kept(uint32_t guide_count, uint32_t stencil_slots) {
     return stencil_slots == 0u || stencil_slots > count ? count : stencil_slots;
 }
 
+static_assert((cluster_scratch_rows(kMaxClusters) + kTailCtas - 1u) / kTailCtas <= kTailMaxThreads, "one CTA cluster");
+
 cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, const nxg_uint3 *triangles,
                          uint32_t triangle_count, const nxg_vec3 *guide_roots, const nxg_vec3 *guide_normals,
                          uint32_t guide_count, uint32_t stencil_slots, uint32_t *stencil, cudaStream_t stream) {
@@ -742,7 +873,8 @@ cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, co
     }
     const uint32_t searched = triangle_count - rows;
     const size_t copy = sizeof(float4) * cluster_scratch_words(clusters);
-    const uint32_t tail_threads = ((rows + kTailCtas - 1u) / kTailCtas + 31u) / 32u * 32u;
+    uint32_t tail_threads = ((rows + kTailCtas - 1u) / kTailCtas + 31u) / 32u * 32u;
+    tail_threads = tail_threads < 256u ? 256u : tail_threads;  // (for share_triangle)
     // The largest copy, whatever this call's: the limit is the process's.
     cudaError_t e = cudaFuncSetAttribute(stencil_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(sizeof(float4) * cluster_scratch_words(kMaxClusters)));
@@ -759,15 +891,15 @@ cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, co
     config.gridDim = dim3(1);
     config.blockDim = dim3(1024);
     config.dynamicSmemBytes = 0u;
-    e = cudaLaunchKernelEx(&config, cluster_kernel, guide_roots, guide_normals, guide_count, clusters,
+    e = cudaLaunchKernelEx(&config, cluster_kernel, positions, vertex_count, triangles, searched, guide_roots, guide_normals, guide_count, clusters,
                            reinterpret_cast<float4 *>(stencil + static_cast<size_t>(searched) * kSlots));
     if (e != cudaSuccess) { return e; }
     config.numAttrs = 1u;
-    config.gridDim = dim3((searched + kStencilThreads - 1u) / kStencilThreads);
+    config.gridDim = dim3((triangle_count + kStencilThreads - 1u) / kStencilThreads);
     config.blockDim = dim3(kStencilThreads);
     config.dynamicSmemBytes = 0u;
-    e = cudaLaunchKernelEx(&config, stencil_cluster_kernel, positions, vertex_count, triangles, searched, guide_roots,
-                           guide_normals, guide_count, clusters, keep, stencil);
+    e = cudaLaunchKernelEx(&config, stencil_cluster_kernel, positions, vertex_count, triangles, searched, triangle_count,
+                           guide_roots, guide_normals, guide_count, clusters, keep, stencil);
     if (e != cudaSuccess) { return e; }
     config.numAttrs = 2u;
     config.gridDim = dim3(kTailCtas);
