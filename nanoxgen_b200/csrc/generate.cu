@@ -795,7 +795,10 @@ uint32_t launch_order(const nxg_device_asset_desc &asset, uint32_t seed, uint32_
     const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((count + threads - 1u) / threads,
                                                                       static_cast<uint64_t>(sms) * 4u));
     const size_t shm = bins <= dev::kPrivateBins ? bins * 4u : 0u;
-    if ((status = launch_chained(cleared, dev::strand_keys_kernel, blocks, threads, shm, stream, a, seed, first,
+    // An ordinary launch: chained to the guide offsets before it, both kernels
+    // share the SMs to neither's gain (whole calls of 1,000,000 x 32 without noise
+    // 238 us chained, 231 not; with noise 577, 569).
+    if ((status = launch_chained(false, dev::strand_keys_kernel, blocks, threads, shm, stream, a, seed, first,
                                  count, keys, hist, bins)) ||
         (status = launch_chained(true, dev::exclusive_scan_kernel, 1u, 1024u, 0u, stream, hist, bins))) {
         return status;
