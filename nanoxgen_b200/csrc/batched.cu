@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(256) batched_prepare_kernel(const __grid_const
 // the lane walk's region per warp.
 constexpr uint32_t kBatchMaxCvs = 128u;
 __host__ __device__ constexpr size_t batch_smem_bytes(int cls, bool classic, uint32_t warps) {
-    return walk_head_bytes(cls == 0, kBatchMaxCvs, warps) + walk_warp_bytes(cls == 0, classic) * warps;
+    return walk_head_bytes(cls == 0, kBatchMaxCvs, warps, kWalkChunk) +
+           walk_warp_bytes(cls == 0, classic, kWalkChunk) * warps;
 }
 // 32-strand batches per warp in one work item of each class: four for the
 // noisy class (fewer CTA-wide claims between long batches), one for the
@@ -268,10 +269,10 @@ __global__ void __launch_bounds__(CLS == 1 ? 256 : 32 * kWalkNoiseWarps, CLS == 
     // launch's CTAs leave SMs free; it waits at its end only.
     if (b.first_class == static_cast<uint32_t>(CLS)) { chain_wait(); }
     chain_start();
-    float *tvals = reinterpret_cast<float *>(smem + (CLS == 0 ? kTableFloat4 << walk_table_copies(warps) : 0));
+    float *tvals = reinterpret_cast<float *>(smem + (CLS == 0 ? kTableFloat4 << walk_table_copies(warps, kWalkChunk) : 0));
     float *rvals = tvals + walk_padded(kBatchMaxCvs);
     unsigned char *mine = reinterpret_cast<unsigned char *>(rvals + walk_padded(kBatchMaxCvs)) +
-                          walk_warp_bytes(CLS == 0, CLASSIC) * warp;
+                          walk_warp_bytes(CLS == 0, CLASSIC, kWalkChunk) * warp;
     const uint32_t total = b.total_items[CLS];
     const int first = static_cast<int>(b.desc_first[CLS]);
     const int last = static_cast<int>(b.desc_end[CLS]) - 1;

@@ -162,7 +162,7 @@ uint32_t nxg_generate_packed_classic(const nxg_device_asset_desc *asset, const n
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
                                 workspace_bytes, s, nullptr, classic,
-                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u, false),
+                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u, false, true),
                                 false);
 }
 

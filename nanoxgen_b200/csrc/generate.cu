@@ -105,27 +105,27 @@ __global__ void generate_kernel(LaunchArgs g, const float4 *offsets) {
 // 1,037, four 1,135).  The arguments stay in the constant
 // bank (__grid_constant__): an out-of-line call taking them by reference
 // otherwise copies them to every thread's stack first.
-template <bool NOISE, bool CLASSIC>
-__global__ void __launch_bounds__(NOISE ? 32 * kWalkNoiseWarps : 256, NOISE ? 1 : 3)
+template <bool NOISE, bool CLASSIC, int CHUNK = kWalkChunk>
+__global__ void __launch_bounds__(NOISE ? 32 * walk_noise_warps(CHUNK) : 256, NOISE ? 1 : 3)
     generate_walk_kernel(const __grid_constant__ LaunchArgs g, const float4 *offsets) {
     extern __shared__ float4 smem[];
     const uint32_t P = g.p.cvs_per_strand;
     const uint32_t padded = walk_padded(P);
-    float *tvals = reinterpret_cast<float *>(smem + (NOISE ? kTableFloat4 << walk_table_copies(blockDim.x >> 5) : 0));
+    float *tvals = reinterpret_cast<float *>(smem + (NOISE ? kTableFloat4 << walk_table_copies(blockDim.x >> 5, CHUNK) : 0));
     float *rvals = tvals + padded;
-    walk_fill_head<NOISE>(g, smem, tvals, rvals);  // of the asset and the arguments alone
+    walk_fill_head<NOISE, CHUNK>(g, smem, tvals, rvals);  // of the asset and the arguments alone
     __syncthreads();
     chain_start();
     chain_wait();
     const int lane = threadIdx.x & 31;
     const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    unsigned char *mine = reinterpret_cast<unsigned char *>(rvals + padded) + walk_warp_bytes(NOISE, CLASSIC) * warp;
+    unsigned char *mine = reinterpret_cast<unsigned char *>(rvals + padded) + walk_warp_bytes(NOISE, CLASSIC, CHUNK) * warp;
     const uint32_t begin = static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x) * g.count / gridDim.x);
     const uint32_t end = static_cast<uint32_t>(static_cast<uint64_t>(blockIdx.x + 1u) * g.count / gridDim.x);
     for (uint32_t batch = begin + warp * g.batch; batch < end; batch += warps * g.batch) {
         const int in_batch = static_cast<int>(min(g.batch, end - batch));
         if constexpr (NOISE) {
-            walk_noise_batch<CLASSIC>(g, offsets, mine, smem, tvals, rvals, lane, batch, in_batch);
+            walk_noise_batch<CLASSIC, CHUNK>(g, offsets, mine, smem, tvals, rvals, lane, batch, in_batch);
         } else {
             walk_plain_batch<CLASSIC>(g, offsets, mine, tvals, rvals, lane, batch, in_batch);
         }
@@ -833,21 +833,34 @@ namespace {
 // 100,000 x 32 71.5 us against 78.5 without it, 1,000,000 x 24 and 200 guides
 // 517 / 537; without noise 100,000 x 32 31.8 / 36.8, 500,000 x 12 87.5 / 110.5,
 // 2,000,000 x 24 378 / 414.
-bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, uint32_t samples) {
+// Whole stages leave the rows little of L1, so there it pays earlier: Classic
+// scalars on 170,000 x 24 109.1 / 117.2 us, on 130,000 x 24 100.5 / 102.0, of 700
+// guides 98.3 / 96.3.
+bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, bool whole, uint32_t samples) {
     const uint64_t points = uint64_t{count} * P * samples;
     if (uint64_t{guide_count} * P * 16u <= (uint64_t{128} << 10)) { return false; }
-    return noise ? points >= 7000000u : points >= 24000000u && count <= 1700000u;
+    return noise ? points >= (whole ? 4000000u : 7000000u) : points >= 24000000u && count <= 1700000u;
+}
+
+// CVs of a strand that the noisy walk stages at a time (walk.cuh).
+int noise_chunk(uint32_t P, bool classic, const nxg_generation_params &params) {
+    const bool rewritten = classic || params.noise_preserve_length > 0.001f;
+    if (!rewritten || P <= static_cast<uint32_t>(dev::kWalkChunk) || P > static_cast<uint32_t>(dev::kWalkWholeCvs)) {
+        return dev::kWalkChunk;
+    }
+    return P <= 24u ? 24 : 32;
 }
 
 } // namespace
 
 LaunchForm launch_form(uint32_t guide_count, const nxg_generation_params &params, uint32_t count, uint32_t samples,
-                       bool prepared) {
+                       bool prepared, bool classic) {
     const uint32_t P = params.cvs_per_strand;
     const bool noise = resolve_params(params, 1.0f).noise != 0u;
     LaunchForm form;
     form.tile = registered_tile(P, noise);
-    form.ordered = prepared || lane_groups(form.tile) || wants_order(guide_count, count, P, noise, samples);
+    form.ordered = prepared || lane_groups(form.tile) ||
+                   wants_order(guide_count, count, P, noise, noise_chunk(P, classic, params) != dev::kWalkChunk, samples);
     return form;
 }
 
@@ -952,7 +965,9 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
                     : uint32_t{NXG_ERROR_NONE};
     };
     if (walk) {
-        uint32_t warps = noise ? dev::kWalkNoiseWarps : 8u;
+        const int chunk = noise_chunk(P, classic_scalars, params);
+        const uint32_t full = noise ? dev::walk_noise_warps(chunk) : 8u;
+        uint32_t warps = full;
         if (packed) {  // a registered CTA size is a bound
             const uint32_t tile_warps = (packed >> 16) & 0xffu;
             warps = std::min(warps, tile_warps ? tile_warps : (config.block_size + 31u) / 32u);
@@ -966,19 +981,20 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
             // (20,000 strands x 160 CVs with noise 159 -> 113 us, x 100 CVs
             // without 72 -> 31 us), and the last batches of a larger one are
             // not nearly empty.  Below a warp per SM the CTAs shrink too.
-            const uint64_t slots = static_cast<uint64_t>(sms) * (noise ? dev::kWalkNoiseWarps : 24u);
+            const uint64_t slots = static_cast<uint64_t>(sms) * (noise ? full : 24u);
             const uint64_t rounds = (count + slots * 32u - 1u) / (slots * 32u);
             const uint64_t share = (count + slots * rounds - 1u) / (slots * rounds);
             g.batch = static_cast<uint32_t>(std::clamp<uint64_t>((share + 3u) / 4u * 4u, noise ? 8u : 4u, 32u));
             const uint64_t needed = (uint64_t{count} + g.batch - 1u) / g.batch;
             warps = static_cast<uint32_t>(std::min<uint64_t>(warps, (needed + sms - 1u) / sms));
         }
-        const auto fn = noise ? (classic_scalars ? dev::generate_walk_kernel<true, true>
-                                                 : dev::generate_walk_kernel<true, false>)
-                              : (classic_scalars ? dev::generate_walk_kernel<false, true>
-                                                 : dev::generate_walk_kernel<false, false>);
+        const auto pick = [&](auto plain, auto classic) { return classic_scalars ? classic : plain; };
+        const auto fn = !noise ? pick(dev::generate_walk_kernel<false, false>, dev::generate_walk_kernel<false, true>)
+            : chunk == 32 ? pick(dev::generate_walk_kernel<true, false, 32>, dev::generate_walk_kernel<true, true, 32>)
+            : chunk == 24 ? pick(dev::generate_walk_kernel<true, false, 24>, dev::generate_walk_kernel<true, true, 24>)
+                          : pick(dev::generate_walk_kernel<true, false>, dev::generate_walk_kernel<true, true>);
         return launch(fn, warps * 32u, g.batch, [&](uint32_t w) {
-            return dev::walk_head_bytes(noise, P, w) + dev::walk_warp_bytes(noise, classic_scalars) * w;
+            return dev::walk_head_bytes(noise, P, w, chunk) + dev::walk_warp_bytes(noise, classic_scalars, chunk) * w;
         });
     }
     const int lanes = static_cast<int>(packed & 0xffu), ppt = static_cast<int>((packed >> 8) & 0xffu);
@@ -1068,7 +1084,7 @@ uint32_t nxg_generate_packed_range(const nxg_device_asset_desc *asset, const nxg
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
                                 workspace_bytes, s, nullptr, nullptr,
-                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u, false), false);
+                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u, false, false), false);
 }
 
 uint32_t nxg_prepare_strand_order(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
@@ -1112,7 +1128,7 @@ uint32_t nxg_generate_packed_ordered(const nxg_device_asset_desc *asset, const n
     return nxg::launch_generate(*asset, deformed ? *deformed : none, *params, *output,
                                 config ? *config : default_config, first_strand, strand_count, workspace,
                                 workspace_bytes, static_cast<cudaStream_t>(stream), nullptr, nullptr,
-                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u, true), true);
+                                nxg::launch_form(asset->header.guide_count, *params, strand_count, 1u, true, false), true);
 }
 
 uint32_t nxg_query_strand_states(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,
@@ -1330,7 +1346,7 @@ extern "C" uint32_t nxg_generate_motion_packed(const nxg_device_asset_desc *asse
     const auto s = static_cast<cudaStream_t>(stream);
     nxg::set_last_cuda_error(0);
     const nxg::LaunchForm form =
-        nxg::launch_form(asset->header.guide_count, *params, params->strand_count, sample_count, false);
+        nxg::launch_form(asset->header.guide_count, *params, params->strand_count, sample_count, false, false);
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, outputs[i], cfg, 0u,
                                      params->strand_count, workspace, workspace_bytes, s, nullptr, nullptr, form,
@@ -1358,7 +1374,7 @@ extern "C" uint32_t nxg_generate_motion(const nxg_device_asset_desc *asset, cons
     nxg_packed_output_desc none{};
     none.radius_scale = 1.0f;
     const nxg::LaunchForm form =
-        nxg::launch_form(asset->header.guide_count, *params, params->strand_count, sample_count, false);
+        nxg::launch_form(asset->header.guide_count, *params, params->strand_count, sample_count, false, false);
     for (uint32_t i = 0; i < sample_count && !error; ++i) {
         float *dst = reinterpret_cast<float *>(output->points) + per_sample * i;
         error = nxg::launch_generate(*asset, samples[i].deformation, *params, none, cfg, 0u, params->strand_count,

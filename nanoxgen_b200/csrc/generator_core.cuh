@@ -652,9 +652,9 @@ struct LaunchForm {
     bool ordered;
 };
 // `samples`: frames that share one strand order; `prepared`: the caller has
-// prepared it.
+// prepared it; `classic`: per-root scalars are applied.
 LaunchForm launch_form(uint32_t guide_count, const nxg_generation_params &params, uint32_t count, uint32_t samples,
-                       bool prepared);
+                       bool prepared, bool classic);
 // `order_ready`: the workspace holds the strand order of this range.
 uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_desc &deformed,
                          const nxg_generation_params &params, const nxg_packed_output_desc &output,

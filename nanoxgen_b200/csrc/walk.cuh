@@ -19,9 +19,11 @@
 //                            needed; the noise comes from a window of lattice
 //                            columns that moves along the strand;
 //   store  (8 lanes/strand)  the chunk's float4s as coalesced streaming
-//                            stores; preserveLength on strands of more than
-//                            one chunk and Classic scalars are applied to the
-//                            written points afterwards, from L2.
+//                            stores; preserveLength and Classic scalars are
+//                            applied to the stage before it, or, on strands of
+//                            more than 32 CVs (in the batched launch more than
+//                            one chunk), to the written points afterwards,
+//                            from L2.
 //
 // What bounds the noisy walk: of 1,000,000 strands x 32 CVs, separately built
 // variants put about 120 us each on the walk itself (near the issue rate),
@@ -37,7 +39,8 @@
 // on lane groups with scans, 228 us; 20,011 x 160: 1,241 us on one thread per
 // strand, 97 us (121 before the equal batches of small calls).
 //
-// Stage rows are 49 words apart and a CV takes 3 words; both strides are odd,
+// Stage rows are 49 words apart (73 and 97 where strands are staged whole) and a
+// CV takes 3 words; both strides are odd,
 // so a warp reading column c of 32 rows (frame step) and a warp reading one
 // row are free of shared-memory bank conflicts, and the eight-lane base and
 // store steps (four strands of eight CVs per access) meet at most two lanes
@@ -50,7 +53,15 @@ namespace nxg {
 namespace dev {
 
 constexpr int kWalkChunk = 16;                     // CVs staged at a time
-constexpr int kWalkRowFloats = 3 * kWalkChunk + 1;  // a row holds x, y, z per CV (49 words: an odd stride)
+// Strands of up to 32 CVs whose points are rewritten once the whole strand is
+// known (preserveLength, Classic scalars) are staged whole instead, CHUNK 24 or
+// 32, and rewritten in the stage: through L2 the second pass cost more than
+// the chunks gain.  With noise and Classic scalars 500,000 x 24 331 -> 277 us,
+// x 32 370 -> 341; preserveLength 500,000 x 17 325 -> 250, x 24 320 -> 268, x 32
+// 357 -> 328.
+constexpr int kWalkWholeCvs = 32;
+// Words of a stage row: x, y, z per CV, and the strand's radius override (an odd stride).
+__host__ __device__ constexpr int walk_row(int chunk) { return 3 * chunk + 1; }
 // Noise lattice columns per axis and strand.  Five cover four lattice cells; a
 // walk crosses a cell every five or six CVs at the sizes grooms use, so a
 // strand refills its window about once (four columns: 533 us against 526 on
@@ -67,26 +78,33 @@ constexpr int kWalkNoiseWarps = 12;                // warps of a full noise CTA
 // with one copy, eight random entries in eight bank groups, 11.6): 1,000,000
 // strands x 32 CVs 574 -> 551 us.  A CTA of a few warps runs too few strands
 // to pay for the copies (2,000 strands x 16: 14.2 us with one, 15.5 with eight).
-__host__ __device__ constexpr uint32_t walk_table_copies(uint32_t warps) { return warps >= 8u ? 3u : 0u; }
+// A CTA of whole 32-CV stages has room for four.
+__host__ __device__ constexpr uint32_t walk_table_copies(uint32_t warps, int chunk) {
+    return warps < 8u ? 0u : (chunk > 24 ? 2u : 3u);
+}
+// Warps of a full CTA: what shared memory holds.
+__host__ __device__ constexpr uint32_t walk_noise_warps(int chunk) { return chunk > 24 ? 11u : kWalkNoiseWarps; }
 
 // Shared-memory bytes per warp.  With noise: stage | lattice window | records
 // | output words.  Without (the base step writes the output directly):
 // records | output words.
-constexpr size_t kWalkStageBytes = sizeof(float) * 32u * kWalkRowFloats;
+__host__ __device__ constexpr size_t walk_stage_bytes(int chunk) {
+    return sizeof(float) * 32u * static_cast<size_t>(walk_row(chunk));
+}
 constexpr size_t kWalkLatticeBytes = sizeof(float2) * 3u * kWalkWindow * 32u;
 constexpr size_t kWalkRecordBytes = sizeof(float4) * kWalkRecords * 32u;
 constexpr size_t kWalkClassicRecordBytes = sizeof(float4) * kWalkClassicRecords * 32u;
 constexpr size_t kWalkLocalBytes = sizeof(uint32_t) * 32u;
-__host__ __device__ constexpr size_t walk_warp_bytes(bool noise, bool classic) {
-    return (noise ? kWalkStageBytes + kWalkLatticeBytes + kWalkRecordBytes
+__host__ __device__ constexpr size_t walk_warp_bytes(bool noise, bool classic, int chunk) {
+    return (noise ? walk_stage_bytes(chunk) + kWalkLatticeBytes + kWalkRecordBytes
                   : (classic ? kWalkClassicRecordBytes : kWalkRecordBytes)) +
            kWalkLocalBytes;
 }
 // Per CTA, before the warps: gradient table (noise) | t values | radii, each
 // of P values and padding to a multiple of four (walk_pair reads t in pairs).
 __host__ __device__ constexpr uint32_t walk_padded(uint32_t P) { return (P + 4u) & ~3u; }
-__host__ __device__ constexpr size_t walk_head_bytes(bool noise, uint32_t P, uint32_t warps) {
-    return (noise ? sizeof(float4) * (kTableFloat4 << walk_table_copies(warps)) : 0u) +
+__host__ __device__ constexpr size_t walk_head_bytes(bool noise, uint32_t P, uint32_t warps, int chunk) {
+    return (noise ? sizeof(float4) * (kTableFloat4 << walk_table_copies(warps, chunk)) : 0u) +
            2u * sizeof(float) * walk_padded(P);
 }
 // Longest strand the walk takes (its t values and radii are in shared memory).
@@ -606,11 +624,12 @@ __device__ __forceinline__ void walk_base_direct(const LaunchArgs &g, float4 *re
 // and for an odd n slot n too; past the strand's end they repeat the tip, a
 // zero segment to the walk.  Lanes as in walk_base_direct.  Every lane of the
 // warp calls it.
+template <int CHUNK>
 __device__ __forceinline__ void walk_base_chunk(const LaunchArgs &g, const float4 *records, float *stage,
                                                 const float *tvals, const float4 *offsets, int lane, int in_batch,
                                                 int a, int n, int P) {
-    constexpr int kPerLane = kWalkChunk / 8;
-    constexpr int kPasses = 2;
+    constexpr int kPerLane = CHUNK / 8;
+    constexpr int kPasses = CHUNK == kWalkChunk ? 2 : 1;  // at most sixteen loads in flight
     constexpr uint32_t kTrip = 4u;
     const int c = lane & 7;
     const float ls = g.p.length_scale;
@@ -676,7 +695,7 @@ __device__ __forceinline__ void walk_base_chunk(const LaunchArgs &g, const float
             if (s >= in_batch) { continue; }
             const float4 head = records[4 * 32 + s];
             const float4 tail = records[5 * 32 + s];
-            float *row = stage + s * kWalkRowFloats;
+            float *row = stage + s * walk_row(CHUNK);
             const F3 root = {head.x, head.y, head.z}, normal = {tail.x, tail.y, tail.z};
 #pragma unroll
             for (int m = 0; m < kPerLane; ++m) {
@@ -973,10 +992,10 @@ __device__ __forceinline__ void walk_pair(WalkCursor &s, F3 n0, F3 n1, f32x2 t, 
 // Fills a CTA's head (every thread calls it; a barrier must follow): the
 // gradient table with noise, t = cv / (P - 1) (generate.h:295-298) and the
 // radii, the padding after the tip repeating it.
-template <bool NOISE>
+template <bool NOISE, int CHUNK = kWalkChunk>
 __device__ __forceinline__ void walk_fill_head(const LaunchArgs &g, float4 *table, float *tvals, float *rvals) {
     if constexpr (NOISE) {
-        const uint32_t copies = walk_table_copies(blockDim.x >> 5);
+        const uint32_t copies = walk_table_copies(blockDim.x >> 5, CHUNK);
         for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(kTableFloat4) << copies; i += blockDim.x) {
             const float *gradient = g.a.gradients + 3u * (i >> copies);
             table[i] = make_float4(__ldg(gradient), __ldg(gradient + 1), __ldg(gradient + 2), 0.0f);
@@ -999,14 +1018,15 @@ __device__ __forceinline__ float walk_preserve_scale(const ParamArgs &p, float o
 
 // Length of this lane's base curve (generate.h:420-433), chunk by chunk.
 // Every lane of the warp calls it.
+template <int CHUNK>
 static __device__ __noinline__ float walk_base_length(const LaunchArgs &g, const float4 *records, float *stage,
                                                   const float *tvals, const float4 *offsets, int lane, int in_batch,
                                                   int P, F3 first) {
-    const float *row = stage + lane * kWalkRowFloats;
+    const float *row = stage + lane * walk_row(CHUNK);
     float length = 0.0f;
-    for (int a = 0; a < P - 1; a += kWalkChunk) {
-        const int n = min(kWalkChunk, P - 1 - a);
-        walk_base_chunk(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+    for (int a = 0; a < P - 1; a += CHUNK) {
+        const int n = min(CHUNK, P - 1 - a);
+        walk_base_chunk<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
         __syncwarp();
         for (int i = 0; i < n; ++i) {
             const F3 next = stage_get(row, i);
@@ -1021,11 +1041,13 @@ static __device__ __noinline__ float walk_base_length(const LaunchArgs &g, const
 
 // Store step of one chunk, eight lanes per strand as in walk_base_chunk: each
 // store instruction writes four strands' runs of eight consecutive float4s.
+// RADII: a strand's last stage word overrides its radius unless it is negative.
 // Every lane of the warp calls it.
+template <int CHUNK, bool RADII>
 __device__ __forceinline__ void walk_store_chunk(const LaunchArgs &g, const float *stage, const uint32_t *locals,
                                                  const float *rvals, int lane, int in_batch, int a, int n, int P,
                                                  bool again) {
-    constexpr int kPerLane = kWalkChunk / 8;
+    constexpr int kPerLane = CHUNK / 8;
     const int c = lane & 7;
     float rv[kPerLane];
 #pragma unroll
@@ -1033,12 +1055,15 @@ __device__ __forceinline__ void walk_store_chunk(const LaunchArgs &g, const floa
     for (int first = 0; first < in_batch; first += 4) {
         const int s = first + (lane >> 3);  // at most 31
         const uint32_t word = s < in_batch ? locals[s] : 0x80000000u;
-        const float *row = stage + s * kWalkRowFloats;
+        const float *row = stage + s * walk_row(CHUNK);
+        float radius = -1.0f;
+        if constexpr (RADII) { radius = row[3 * CHUNK]; }
 #pragma unroll
         for (int m = 0; m < kPerLane; ++m) {
             if (c + 8 * m < n) {
                 const F3 q = stage_get(row, c + 8 * m);
-                walk_emit(g, word, P, a + c + 8 * m, make_float4(q.x, q.y, q.z, rv[m]), again);
+                walk_emit(g, word, P, a + c + 8 * m, make_float4(q.x, q.y, q.z, RADII && !(radius < 0.0f) ? radius : rv[m]),
+                          again);
             }
         }
     }
@@ -1144,19 +1169,76 @@ __device__ __forceinline__ void walk_classic_finish(const LaunchArgs &g, const u
     walk_rescale<true>(g, locals, centre, kept, front, scale, radius, lane, in_batch, P);
 }
 
+// The sampled spline's length of a staged strand, out of line: it is rare.
+static __device__ __noinline__ float walk_stage_spline_length(const float *row, int P) {
+    __builtin_assume(__isShared(row));
+    return classic_spline_length_by([row](int c) { return stage_get(row, c); }, P);
+}
+
+// This lane's staged strand, all its points there: its preserveLength scale
+// `keep` about the root `centre` and, CLASSIC, the rules of emit_strand (scale
+// about the first point, width override into the row's last word, the drop
+// rule with its chord bound and sampled-spline measure; a dropped strand's
+// point count becomes 0).
+template <bool CLASSIC, int CHUNK>
+__device__ __forceinline__ void walk_finish_stage(const LaunchArgs &g, float *row, uint32_t word, F3 centre, float keep,
+                                                  int P) {
+    const auto point = [=](int c) {
+        const F3 q = stage_get(row, c);
+        return keep != 1.0f ? walk_scaled(centre, q, keep) : q;
+    };
+    F3 front = {0.0f, 0.0f, 0.0f};
+    float scale = 1.0f;
+    bool length = false;
+    if constexpr (CLASSIC) {
+        const ParamArgs &p = g.p;
+        float radius = -1.0f;
+        if (!(word >> 31)) {
+            const float2 sc = __ldg(g.scalars + word);
+            front = point(0);
+            length = g.classic_length != 0u;
+            scale = length ? sc.x : 1.0f;
+            const float raw_width = g.classic_width ? sc.y
+                : (p.radius_scale > 0.0f ? __fdiv_rn(__fmul_rn(2.0f, strand_radius(p, 0.0f)), p.radius_scale) : 0.0f);
+            bool stays = !(raw_width < 1.0e-4f);
+            const F3 chord = point(P - 1) - front;
+            if (stays && !(sqrtf(dot(chord, chord)) * scale > 1.01e-4f)) {
+                if (keep != 1.0f) {
+                    for (int c = 0; c < P; ++c) { stage_put(row, c, point(c)); }
+                    keep = 1.0f;
+                }
+                stays = !(__fmul_rn(walk_stage_spline_length(row, P), scale) < 1.0e-4f);
+            }
+            if (g.classic_width) {
+                radius = __fmul_rn(__fmul_rn(0.5f, raw_width < 0.0f ? 0.0f : raw_width), p.radius_scale);
+            }
+            if (!stays && g.point_counts != nullptr) { g.point_counts[word] = 0u; }
+        }
+        row[3 * CHUNK] = radius;
+    }
+    if (keep == 1.0f && !length) { return; }
+    for (int c = 0; c < P; ++c) {
+        F3 v = stage_get(row, c);
+        if (keep != 1.0f) { v = walk_scaled(centre, v, keep); }
+        if (length) { v = xadd(front, xmul(xsub(v, front), scale)); }
+        stage_put(row, c, v);
+    }
+}
+
 // One batch of a warp with noise: strands [batch, batch + in_batch) of the
 // order through setup, base, frame and store.  Every lane of the warp calls
 // it; lanes past in_batch set up its first strand again and are ignored.
-template <bool CLASSIC>
+template <bool CLASSIC, int CHUNK = kWalkChunk>
 __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const float4 *offsets, unsigned char *mine,
                                                  const float4 *table, const float *tvals, const float *rvals,
                                                  int lane, uint32_t batch, int in_batch) {
     float *stage = reinterpret_cast<float *>(mine);
-    float2 *lattice = reinterpret_cast<float2 *>(mine + kWalkStageBytes) + lane;
-    const uint32_t copies = walk_table_copies(blockDim.x >> 5);
+    float2 *lattice = reinterpret_cast<float2 *>(mine + walk_stage_bytes(CHUNK)) + lane;
+    const uint32_t copies = walk_table_copies(blockDim.x >> 5, CHUNK);
     table += static_cast<uint32_t>(lane) & ((1u << copies) - 1u);
-    float4 *records = reinterpret_cast<float4 *>(mine + kWalkStageBytes + kWalkLatticeBytes);
-    uint32_t *locals = reinterpret_cast<uint32_t *>(mine + kWalkStageBytes + kWalkLatticeBytes + kWalkRecordBytes);
+    float4 *records = reinterpret_cast<float4 *>(mine + walk_stage_bytes(CHUNK) + kWalkLatticeBytes);
+    uint32_t *locals =
+        reinterpret_cast<uint32_t *>(mine + walk_stage_bytes(CHUNK) + kWalkLatticeBytes + kWalkRecordBytes);
     const ParamArgs &p = g.p;
     const int P = static_cast<int>(p.cvs_per_strand);
     const bool counts = lane < in_batch;
@@ -1168,16 +1250,16 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
     float f_eff = p.noise_frequency;
     const float mscale = 0.5f * (p.noise_mask * p.noise_amplitude);
     const bool preserve = p.noise_preserve_length > 0.001f;
-    const bool one_chunk = P <= kWalkChunk;
-    const bool again = CLASSIC || (preserve && !one_chunk);
-    float *row = stage + lane * kWalkRowFloats;
+    const bool one_chunk = CHUNK != kWalkChunk || P <= CHUNK;  // staged whole
+    const bool again = (CLASSIC || preserve) && !one_chunk;
+    float *row = stage + lane * walk_row(CHUNK);
     WalkWindow window;
     window.limit = -1.0f;
     F3 previous = s.cur;
     float noisy = 0.0f;
-    for (int a = 0; a < P; a += kWalkChunk) {
-        const int n = min(kWalkChunk, P - a);
-        walk_base_chunk(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+    for (int a = 0; a < P; a += CHUNK) {
+        const int n = min(CHUNK, P - a);
+        walk_base_chunk<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
         __syncwarp();
         if (a == 0) {
             // The effective frequency max(0.5 / length, frequency)
@@ -1193,8 +1275,8 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
                 !__all_sync(kFull, sure(walk_base_point(records, lane, P - 1, tvals[P - 1], p.length_scale,
                                                         offsets)))) {
                 f_eff = walk_effective_frequency(
-                    p, walk_base_length(g, records, stage, tvals, offsets, lane, in_batch, P, s.cur));
-                walk_base_chunk(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+                    p, walk_base_length<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, P, s.cur));
+                walk_base_chunk<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
                 __syncwarp();
             }
         }
@@ -1203,7 +1285,7 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
         for (int i = 0; i < n; i += 2) {
             // The next pair is requested before this one is replaced (past
             // the chunk: slots that are not used).
-            const int ahead = min(i + 2, kWalkChunk - 2);
+            const int ahead = min(i + 2, CHUNK - 2);
             const F3 ahead0 = stage_get(row, ahead), ahead1 = stage_get(row, ahead + 1);
             F3 qa, qb;
             walk_pair(s, n0, n1, *reinterpret_cast<const f32x2 *>(tvals + a + i), mscale, f_eff, wr.domain, counts,
@@ -1219,26 +1301,30 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
             n0 = ahead0;
             n1 = ahead1;
         }
-        if (preserve && one_chunk) {
-            const float scale = walk_preserve_scale(p, s.arc, noisy);
-            if (scale != 1.0f) {
-                for (int c = 0; c < P; ++c) {
-                    stage_put(row, c, wr.position + (stage_get(row, c) - wr.position) * scale);
-                }
-            }
+        if (one_chunk && (CLASSIC || preserve)) {
+            walk_finish_stage<CLASSIC, CHUNK>(g, row, counts ? locals[lane] : 0x80000000u, wr.position,
+                                              preserve ? walk_preserve_scale(p, s.arc, noisy) : 1.0f, P);
         }
         __syncwarp();
-        walk_store_chunk(g, stage, locals, rvals, lane, in_batch, a, n, P, again);
+        if (CLASSIC && one_chunk) {
+            walk_store_chunk<CHUNK, true>(g, stage, locals, rvals, lane, in_batch, a, n, P, false);
+        } else {
+            walk_store_chunk<CHUNK, false>(g, stage, locals, rvals, lane, in_batch, a, n, P, again);
+        }
         __syncwarp();
     }
-    const float kept = preserve && !one_chunk && counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
-    if constexpr (CLASSIC) {
-        walk_classic_finish(g, locals, wr.position, kept, wr.lead, stage_get(row, (P - 1) % kWalkChunk), lane, in_batch,
-                            P);
-    } else if (__any_sync(kFull, kept != 1.0f)) {
-        walk_rescale<false>(g, locals, wr.position, kept, wr.position, 1.0f, -1.0f, lane, in_batch, P);
+    if constexpr (CHUNK == kWalkChunk) {
+        const float kept = preserve && !one_chunk && counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
+        if constexpr (CLASSIC) {
+            if (!one_chunk) {
+                walk_classic_finish(g, locals, wr.position, kept, wr.lead, stage_get(row, (P - 1) % kWalkChunk), lane,
+                                    in_batch, P);
+            }
+        } else if (__any_sync(kFull, kept != 1.0f)) {
+            walk_rescale<false>(g, locals, wr.position, kept, wr.position, 1.0f, -1.0f, lane, in_batch, P);
+        }
+        __syncwarp();
     }
-    __syncwarp();
 }
 
 // One batch of a warp without noise: setup and the base step straight to the
