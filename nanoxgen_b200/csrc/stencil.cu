@@ -33,8 +33,8 @@
 // where the sort finds a sample of the warps scattered over the mesh: a visit
 // to a cluster costs a warp as much as all pairs cost it over six to eight
 // clusters' guides (200,000 x 4,096 in random triangle order 3,609 us by
-// clusters, 1,200 by all pairs).  155 us at the size
-// above (sorting 21, search 106, the last rows' search partly beside it): bound
+// clusters, 1,200 by all pairs).  149 us at the size
+// above (sorting 23, search 90, the last rows' search mostly beside it): bound
 // by the latency of a warp's chain of clusters.  The sorted guides need memory this entry point has no argument
 // for: they are put into the last rows of the output, whose triangles a second
 // kernel searches from its own shared-memory copy and writes last.
@@ -231,7 +231,7 @@ __device__ __forceinline__ void search_all(TriangleSearch &t, GuideTile &tile, c
 // Measured slower: two triangles per thread sharing each guide load (fewer
 // warps per SM to hide the dependency chains), and a 40-register cap that
 // fits a 200,000-triangle mesh in one wave (spills).
-__global__ void __launch_bounds__(kStencilThreads)
+__global__ void __launch_bounds__(kStencilThreads, 9)
 stencil_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count, const nxg_uint3 *__restrict__ triangles,
                uint32_t triangle_count, const nxg_vec3 *__restrict__ guide_roots,
                const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count, uint32_t keep,
@@ -304,8 +304,8 @@ __device__ __forceinline__ WarpBox warp_box(const TriangleSearch &t) {
 // the roots' box) and writes the scratch; one CTA.  The order within a cell is
 // arbitrary.  Each warp also looks at the triangles of one warp of the search.
 __global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
-                                                       const nxg_uint3 *__restrict__ triangles, uint32_t searched,
-                                                       const nxg_vec3 *__restrict__ guide_roots,
+                                                       const nxg_uint3 *__restrict__ triangles,
+                                                       uint32_t triangle_count, const nxg_vec3 *__restrict__ guide_roots,
                                                        const nxg_vec3 *__restrict__ guide_normals, uint32_t guide_count,
                                                        uint32_t clusters, float4 *scratch) {
     constexpr uint32_t kBits = 4u;  // 4,096 cells, of which a surface meets about a fifth
@@ -322,7 +322,8 @@ __global__ void __launch_bounds__(1024) cluster_kernel(const nxg_vec3 *__restric
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     bool wild = false;
     TriangleSearch sample;
-    begin_triangle(sample, warp * (searched / 1024u) * 32u + lane, positions, vertex_count, triangles, searched);
+    begin_triangle(sample, warp * (triangle_count / 1024u) * 32u + lane, positions, vertex_count, triangles,
+                   triangle_count);
 #pragma unroll
     for (uint32_t q = 0; q < kOwn; ++q) {
         const uint32_t i = q * 1024u + tid;
@@ -693,10 +694,10 @@ __device__ __forceinline__ bool wild_triangle(const TriangleSearch &t) {
 }
 
 // Whether the CTA's triangles lie scattered over too many clusters: whether its
-// warps' boxes touch more than a twentieth of the clusters and 2.5 on average
-// (neighbours touch 2.3 to 4, two patches of sixteen 8 of 20, 19 of 128; all
-// pairs cost as much as visits to a seventh of them).  Every thread of the CTA
-// calls it.
+// warps' boxes touch more than a quarter of the clusters and three on average
+// (neighbours touch 2 to 5; all pairs cost as much as visits to a seventh of
+// them, but a CTA alone takes as long for them as the whole search does).  Every
+// thread of the CTA calls it.
 __device__ __forceinline__ bool scattered_triangles(const WarpBox &bounds, const float4 *scratch, uint32_t clusters) {
     const float4 *boxes = scratch + clusters * kClusterWords;
     uint32_t touched = 0u;
@@ -709,7 +710,7 @@ __device__ __forceinline__ bool scattered_triangles(const WarpBox &bounds, const
     touched = __reduce_add_sync(kFull, touched);
     if ((threadIdx.x & 31u) == 0u) { atomicAdd(&sum, touched); }
     __syncthreads();
-    return sum * 20u > (blockDim.x >> 5) * (clusters + 50u);
+    return sum * 4u > (blockDim.x >> 5) * (clusters + 12u);
 }
 
 // The all-pairs search of one triangle, which every thread of the CTA holds, for
@@ -748,23 +749,24 @@ __device__ __forceinline__ void share_triangle(TriangleSearch &t, const nxg_vec3
     }
 }
 
-// Triangles [0, searched) from the scratch in global memory (the rows from
-// `searched` on); where every triangle takes all pairs, those of the scratch's
-// rows too but for the last row, which says so.
+// Triangles [0, first) from the scratch in global memory (the rows from `first`
+// on); where every triangle takes all pairs, those of the scratch's rows too but
+// for the last row, which says so.
 __global__ void __launch_bounds__(kStencilThreads, 8)
 stencil_cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
-                       const nxg_uint3 *__restrict__ triangles, uint32_t searched, uint32_t triangle_count,
+                       const nxg_uint3 *__restrict__ triangles, uint32_t first, uint32_t triangle_count,
                        const nxg_vec3 *__restrict__ guide_roots, const nxg_vec3 *__restrict__ guide_normals,
                        uint32_t guide_count, uint32_t clusters, uint32_t keep, uint32_t *stencil) {
     __shared__ __align__(16) GuideTile tile;
     chain_wait();
     chain_start();  // from here on the scratch is complete, which the next kernel relies on
-    const uint32_t ti = blockIdx.x * kStencilThreads + threadIdx.x;
-    const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(searched) * kSlots);
+    const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(first) * kSlots);
     const bool all = __ldcg(&scratch[clusters * (kClusterWords + kClusterBoxes)].x) != 0.0f;
-    if (!all && blockIdx.x * kStencilThreads >= searched) { return; }
+    const uint32_t end = all ? triangle_count - 1u : first;
+    if (blockIdx.x * kStencilThreads >= end) { return; }
+    const uint32_t ti = blockIdx.x * kStencilThreads + threadIdx.x;
     TriangleSearch t;
-    begin_triangle(t, ti, positions, vertex_count, triangles, all ? triangle_count - 1u : searched);
+    begin_triangle(t, ti, positions, vertex_count, triangles, end);
     const WarpBox bounds = warp_box(t);
     if (__syncthreads_or(all || wild_triangle(t)) || scattered_triangles(bounds, scratch, clusters)) {
         search_all(t, tile, guide_roots, guide_normals, guide_count);
@@ -782,12 +784,12 @@ stencil_cluster_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_c
 // alone, and one CTA shares its guides out to its threads unless one is wild.
 __global__ void __launch_bounds__(kTailMaxThreads)
 stencil_tail_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_count,
-                    const nxg_uint3 *__restrict__ triangles, uint32_t searched, uint32_t triangle_count,
+                    const nxg_uint3 *__restrict__ triangles, uint32_t first, uint32_t triangle_count,
                     const nxg_vec3 *__restrict__ guide_roots, const nxg_vec3 *__restrict__ guide_normals,
                     uint32_t guide_count, uint32_t clusters, uint32_t keep, uint32_t *stencil) {
     extern __shared__ float4 copy[];
     __shared__ __align__(16) GuideTile tile;
-    const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(searched) * kSlots);
+    const float4 *scratch = reinterpret_cast<const float4 *>(stencil + static_cast<size_t>(first) * kSlots);
     for (uint32_t i = threadIdx.x; i < cluster_scratch_words(clusters); i += blockDim.x) {
         copy[i] = __ldcg(scratch + i);
     }
@@ -795,7 +797,6 @@ stencil_tail_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_coun
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const float4 flags = copy[clusters * (kClusterWords + kClusterBoxes)];
     const bool all = flags.x != 0.0f;
-    const uint32_t ti = searched + blockIdx.x * blockDim.x + threadIdx.x;
     TriangleSearch t;
     if (all && flags.y == 0.0f) {
         begin_triangle(t, triangle_count - 1u, positions, vertex_count, triangles, triangle_count);
@@ -807,6 +808,7 @@ stencil_tail_kernel(const nxg_vec3 *__restrict__ positions, uint32_t vertex_coun
             return;
         }
     }
+    const uint32_t ti = first + blockIdx.x * blockDim.x + threadIdx.x;
     begin_triangle(t, ti, positions, vertex_count, triangles, triangle_count);
     if (all && ti != triangle_count - 1u) { t.live = t.invalid = false; }
     const WarpBox bounds = warp_box(t);
@@ -871,13 +873,19 @@ cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, co
                                                                guide_roots, guide_normals, guide_count, keep, stencil);
         return cudaGetLastError();
     }
-    const uint32_t searched = triangle_count - rows;
+    const uint32_t first = triangle_count - rows;  // row of the scratch
     const size_t copy = sizeof(float4) * cluster_scratch_words(clusters);
-    uint32_t tail_threads = ((rows + kTailCtas - 1u) / kTailCtas + 31u) / 32u * 32u;
-    tail_threads = tail_threads < 256u ? 256u : tail_threads;  // (for share_triangle)
+    const uint32_t tail_threads = ((rows + kTailCtas - 1u) / kTailCtas + 31u) / 32u * 32u;
     // The largest copy, whatever this call's: the limit is the process's.
     cudaError_t e = cudaFuncSetAttribute(stencil_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(sizeof(float4) * cluster_scratch_words(kMaxClusters)));
+    // The same share of the SM's memory for both kernels: with the shares of
+    // their own occupancies the second did not start beside the first until its
+    // SMs were empty (39,600 x 1,000 62 -> 53 us, 200,000 x 4,096 130 -> 118).
+    for (const void *fn : {reinterpret_cast<const void *>(stencil_cluster_kernel),
+                           reinterpret_cast<const void *>(stencil_tail_kernel)}) {
+        if (e == cudaSuccess) { e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 58); }
+    }
     if (e != cudaSuccess) { return e; }
     cudaLaunchConfig_t config{};
     cudaLaunchAttribute attributes[2];
@@ -891,22 +899,23 @@ cudaError_t launch_stencils(const nxg_vec3 *positions, uint32_t vertex_count, co
     config.gridDim = dim3(1);
     config.blockDim = dim3(1024);
     config.dynamicSmemBytes = 0u;
-    e = cudaLaunchKernelEx(&config, cluster_kernel, positions, vertex_count, triangles, searched, guide_roots, guide_normals, guide_count, clusters,
-                           reinterpret_cast<float4 *>(stencil + static_cast<size_t>(searched) * kSlots));
+    e = cudaLaunchKernelEx(&config, cluster_kernel, positions, vertex_count, triangles, triangle_count, guide_roots,
+                           guide_normals, guide_count, clusters,
+                           reinterpret_cast<float4 *>(stencil + static_cast<size_t>(first) * kSlots));
     if (e != cudaSuccess) { return e; }
     config.numAttrs = 1u;
     config.gridDim = dim3((triangle_count + kStencilThreads - 1u) / kStencilThreads);
     config.blockDim = dim3(kStencilThreads);
     config.dynamicSmemBytes = 0u;
-    e = cudaLaunchKernelEx(&config, stencil_cluster_kernel, positions, vertex_count, triangles, searched, triangle_count,
+    e = cudaLaunchKernelEx(&config, stencil_cluster_kernel, positions, vertex_count, triangles, first, triangle_count,
                            guide_roots, guide_normals, guide_count, clusters, keep, stencil);
     if (e != cudaSuccess) { return e; }
     config.numAttrs = 2u;
     config.gridDim = dim3(kTailCtas);
     config.blockDim = dim3(tail_threads);
     config.dynamicSmemBytes = copy;
-    return cudaLaunchKernelEx(&config, stencil_tail_kernel, positions, vertex_count, triangles, searched,
-                              triangle_count, guide_roots, guide_normals, guide_count, clusters, keep, stencil);
+    return cudaLaunchKernelEx(&config, stencil_tail_kernel, positions, vertex_count, triangles, first, triangle_count,
+                              guide_roots, guide_normals, guide_count, clusters, keep, stencil);
 }
 
 size_t align256(size_t n) { return (n + 255u) & ~size_t{255u}; }

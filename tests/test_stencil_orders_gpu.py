@@ -48,18 +48,21 @@ def test_rows_do_not_depend_on_the_triangle_order(cuda, nxg_lib, how, guides):
         assert torch.equal(rows[first:first + 6000], build_stencils(mesh, mine[first:first + 6000].contiguous(), *g))
 
 
-@pytest.mark.parametrize("last", ["degenerate", "wild", "plain"])
+@pytest.mark.parametrize("special", ["degenerate", "wild", "plain", "invalid"])
 @pytest.mark.parametrize("slots", [8, 3])
-def test_last_triangle_of_a_scattered_mesh(cuda, nxg_lib, last, slots):
+def test_row_searched_by_itself(cuda, nxg_lib, special, slots):
     """In a mesh in no order the last row is searched by itself: a degenerate
-    triangle (its face normal penalises half the guides), one beyond the
-    finite range, and an ordinary one."""
+    triangle (its face normal penalises half the guides), one beyond the finite
+    range, an ordinary one, and one of no vertices."""
     rng = np.random.default_rng(3)
+    guides = 1000
     pos, _, tris = fixtures.sphere_mesh(200, 126)
     tris = tris[rng.permutation(len(tris))].astype(np.uint32)
     pos = np.concatenate([pos, np.float32([[np.inf, 0, 0]])])
-    tris[-1] = {"degenerate": [7000, 7000, 7000], "wild": [len(pos) - 1, 5, 6], "plain": tris[-1]}[last]
-    t = rng.integers(0, len(tris) - 1, 1000)
+    row = len(tris) - 1
+    of = {"degenerate": [7000, 7000, 7000], "wild": [len(pos) - 1, 5, 6], "plain": tris[row], "invalid": [len(pos)] * 3}
+    tris[row] = of[special]
+    t = rng.integers(0, row, guides)
     root = pos[tris[t]].mean(1).astype(np.float32)
     root[500:] = root[:500]
     normal = (root / np.linalg.norm(root, axis=1, keepdims=True)).astype(np.float32)
