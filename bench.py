@@ -30,8 +30,6 @@ sys.path.insert(0, ROOT)
 
 STRANDS_PER_GPU = 1_000_000
 FALLBACK_HBM_GBS = 6650.0
-# strand_keys, exclusive_scan, scatter_order (the strand order), guide_offsets,
-# strand_roots, generate
 # Launches per step of the large workload: strand keys, bin scan, scatter,
 # guide offsets, then the lane-walk generator (tile lanes 1) or strand roots
 # plus the lane-group generator.

@@ -397,9 +397,9 @@ uint32_t generate_batched(const nxg_device_asset_desc *assets, const nxg_deforme
             reinterpret_cast<std::uintptr_t>(outputs[d].point_counts) % 4u != 0u) {
             return NXG_ERROR_MISALIGNED_OUTPUT;
         }
-        if (params[d].cvs_per_strand > 128u ||
+        if (params[d].cvs_per_strand > dev::kBatchMaxCvs ||
             uint64_t{assets[d].header.guide_count} * params[d].cvs_per_strand * 16u > (uint64_t{1} << 30)) {
-            return NXG_ERROR_INVALID_ARGUMENT;  // long strands take nxg_generate_packed's serial kernel
+            return NXG_ERROR_INVALID_ARGUMENT;  // more CVs than the CTAs' heads hold (kBatchMaxCvs), or the table's cap
         }
     }
     const BatchLayout layout = batch_layout(assets, params, count);

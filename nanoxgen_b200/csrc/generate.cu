@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(NOISE ? 32 * walk_noise_warps(CHUNK) : 256, NO
     }
 }
 
-// The Classic application for the serial generator (P > 128): one thread
+// The Classic application for the serial generator: one thread
 // per strand re-reads its written points (xgen_classic_runtime.cpp:1650-1678,
 // :1827-1858), measuring cLength for every strand.
 __global__ void classic_serial_apply_kernel(LaunchArgs g) {
@@ -223,7 +223,7 @@ __global__ void guide_offsets_kernel(AssetArgs a, FrameArgs f, uint32_t P, float
     }
 }
 
-// Strands longer than 128 CVs: one thread walks the reference's cursor
+// Strands whose offset table does not fit: one thread walks the reference's cursor
 // (generate.h:445-642) directly.  Slot records live in registers.
 __device__ F3 serial_base_cv(const LaunchArgs &g, const Root &root, const Slot *slots, float wsum,
                              int nearest, uint32_t cv) {
@@ -634,10 +634,6 @@ dev::AssetArgs resolve_asset(const nxg_device_asset_desc &desc) {
     return a;
 }
 
-namespace {
-
-} // namespace
-
 dev::FrameArgs resolve_frame(const dev::AssetArgs &a, const nxg_deformed_desc &d) {
     dev::FrameArgs f{};
     f.positions = d.positions ? reinterpret_cast<const float *>(d.positions) : a.positions;
@@ -648,10 +644,6 @@ dev::FrameArgs resolve_frame(const dev::AssetArgs &a, const nxg_deformed_desc &d
     f.deformed_guide_cvs = d.guide_cvs != nullptr;
     return f;
 }
-
-namespace {
-
-} // namespace
 
 dev::ParamArgs resolve_params(const nxg_generation_params &p, float radius_scale) {
     dev::ParamArgs r{};

@@ -841,13 +841,6 @@ __device__ __forceinline__ float walk_effective_frequency(const ParamArgs &p, fl
     return original_length > 0.0f ? fmaxf(0.5f / original_length, p.noise_frequency) : p.noise_frequency;
 }
 
-// |b - a| in fixed IEEE operations (no contraction left to the compiler), so
-// the length pass and the cursor walk's arc-length prefix agree bit for bit.
-__device__ __forceinline__ float walk_segment_length(F3 b, F3 a) {
-    const F3 d = b - a;
-    return sqrt_approx(__fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x))));
-}
-
 // A strand's cursor between two CVs: the tangent after the last CV handled
 // and the transported normal there, the base point of the next CV and the
 // arc length at it.
