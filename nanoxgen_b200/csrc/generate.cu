@@ -813,14 +813,14 @@ namespace {
 // order makes the warps of an SM read the same guide rows from L1, and costs
 // three launches, two passes over a key per strand, and scattered instead of
 // sequential outputs.  It pays where that locality is missing (a table beyond
-// L1) over enough points.  Whole calls, ordered against not, 4,096 guides:
-// with noise 100,000 x 32 86.2 / 78.7 us, 200,000 x 32 142.9 / 143.5, 300,000
-// x 32 198.2 / 207.6, 4,000,000 x 24 2,062 / 2,475; without noise, where more
-// warps hide the rows' latency, 200,000 x 16 61.5 / 51.3, 1,000,000 x 32 242.7
-// / 244.1, 300,000 x 100 200.0 / 203.4, and 2,000,000 x 32 519.6 / 472.1, the
-// root outputs (60 bytes per strand, partial sectors when scattered) no longer
-// fitting L2.
-// A motion call orders its strands once for all samples.  An order that the
+// L1) over enough points.  Whole calls, ordered against not, 4,096 guides unless
+// said otherwise: with noise 100,000 x 32 86.0 / 79.3 us, 200,000 x 32 143.0 /
+// 143.9, 300,000 x 32 197.7 / 209.1 (of 700 guides 197.4 / 202.4), 1,000,000 x 24
+// of 700 guides 528 / 574, 4,000,000 x 24 2,060 / 2,463.  Without noise more warps
+// hide the rows' latency and the scattered root outputs weigh more (60 bytes per
+// strand), so only long strands gain: 300,000 x 100 197.3 / 200.8, but 1,000,000 x
+// 32 241.1 / 238.9, 800,000 x 31 230.6 / 219.1, 2,000,000 x 32 498 / 462.
+// A motion call orders its strands once for all samples (each then as below).  An order that the
 // caller has prepared costs nothing more and is always taken: with noise
 // 100,000 x 32 71.5 us against 78.5 without it, 1,000,000 x 24 and 200 guides
 // 517 / 537; without noise 100,000 x 32 31.8 / 36.8, 500,000 x 12 87.5 / 110.5,
@@ -831,7 +831,8 @@ namespace {
 bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, bool whole, uint32_t samples) {
     const uint64_t points = uint64_t{count} * P * samples;
     if (uint64_t{guide_count} * P * 16u <= (uint64_t{128} << 10)) { return false; }
-    return noise ? points >= (whole ? 4000000u : 7000000u) : points >= 24000000u && count <= 1700000u;
+    if (noise) { return points >= (whole ? 4000000u : 7000000u); }
+    return points >= 24000000u && count <= (samples > 1u ? 1700000u : 500000u);
 }
 
 // CVs of a strand that the noisy walk stages at a time (walk.cuh).
