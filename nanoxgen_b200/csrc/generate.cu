@@ -580,15 +580,20 @@ bool parallel_path(uint32_t guide_count, uint32_t P) {
 // Strands of more than kMaxParallelCvs CVs take the lane walk too where the
 // workspace holds their offset table (20,011 strands x 160 CVs with noise, 512
 // guides: 1,214 us on the serial kernel).  The workspace need not: a caller's
-// that holds the order alone stays valid and takes the serial kernel.
-bool long_walk_path(uint32_t guide_count, uint32_t P) {
-    return P > kMaxParallelCvs && P <= dev::kWalkMaxCvs && uint64_t{guide_count} * P * 16u <= kMaxOffsetTableBytes;
+// that holds the order alone stays valid and takes the serial kernel.  The
+// queried size asks for the table while it is no larger than the description's
+// own points, so it never dominates a caller's memory: by the strands of the
+// whole description, whose ranges are then generated alike.
+bool long_walk_path(uint32_t guide_count, uint32_t strands, uint32_t P) {
+    return P > kMaxParallelCvs && P <= dev::kWalkMaxCvs && guide_count <= strands &&
+           uint64_t{guide_count} * P * 16u <= kMaxOffsetTableBytes;
 }
 
 // keys[count] | order[count] | bins[guides + 1] | offsets[guides * P] (float4)
 // followed by the guide frame records [guides * 2] (float4).  `total` is what
 // a caller has to provide, `walked` what the lane walk needs.
-WorkspaceLayout workspace_layout(uint32_t guide_count, uint32_t count, uint32_t P) {
+// `strands`: the description's, where the launch is a range of them.
+WorkspaceLayout workspace_layout(uint32_t guide_count, uint32_t count, uint32_t P, uint32_t strands = 0u) {
     WorkspaceLayout w{};
     w.keys = 0u;
     w.order = align_up(uint64_t{count} * 4u, kWorkspaceAlign);
@@ -596,7 +601,8 @@ WorkspaceLayout workspace_layout(uint32_t guide_count, uint32_t count, uint32_t 
     w.offsets = w.hist + align_up((uint64_t{guide_count} + 1u) * 4u, kWorkspaceAlign);
     const uint64_t table = align_up(uint64_t{guide_count} * (P + 2u) * 16u, kWorkspaceAlign);
     w.total = w.offsets + (parallel_path(guide_count, P) ? table : 0u);
-    w.walked = w.offsets + (parallel_path(guide_count, P) || long_walk_path(guide_count, P) ? table : 0u);
+    const bool walked = parallel_path(guide_count, P) || long_walk_path(guide_count, std::max(count, strands), P);
+    w.walked = w.offsets + (walked ? table : 0u);
     return w;
 }
 
@@ -866,7 +872,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
                          const nxg_classic_apply_desc *classic, LaunchForm form, bool order_ready) {
     set_last_cuda_error(0);
     const uint32_t P = params.cvs_per_strand;
-    const WorkspaceLayout ws = workspace_layout(asset.header.guide_count, count, P);
+    const WorkspaceLayout ws = workspace_layout(asset.header.guide_count, count, P, params.strand_count);
     auto *wbase = static_cast<unsigned char *>(workspace);
     LaunchArgs g{};
     g.a = resolve_asset(asset);
@@ -888,7 +894,7 @@ uint32_t launch_generate(const nxg_device_asset_desc &asset, const nxg_deformed_
     const int sms = device_sm_count();
     uint32_t status = NXG_ERROR_NONE;
     const bool parallel = parallel_path(asset.header.guide_count, P);
-    if (!parallel && (!long_walk_path(asset.header.guide_count, P) || workspace_bytes < ws.walked)) {
+    if (!parallel && (ws.walked == ws.total || workspace_bytes < ws.walked)) {  // without the table
         if (!order_ready &&
             (status = launch_order(asset, params.seed, first, count, P, workspace, stream, false))) {
             return status;
@@ -1040,11 +1046,8 @@ extern "C" {
 uint64_t nxg_packed_workspace_size(const nxg_device_asset_desc *asset, const nxg_generation_params *params,
                                    uint32_t strand_count) {
     if (!asset || !params || strand_count == 0u) { return 0u; }
-    // The optional table (past 128 CVs) is asked for while it is no larger than
-    // the description's own points, so it never dominates a caller's memory:
-    // by the whole description, whose ranges are then all generated alike.
-    const auto ws = nxg::workspace_layout(asset->header.guide_count, strand_count, params->cvs_per_strand);
-    return asset->header.guide_count <= std::max(strand_count, params->strand_count) ? ws.walked : ws.total;
+    return nxg::workspace_layout(asset->header.guide_count, strand_count, params->cvs_per_strand, params->strand_count)
+        .walked;
 }
 
 uint32_t nxg_generate_packed(const nxg_device_asset_desc *asset, const nxg_deformed_desc *deformed,

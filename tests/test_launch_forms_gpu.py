@@ -113,3 +113,31 @@ def test_base_points_past_128_cvs(sphere):
     rms = lambda e: float(np.sqrt((e.astype(np.float64) ** 2).mean()))
     assert np.abs(got - wide).max() <= 8 * 2.0 ** -24 * np.abs(wide).max()
     assert rms(got - wide) < 0.97 * rms(thrice - wide)
+
+
+@pytest.mark.parametrize("strands", [10, 63, 64, 100])
+def test_long_strands_whatever_the_room(sphere, strands):
+    """Past 128 CVs the kernel depends on the description, not on how much more
+    room a workspace has than was asked for: the static scratch and a larger
+    workspace give the bits of the queried one, below, at and above the 64
+    guides."""
+    import ctypes
+    import torch
+    from nanoxgen_b200 import _abi
+    from nanoxgen_b200.generator import generate_packed, packed_output_descriptor
+    d, params = sphere
+    params = params.copy(strand_count=strands, cvs_per_strand=140)
+    want = generate_packed(d, params).points
+    asked = int(_abi.lib().nxg_packed_workspace_size(ctypes.byref(d.desc), ctypes.byref(params), strands))
+    room = torch.empty(asked + (8 << 20), dtype=torch.uint8, device="cuda")
+    frame, config = _abi.DeformedDesc(), _abi.LaunchConfig(128)
+    stream = torch.cuda.current_stream().cuda_stream
+    for scratch in (False, True):
+        got = torch.full_like(want, float("nan"))
+        call = [ctypes.byref(x) for x in (d.desc, frame, params, packed_output_descriptor(got), config)]
+        if scratch:
+            code = _abi.lib().nxg_generate_packed_static_scratch(*call, stream)
+        else:
+            code = _abi.lib().nxg_generate_packed(*call, room.data_ptr(), room.numel(), stream)
+        assert code == 0
+        assert torch.equal(got, want)
