@@ -353,7 +353,8 @@ __device__ inline bool fx_noise(FxCurve &k, int P, const DeviceExpression *m, co
                 // The last CV alone is not worth another window.
                 bool lattice = after <= window.limit;
                 if (cv + 1 < P && __any_sync(lanes, !lattice)) {
-                    const uint4 w = walk_fill_window(domain, distance, window, lat, table, 0u, lanes);
+                    const uint4 w = walk_fill_window(domain, distance, window, lat, table, 0u,
+                                                     !(after - distance <= kWalkDirect), lanes);
                     window = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
                     lattice = after <= window.limit;
                 }

@@ -67,6 +67,11 @@ __host__ __device__ constexpr int walk_row(int chunk) { return 3 * chunk + 1; }
 // strand refills its window about once (four columns: 533 us against 526 on
 // 1,000,000 strands x 32).
 constexpr int kWalkWindow = 5;
+// Segments of more lattice cells than this leave a window after one pair of CVs,
+// whose six values the direct noise gives for less than a window costs (200,000
+// strands x 32 at 2 cells a segment 282 us from windows, 252 directly; at 6, where
+// no window holds a pair, 406 with the windows tried first, 252).
+constexpr float kWalkDirect = 1.5f;
 constexpr int kWalkRecords = 6;                    // float4 setup records per strand
 constexpr int kWalkClassicRecords = 8;             // with the Classic values of walk_classic_setup
 constexpr int kWalkNoiseWarps = 12;                // warps of a full noise CTA
@@ -756,12 +761,17 @@ __device__ __forceinline__ f32x2 walk_lattice_pair(const float2 *lat, uint32_t b
 // fits) beyond the round-down floor's range.  A walk that leaves its window at
 // the end starts the next one inside it, so the first two
 // columns are moved there from the old window and only the others are
-// computed (551 -> 533 us on 1,000,000 strands x 32).  Out of line: it is called about twice per strand, and its
+// computed (551 -> 533 us on 1,000,000 strands x 32).  Where one of the lanes says
+// `direct`, the old window stays.  Out of line: it is called about twice per strand, and its
 // registers inlined spill the walk's loop.  Every one of `lanes` calls it.
 static __device__ __noinline__ uint4 walk_fill_window(F3 dom, float distance, WalkWindow old, float2 *lat,
-                                                      const float4 *table, uint32_t copies, unsigned lanes) {
+                                                      const float4 *table, uint32_t copies, bool direct,
+                                                      unsigned lanes) {
     __builtin_assume(__isShared(lat));
     __builtin_assume(__isShared(table));
+    if (__any_sync(lanes, direct)) {
+        return make_uint4(old.bias[0], old.bias[1], old.bias[2], __float_as_uint(old.limit));
+    }
     uint32_t bias[3], moved[3];
     float lo[3];
     bool near = old.limit >= 0.0f;
@@ -950,7 +960,8 @@ __device__ __forceinline__ void walk_pair(WalkCursor &s, F3 n0, F3 n1, f32x2 t, 
             mvn = dot2(mv, tn);
         }
         if (__any_sync(kFull, counts && !(db <= wl.limit))) {
-            const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies, kFull);
+            const uint4 w = walk_fill_window(dom, da, wl, lat, table, copies,
+                                             counts && !(db - da <= kWalkDirect), kFull);
             wl = WalkWindow{{w.x, w.y, w.z}, __uint_as_float(w.w)};
             lattice = __all_sync(kFull, db <= wl.limit || !counts);
         }
