@@ -841,13 +841,19 @@ bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, b
     return points >= 24000000u && count <= (samples > 1u ? 1700000u : 500000u);
 }
 
-// CVs of a strand that the noisy walk stages at a time (walk.cuh).
+// CVs of a strand that the noisy walk stages at a time (walk.cuh).  Up to 24 the
+// whole strand, where two chunks leave the second half empty (1,000,000 x 24 488
+// us, in chunks 522; x 17 468 / 506).  Up to 32 only where its points are
+// rewritten: otherwise two full chunks are the faster (1,000,000 x 32 570, whole
+// 604), except below the frequency floor, where a chunked strand is staged twice
+// (703, whole 582).  A range of strands takes the whole call's path, so the
+// number of strands has no part in it.
 int noise_chunk(uint32_t P, bool classic, const nxg_generation_params &params) {
-    const bool rewritten = classic || params.noise_preserve_length > 0.001f;
-    if (!rewritten || P <= static_cast<uint32_t>(dev::kWalkChunk) || P > static_cast<uint32_t>(dev::kWalkWholeCvs)) {
+    if (P <= static_cast<uint32_t>(dev::kWalkChunk) || P > static_cast<uint32_t>(dev::kWalkWholeCvs)) {
         return dev::kWalkChunk;
     }
-    return P <= 24u ? 24 : 32;
+    if (P <= 24u) { return 24; }
+    return classic || params.noise_preserve_length > 0.001f ? 32 : dev::kWalkChunk;
 }
 
 } // namespace

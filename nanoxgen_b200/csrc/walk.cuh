@@ -53,12 +53,12 @@ namespace nxg {
 namespace dev {
 
 constexpr int kWalkChunk = 16;                     // CVs staged at a time
-// Strands of up to 32 CVs whose points are rewritten once the whole strand is
-// known (preserveLength, Classic scalars) are staged whole instead, CHUNK 24 or
-// 32, and rewritten in the stage: through L2 the second pass cost more than
-// the chunks gain.  With noise and Classic scalars 500,000 x 24 331 -> 277 us,
-// x 32 370 -> 341; preserveLength 500,000 x 17 325 -> 250, x 24 320 -> 268, x 32
-// 357 -> 328.
+// Strands of up to 24 CVs, and rewritten ones of up to 32 (noise_chunk), are staged
+// whole instead, CHUNK 24 or 32.  There preserveLength and Classic scalars, which
+// rewrite the points once the whole strand is known, do so in the stage: through
+// L2 the second pass cost more than the chunks gain.  With noise and Classic
+// scalars 500,000 x 24 331 -> 277 us, x 32 370 -> 341; preserveLength 500,000 x 17
+// 325 -> 250, x 24 320 -> 268, x 32 357 -> 328.
 constexpr int kWalkWholeCvs = 32;
 // Words of a stage row: x, y, z per CV, and the strand's radius override (an odd stride).
 __host__ __device__ constexpr int walk_row(int chunk) { return 3 * chunk + 1; }
@@ -1020,29 +1020,6 @@ __device__ __forceinline__ float walk_preserve_scale(const ParamArgs &p, float o
     return fabsf(noisy - target) >= 0.0001f ? target / noisy : 1.0f;
 }
 
-// Length of this lane's base curve (generate.h:420-433), chunk by chunk.
-// Every lane of the warp calls it.
-template <int CHUNK>
-static __device__ __noinline__ float walk_base_length(const LaunchArgs &g, const float4 *records, float *stage,
-                                                  const float *tvals, const float4 *offsets, int lane, int in_batch,
-                                                  int P, F3 first) {
-    const float *row = stage + lane * walk_row(CHUNK);
-    float length = 0.0f;
-    for (int a = 0; a < P - 1; a += CHUNK) {
-        const int n = min(CHUNK, P - 1 - a);
-        walk_base_chunk<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
-        __syncwarp();
-        for (int i = 0; i < n; ++i) {
-            const F3 next = stage_get(row, i);
-            const F3 d = next - first;
-            length = __fadd_rn(length, sqrt_approx(dot(d, d)));
-            first = next;
-        }
-        __syncwarp();
-    }
-    return length;
-}
-
 // Store step of one chunk, eight lanes per strand as in walk_base_chunk: each
 // store instruction writes four strands' runs of eight consecutive float4s.
 // RADII: a strand's last stage word overrides its radius unless it is negative.
@@ -1261,27 +1238,45 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
     window.limit = -1.0f;
     F3 previous = s.cur;
     float noisy = 0.0f;
-    for (int a = 0; a < P; a += CHUNK) {
+    // Below the frequency floor the chunks are staged once to measure the base
+    // curve (`measuring`) and once more to be walked.
+    bool measuring = false;
+    float base_length = 0.0f;
+    F3 measured = s.cur;
+    for (int a = 0; a < P;) {
         const int n = min(CHUNK, P - a);
         walk_base_chunk<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
         __syncwarp();
-        if (a == 0) {
+        if (a == 0 && base_length >= 0.0f) {
             // The effective frequency max(0.5 / length, frequency)
             // (generate.h:543) is the frequency itself for a strand of at
             // least 0.5 / frequency, which a chord that long from the root to
             // the chunk's last point or to the tip shows; else the base curve
-            // is measured.
+            // is measured (generate.h:420-433).
             const auto sure = [&](F3 point) {
                 const F3 chord = point - s.cur;
                 return sqrt_approx(dot(chord, chord)) * p.noise_frequency * 0.9999f >= 0.5f || !counts;
             };
-            if (!__all_sync(kFull, sure(stage_get(row, min(n, P - 1) - 1))) &&
-                !__all_sync(kFull, sure(walk_base_point(records, lane, P - 1, tvals[P - 1], p.length_scale,
-                                                        offsets)))) {
-                f_eff = walk_effective_frequency(
-                    p, walk_base_length<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, P, s.cur));
-                walk_base_chunk<CHUNK>(g, records, stage, tvals, offsets, lane, in_batch, a, n, P);
+            measuring = !__all_sync(kFull, sure(stage_get(row, min(n, P - 1) - 1))) &&
+                        (P <= CHUNK || !__all_sync(kFull, sure(walk_base_point(records, lane, P - 1, tvals[P - 1],
+                                                                               p.length_scale, offsets))));
+        }
+        if (measuring) {
+            for (int i = 0; i < min(n, P - 1 - a); ++i) {
+                const F3 next = stage_get(row, i);
+                const F3 d = next - measured;
+                base_length = __fadd_rn(base_length, sqrt_approx(dot(d, d)));
+                measured = next;
+            }
+            if (a + CHUNK >= P - 1) {
+                f_eff = walk_effective_frequency(p, base_length);
+                base_length = -1.0f;  // measured
+                measuring = false;
+            }
+            if (a + CHUNK < P - 1 || a > 0) {  // the next chunk, or the first again
+                a = measuring ? a + CHUNK : 0;
                 __syncwarp();
+                continue;
             }
         }
         F3 n0 = stage_get(row, 0), n1 = stage_get(row, 1);
@@ -1316,6 +1311,7 @@ __device__ __forceinline__ void walk_noise_batch(const LaunchArgs &g, const floa
             walk_store_chunk<CHUNK, false>(g, stage, locals, rvals, lane, in_batch, a, n, P, again);
         }
         __syncwarp();
+        a += CHUNK;
     }
     if constexpr (CHUNK == kWalkChunk) {
         const float kept = preserve && !one_chunk && counts ? walk_preserve_scale(p, s.arc, noisy) : 1.0f;
