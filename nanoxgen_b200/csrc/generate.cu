@@ -820,20 +820,20 @@ namespace {
 // three launches, two passes over a key per strand, and scattered instead of
 // sequential outputs.  It pays where that locality is missing (a table beyond
 // L1) over enough points.  Whole calls, ordered against not, 4,096 guides unless
-// said otherwise: with noise 100,000 x 32 86.0 / 79.3 us, 200,000 x 32 143.0 /
-// 143.9, 300,000 x 32 197.7 / 209.1 (of 700 guides 197.4 / 202.4), 1,000,000 x 24
-// of 700 guides 528 / 574, 4,000,000 x 24 2,060 / 2,463.  Without noise more warps
+// said otherwise: with noise 100,000 x 32 85.5 / 78.1 us, 200,000 x 32 142.1 /
+// 143.2, 300,000 x 32 196.2 / 207.1 (of 700 guides 196.9 / 201.1).  Without noise more warps
 // hide the rows' latency and the scattered root outputs weigh more (60 bytes per
 // strand), so only long strands gain: 300,000 x 100 197.3 / 200.8, but 1,000,000 x
 // 32 241.1 / 238.9, 800,000 x 31 230.6 / 219.1, 2,000,000 x 32 498 / 462.
 // A motion call orders its strands once for all samples (each then as below).  An order that the
 // caller has prepared costs nothing more and is always taken: with noise
 // 100,000 x 32 71.5 us against 78.5 without it, 1,000,000 x 24 and 200 guides
-// 517 / 537; without noise 100,000 x 32 31.8 / 36.8, 500,000 x 12 87.5 / 110.5,
+// 492 / 513; without noise 100,000 x 32 31.8 / 36.8, 500,000 x 12 87.5 / 110.5,
 // 2,000,000 x 24 378 / 414.
-// Whole stages leave the rows little of L1, so there it pays earlier: Classic
-// scalars on 170,000 x 24 109.1 / 117.2 us, on 130,000 x 24 100.5 / 102.0, of 700
-// guides 98.3 / 96.3.
+// Whole stages leave the rows little of L1, so there it pays earlier: 170,000 x 24
+// 103.4 / 110.7 us (of 700 guides 102.2 / 104.4), 130,000 x 24 95.4 / 96.2 (of 700
+// guides 93.9 / 90.2), 1,000,000 x 24 of 700 guides 490 / 533, 4,000,000 x 24 1,947 /
+// 2,218; with Classic scalars 170,000 x 24 109.5 / 117.5.
 bool wants_order(uint32_t guide_count, uint32_t count, uint32_t P, bool noise, bool whole, uint32_t samples) {
     const uint64_t points = uint64_t{count} * P * samples;
     if (uint64_t{guide_count} * P * 16u <= (uint64_t{128} << 10)) { return false; }
