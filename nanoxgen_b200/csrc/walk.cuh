@@ -36,9 +36,9 @@
 // before it uses one; and the gradient table is held eight times, free of
 // bank conflicts.
 // Twelve warps at 168 registers; sixteen at 128 spilled (729 us).  1,000,000 x
-// 32: 601 us staged whole with all columns, 531 us now; 150,001 x 61: 419 us
-// on lane groups with scans, 204 us; 20,011 x 160: 1,241 us on one thread per
-// strand, 103 us (121 before the equal batches of small calls).
+// 32: 601 us staged whole with all columns, 543 us now; 150,000 x 61 with
+// preserveLength: 408 us on lane groups with scans, 191 us; 20,000 x 160: 1,241 us
+// on one thread per strand, 104 us (121 before the equal batches of small calls).
 //
 // Stage rows are 49 words apart (73 and 97 where strands are staged whole) and a
 // CV takes 3 words; both strides are odd,
